@@ -44,6 +44,9 @@ struct DevCopy {
     std::deque<HostPipe> pipes;
     CNode* nodes = nullptr;
     CTri* tris = nullptr;
+    WNode* wnodes = nullptr;       // expanded records (launch_expand)
+    WTri* wtris = nullptr;
+    DeviceTree view() const { return DeviceTree{nodes, tris, wnodes, wtris}; }
     int32_t* face_vidx = nullptr;  // [F, 3] (meshes only), uploaded on first use
     int32_t* face_slot = nullptr;  // [F] soup slot of each face id, -1 if none
     float* node_box = nullptr;     // [n_nodes, 6] refit scratch
@@ -143,6 +146,18 @@ int cuda_fail(cudaError_t e, const char* what) {
 int host_threads() { return host_build_threads(); }
 
 
+// Expanded records of a device copy: allocated (one block, triangles after
+// nodes) on the first call, filled from its nodes and triangles on stream s.
+cudaError_t expand_copy(cubvh_bvh* h, DevCopy& d, cudaStream_t s) {
+    const size_t nn = h->host.nodes.size(), nt = h->host.tris.size();
+    if (!d.wnodes) {
+        const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&d.wnodes), nn * sizeof(WNode) + nt * sizeof(WTri));
+        if (e != cudaSuccess) { d.wnodes = nullptr; return e; }
+        d.wtris = reinterpret_cast<WTri*>(d.wnodes + nn);
+    }
+    return launch_expand((int64_t)nn, (int64_t)nt, d.nodes, d.tris, d.wnodes, d.wtris, s);
+}
+
 // Device copy of the BVH on the current device (uploaded on first use).
 int device_copy(cubvh_bvh* h, DevCopy** out) {
     int device = 0;
@@ -158,8 +173,10 @@ int device_copy(cubvh_bvh* h, DevCopy** out) {
     if ((e = cudaMalloc(&d.nodes, nb)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(nodes)");
     if ((e = cudaMalloc(&d.tris, tb)) != cudaSuccess) { cudaFree(d.nodes); return cuda_fail(e, "cudaMalloc(triangles)"); }
     if ((e = cudaMemcpy(d.nodes, h->host.nodes.data(), nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(d.tris, h->host.tris.data(), tb, cudaMemcpyHostToDevice)) != cudaSuccess) {
+        (e = cudaMemcpy(d.tris, h->host.tris.data(), tb, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = expand_copy(h, d, 0)) != cudaSuccess || (e = cudaStreamSynchronize(0)) != cudaSuccess) {
         cudaFree(d.nodes); cudaFree(d.tris);
+        if (d.wnodes) cudaFree(d.wnodes);
         return cuda_fail(e, "BVH upload");
     }
     h->dev.push_back(d);
@@ -384,6 +401,12 @@ int cubvh_bvh_create_device(const float* vertices, int64_t n_vertices, const int
     d.device = device;
     d.nodes = db.nodes;
     d.tris = db.tris;
+    if ((e = expand_copy(h, d, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess) {
+        cudaFree(db.nodes); cudaFree(db.tris);
+        if (d.wnodes) cudaFree(d.wnodes);
+        delete h;
+        return cuda_fail(e, "GPU build expansion");
+    }
     h->dev.push_back(d);
     *out = h;
     return CUBVH_OK;
@@ -434,6 +457,7 @@ int cubvh_bvh_destroy(cubvh_bvh* h) {
     for (auto& d : h->dev) {
         if (cudaSetDevice(d.device) == cudaSuccess) {
             cudaFree(d.nodes); cudaFree(d.tris);
+            if (d.wnodes) cudaFree(d.wnodes);
             if (d.face_vidx) cudaFree(d.face_vidx);
             if (d.face_slot) cudaFree(d.face_slot);
             if (d.node_box) cudaFree(d.node_box);
@@ -540,7 +564,7 @@ int cubvh_signed_distance(cubvh_bvh* h, const float* points, int64_t n, uint32_t
     void* ws = nullptr;
     cudaError_t e;
     if ((e = pool_alloc(&ws, wsb, s)) != cudaSuccess) return cuda_fail(e, "query workspace allocation");
-    e = launch_distance(kmode, uvw != nullptr, n, points, distances, face_id, uvw, d->nodes, d->tris,
+    e = launch_distance(kmode, uvw != nullptr, n, points, distances, face_id, uvw, d->view(),
                         (int)h->host.slot_of_face0, near, ws, s);
     if (ws) {
         const cudaError_t e2 = cudaFreeAsync(ws, s);
@@ -789,7 +813,7 @@ int cubvh_signed_distance_host(cubvh_bvh* h, const float* points, int64_t n, uin
             cudaStream_t cs) {
             return launch_distance(kmode, uvw != nullptr, cnt, reinterpret_cast<const float*>(in[0]),
                                    reinterpret_cast<float*>(out[0]), reinterpret_cast<int64_t*>(out[1]),
-                                   uvw ? reinterpret_cast<float*>(out[2]) : nullptr, d->nodes, d->tris, slot0, near,
+                                   uvw ? reinterpret_cast<float*>(out[2]) : nullptr, d->view(), slot0, near,
                                    ws, cs, first, /*yield=*/true);
         });
     CUBVH_GUARD_END
@@ -998,6 +1022,7 @@ int cubvh_bvh_refit(cubvh_bvh* h, const float* vertices, int64_t n_vertices, voi
     }
     e = launch_refit((int64_t)h->host.tris.size(), d->tris, d->face_vidx, vertices, d->nodes, d->node_box,
                      h->host.level_start.data(), (int)h->host.level_start.size() - 1, (cudaStream_t)stream);
+    if (e == cudaSuccess) e = expand_copy(h, *d, (cudaStream_t)stream);
     if (e != cudaSuccess) return cuda_fail(e, "refit launch");
     return CUBVH_OK;
     CUBVH_GUARD_END

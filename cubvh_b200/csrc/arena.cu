@@ -50,6 +50,8 @@ struct cubvh_arena {
     int device = -1;
     CNode* d_nodes = nullptr;
     CTri* d_tris = nullptr;
+    WNode* d_wnodes = nullptr;       // expanded records, triangles after nodes
+    WTri* d_wtris = nullptr;
     int64_t* d_face_off = nullptr;
     int32_t* d_gslot = nullptr;
     // query layout
@@ -84,6 +86,16 @@ void run_workers(int n, F fn) {
     for (auto& th : pool) th.join();
 }
 
+// Expanded records of the arena's trees (allocates and fills, waits).
+cudaError_t arena_expand(cubvh_arena* a, cudaStream_t s) {
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&a->d_wnodes),
+                               (size_t)a->n_nodes * sizeof(WNode) + (size_t)a->n_tris * sizeof(WTri));
+    if (e != cudaSuccess) { a->d_wnodes = nullptr; return e; }
+    a->d_wtris = reinterpret_cast<WTri*>(a->d_wnodes + a->n_nodes);
+    e = launch_expand(a->n_nodes, a->n_tris, a->d_nodes, a->d_tris, a->d_wnodes, a->d_wtris, s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 int arena_device(cubvh_arena* a) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -98,7 +110,8 @@ int arena_device(cubvh_arena* a) {
     // a failed upload leaves the arena host-only (device stays -1, pointers
     // null), so a later call retries from scratch instead of leaking
     auto drop = [&](cudaError_t err, const char* what) {
-        for (void** q : {(void**)&a->d_nodes, (void**)&a->d_tris, (void**)&a->d_face_off, (void**)&a->d_gslot})
+        for (void** q : {(void**)&a->d_nodes, (void**)&a->d_tris, (void**)&a->d_face_off, (void**)&a->d_gslot,
+                         (void**)&a->d_wnodes})
             if (*q) { cudaFree(*q); *q = nullptr; }
         return cuda_err(err, what);
     };
@@ -110,7 +123,8 @@ int arena_device(cubvh_arena* a) {
     if ((e = cudaMemcpy(a->d_nodes, a->nodes.data(), nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(a->d_tris, a->tris.data(), tb, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(a->d_face_off, a->face_off.data(), fb, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemcpy(a->d_gslot, a->gslot.data(), sb, cudaMemcpyHostToDevice)) != cudaSuccess)
+        (e = cudaMemcpy(a->d_gslot, a->gslot.data(), sb, cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = arena_expand(a, 0)) != cudaSuccess)
         return drop(e, "arena upload");
     a->device = dev;
     // the raystab sign pass reads the stab-direction tables: set them on this
@@ -300,6 +314,10 @@ int cubvh_arena_create_device(int32_t n_meshes, const float* const* vertices, co
         return cuda_err(e, "arena face offsets");
     }
     a->device = dev;
+    if ((e = arena_expand(a, s)) != cudaSuccess) {
+        cubvh_arena_destroy(a);
+        return cuda_err(e, "arena expansion");
+    }
     if ((e = ensure_constants(dev)) != cudaSuccess) {
         cubvh_arena_destroy(a);
         return cuda_err(e, "constant upload");
@@ -316,6 +334,7 @@ int cubvh_arena_destroy(cubvh_arena* a) {
         const bool have = cudaGetDevice(&cur) == cudaSuccess;
         if (cudaSetDevice(a->device) == cudaSuccess) {
             cudaFree(a->d_nodes); cudaFree(a->d_tris); cudaFree(a->d_face_off); cudaFree(a->d_gslot);
+            if (a->d_wnodes) cudaFree(a->d_wnodes);
             if (a->d_layout) cudaFree(a->d_layout);
         }
         if (have) cudaSetDevice(cur);
@@ -382,7 +401,7 @@ int cubvh_arena_set_queries(cubvh_arena* a, const int64_t* query_offsets, const 
     const size_t o_bsum = off; off += al(sizeof(uint32_t) * (scan::num_chunks(cells) + 1));
     const size_t o_slots = off; off += al(sizeof(int32_t) * std::max<int64_t>(Q, 1));
     const int64_t hcap = heavy_cap_for(std::max<int64_t>(Q, 1));
-    const size_t o_heavy = off; off += al(sizeof(uint2) * hcap);
+    const size_t o_heavy = off; off += al(sizeof(uint4) * hcap);
     const int64_t n_rs_q = (int64_t)rs.size() * 32;                // raystab candidates (second pass)
     const size_t o_cand = off; off += al(sizeof(uint4) * std::max<int64_t>(n_rs_q, 1));
     std::lock_guard<std::mutex> lk(a->mu);
@@ -401,7 +420,7 @@ int cubvh_arena_set_queries(cubvh_arena* a, const int64_t* query_offsets, const 
         (e = up(o_rs, rs.data(), sizeof(PacketDesc) * rs.size())) != cudaSuccess)
         return cuda_err(e, "arena layout upload");
     ArenaLaunch& L = a->L;
-    L.nodes = a->d_nodes; L.tris = a->d_tris;
+    L.tree = DeviceTree{a->d_nodes, a->d_tris, a->d_wnodes, a->d_wtris};
     L.n_meshes = M; L.n_queries = Q;
     L.qoff = reinterpret_cast<const int64_t*>(base + o_qoff);
     L.meshes = reinterpret_cast<const MeshDesc*>(base + o_mesh);
@@ -415,7 +434,7 @@ int cubvh_arena_set_queries(cubvh_arena* a, const int64_t* query_offsets, const 
     L.hist = reinterpret_cast<uint32_t*>(base + o_hist);
     L.bsum = reinterpret_cast<uint32_t*>(base + o_bsum);
     L.slots = reinterpret_cast<int32_t*>(base + o_slots);
-    L.heavy = reinterpret_cast<uint2*>(base + o_heavy);
+    L.heavy = reinterpret_cast<uint4*>(base + o_heavy);
     L.heavy_cap = hcap;
     L.rs_cand = reinterpret_cast<uint4*>(base + o_cand);
     a->n_queries = Q;

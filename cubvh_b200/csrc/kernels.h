@@ -31,7 +31,7 @@ struct ArenaSortDesc { float lo[3], hi[3]; int32_t bits; int64_t cell_off; };
 
 // Everything one arena launch needs (device pointers unless noted).
 struct ArenaLaunch {
-    const CNode* nodes; const CTri* tris;
+    DeviceTree tree;
     int32_t n_meshes;
     int64_t n_queries;
     const int64_t* qoff;               // [M + 1] first query of each mesh
@@ -43,7 +43,7 @@ struct ArenaLaunch {
     const PacketDesc* rs_packets; int64_t n_rs_packets;  // raystab meshes
     unsigned long long* counters;      // 256 bytes
     uint32_t* order; uint32_t* hist; uint32_t* bsum; int32_t* slots;
-    uint2* heavy; int64_t heavy_cap;   // heavy-query list (heavy_cap_for(n_queries) entries)
+    uint4* heavy; int64_t heavy_cap;   // heavy-query list (heavy_cap_for(n_queries) entries)
     uint4* rs_cand;                    // raystab second-pass candidates (32 * n_rs_packets entries)
 };
 cudaError_t launch_arena_distance(const ArenaLaunch& a, const float* pts, float* dist, int64_t* fid, float* uvw,
@@ -75,13 +75,17 @@ struct NearLists {
 // as many short-lived blocks instead of one persistent wave, so kernels of
 // higher-priority streams get SMs during them (host-buffer pipelines).
 cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts, float* dist, int64_t* fid,
-                            float* uvw, const CNode* nodes, const CTri* tris, int slot_face0, NearLists near,
+                            float* uvw, const DeviceTree& tree, int slot_face0, NearLists near,
                             void* ws, cudaStream_t stream, int64_t qbase = 0, bool yield = false);
 // any_ovf: one device int, set to 1 when some list overflowed.
 cudaError_t launch_near_lists(int64_t n_tris, const CNode* nodes, const CTri* tris, int32_t* cnt, int32_t* lst,
                               double* nrm, int* any_ovf, cudaStream_t stream);
 cudaError_t launch_ray(int64_t n, const float* ro, const float* rd, float* pos, int64_t* fid, float* depth,
                        const CNode* nodes, const CTri* tris, void* ws, cudaStream_t stream);
+
+// Expanded records of a tree (layout.h) from its nodes and triangles.
+cudaError_t launch_expand(int64_t n_nodes, int64_t n_tris, const CNode* nodes, const CTri* tris, WNode* wnodes,
+                          WTri* wtris, cudaStream_t stream);
 
 // refit / backward (grad.cu)
 cudaError_t launch_refit(int64_t n_tris, CTri* tris, const int32_t* face_vidx, const float* V, CNode* nodes,

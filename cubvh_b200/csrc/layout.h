@@ -53,6 +53,44 @@ struct alignas(16) CTri {
 };
 static_assert(sizeof(CTri) == 48, "triangle must be 48 bytes");
 
+// Expanded records of the packet kernels, made on the device from the ones
+// above whenever a tree is uploaded, built or refitted (launch_expand).
+//
+// WNode: the eight child boxes as floats, lower corners (with the child's
+// reference, as child_ref gives it) in the first 128 bytes, upper corners in
+// the second, so that eight lanes read the eight children with two coalesced
+// 16-byte loads and no decoding.  A leaf child's box is the exact box of its
+// triangles, an inner child's the intersection of the quantised box with the
+// child's own corner and extent; an unused child has lo = +inf, hi = -inf.
+struct alignas(16) WNode {
+    float lo[8][4];                // x, y, z, reference (int bits)
+    float hi[8][4];                // x, y, z, unused
+};
+static_assert(sizeof(WNode) == 256, "expanded node must be 256 bytes");
+
+// WTri: a triangle in its own plane, for the FP32 distance filter
+// (tri_d2_w, geom.cuh).  The longest edge runs from a along the unit vector
+// ex for L; ey is the unit vector in the plane towards the third corner c,
+// (vx, vy) and (ux, uy) the unit directions in the (ex, ey) plane of the
+// edges a -> c and b -> c, of lengths lac and lbc.  Everything but a is
+// rounded once from double.  L = infinity marks a triangle that the filter
+// must leave undecided (K >= 1e9).
+struct alignas(16) WTri {
+    float ax, ay, az, len;
+    float exx, exy, exz, lac;
+    float eyx, eyy, eyz, lbc;
+    float vx, vy, ux, uy;
+};
+static_assert(sizeof(WTri) == 64, "expanded triangle must be 64 bytes");
+
+// Device arrays of one tree (or of an arena's trees).
+struct DeviceTree {
+    const CNode* nodes = nullptr;
+    const CTri* tris = nullptr;
+    const WNode* wnodes = nullptr;
+    const WTri* wtris = nullptr;
+};
+
 // Double operations rounded once each, on host and device alike (the device
 // compiler would otherwise fuse a multiply and an add).
 CUBVH_HD inline double mul_rn(double x, double y) {

@@ -7,22 +7,14 @@
 // 32-entry local stack, children re-sorted per visit.
 //
 // Execution model here:
-//  * one thread owns one query, but warps are persistent: each warp walks a
-//    block-cyclic sequence of 32-query blocks (warp w takes blocks w, w + W,
-//    w + 2W, ...) and hands the next query of its current block to any lane
-//    whose query finished (ballot + popc), so lanes never idle while the warp
-//    still has work; there are no global atomics and the assignment is
-//    deterministic;
-//  * traversal is "while-while": lanes keep descending inner nodes until
-//    every lane of the warp holds a leaf (or is done), then all test their
-//    leaves together, which keeps node and leaf work converged;
 //  * point queries are visited in Morton-cell order (a counting sort of the
-//    points into 2^(3b) cells of the BVH box) so that the 32 lanes of a warp
-//    traverse nearly the same nodes; the permutation only reorders work,
-//    every result is written to the query's own index;
-//  * children are visited nearest-first (8 keys sorted as packed 32-bit
-//    integers); the nearest child is descended directly, the rest pushed on
-//    a local-memory stack with their lower-bound key, re-checked on pop.
+//    points into 2^(3b) cells of their bounding box), 32 neighbouring ones a
+//    packet; the permutation only reorders work, every result is written to
+//    the query's own index;
+//  * a warp walks the tree once per packet with warp-uniform control flow
+//    (k_udf, k_ray); persistent warps draw packets from a queue;
+//  * queries and rays that do not fit packets (long searches, incoherent
+//    rays, stab rays) are walked by a warp or a lane each.
 #include <climits>
 #include <cstdint>
 #include <cooperative_groups.h>
@@ -375,6 +367,41 @@ struct PacketQueue {
     }
 };
 
+// How k_udf's packets are handed out: tickets 0 .. nbig - 1 are `big`
+// consecutive packets each, the later ones `grab`.  Warps that draw runs of
+// neighbouring packets carry the seed from one to the next, and the short
+// ones at the end even out what the packets cost.
+struct RunShape {
+    int64_t nbig, big, grab;
+    // tickets that hand out npk packets
+    __host__ __device__ int64_t tickets(int64_t npk) const {
+        const int64_t rest = npk - nbig * big;
+        return nbig + (rest > 0 ? (rest + grab - 1) / grab : 0);
+    }
+};
+// The same queue over tickets (one atomicAdd each); block budget as above.
+struct RunQueue {
+    unsigned long long* ctr;
+    int64_t npk, next, end;
+    RunShape sh;
+    int* left;
+    __device__ __forceinline__ RunQueue(unsigned long long* c, int64_t npk_, RunShape s, int* left_)
+        : ctr(c), npk(npk_), next(0), end(0), sh(s), left(left_) {}
+    __device__ __forceinline__ int64_t take() {
+        if (next == end) {
+            unsigned long long v = ~0ull;
+            if ((threadIdx.x & 31) == 0 && !(left && atomicSub(left, 1) <= 0)) v = atomicAdd(ctr, 1ull);
+            v = __shfl_sync(kFull, v, 0);
+            if (v == ~0ull) return -1;   // budget spent: done
+            const int64_t t = (int64_t)v;
+            next = t < sh.nbig ? t * sh.big : sh.nbig * sh.big + (t - sh.nbig) * sh.grab;
+            end = next + (t < sh.nbig ? sh.big : sh.grab);
+        }
+        const int64_t p = next++;
+        return p < npk ? p : -1;
+    }
+};
+
 // What a launch works on: implicit 32-query packets over one BVH (root node
 // 0), or a table of packets, each up to 32 consecutive positions of the
 // query order on one mesh of an arena (root node, face-0 slot and first
@@ -385,7 +412,7 @@ struct Work {
     int64_t n;                // implicit: queries; table: packets
     int slot0;                // implicit: face-0 slot of the single BVH
     int64_t qbase = 0;        // implicit: index of query 0 within its call (raystab streams)
-    __device__ __forceinline__ int64_t packets() const { return table ? n : (n + 31) >> 5; }
+    __host__ __device__ __forceinline__ int64_t packets() const { return table ? n : (n + 31) >> 5; }
     __device__ __forceinline__ void get(int64_t p, int64_t& start, int& count, int& root, int& s0,
                                         int64_t& qoff) const {
         if (table) {
@@ -403,41 +430,9 @@ __device__ __forceinline__ float3 load3(const float* __restrict__ a, int64_t i) 
 }
 
 // ------------------------------------------------------- unsigned distance
-// Warp-uniform stack of a packet traversal, distributed over the lanes'
-// registers: entry e lives in lane e % 32, register slot e / 32 (kStack = 96
-// entries).  push / pop are called by all lanes with the same arguments.
-struct WarpStack {
-    int r0 = 0, r1 = 0, r2 = 0;
-    uint32_t k0 = 0, k1 = 0, k2 = 0;
-    int sp = 0;
-    __device__ __forceinline__ void push(int ref, uint32_t key) {
-        if ((int)(threadIdx.x & 31) == (sp & 31)) {
-            const int s = sp >> 5;
-            if (s == 0) { r0 = ref; k0 = key; } else if (s == 1) { r1 = ref; k1 = key; } else { r2 = ref; k2 = key; }
-        }
-        ++sp;
-    }
-    __device__ __forceinline__ void pop(int& ref, uint32_t& key) {
-        --sp;
-        const int s = sp >> 5;
-        ref = __shfl_sync(kFull, s == 0 ? r0 : (s == 1 ? r1 : r2), sp & 31);
-        key = __shfl_sync(kFull, s == 0 ? k0 : (s == 1 ? k1 : k2), sp & 31);
-    }
-    // next entry whose key some lane still needs (key <= cullmax)
-    __device__ __forceinline__ bool next(uint32_t cullmax, int& cur) {
-        while (sp > 0) {
-            int ref; uint32_t key;
-            pop(ref, key);
-            if (key <= cullmax) { cur = ref; return true; }
-        }
-        return false;
-    }
-};
-
-// The same stack in the warp's shared memory (ref and key tables of
-// kSmemStack entries each); push / pop are called by all lanes with the same
-// arguments, lane 0 writes.  k_ray uses it (C1 rays 6.49 -> 6.40 ms against
-// the register stack); for the distance kernels it was not faster.
+// Warp-uniform stack of a packet traversal in the warp's shared memory (ref
+// and key tables of kSmemStack entries each); push / pop are called by all
+// lanes with the same arguments, lane 0 writes.
 constexpr int kSmemStack = kStack;
 struct WarpStackSmem {
     int* ref; uint32_t* key;
@@ -460,52 +455,257 @@ struct WarpStackSmem {
     }
 };
 
-constexpr int kCand = 8;         // per-lane candidate list of the distance search
-constexpr int kHeavyMinWork = 256;  // a packet is never handed off below this many visits
+// ------------------------------------------------------- expanded records
+// One thread per (node, child): the child's box as floats (layout.h, WNode).
+__global__ void k_expand_nodes(int64_t n, const CNode* __restrict__ nodes, const CTri* __restrict__ tris,
+                               WNode* __restrict__ out) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 8 * n) return;
+    const int i = (int)(t >> 3), j = (int)(t & 7);
+    const NodeView nd = load_node(nodes, i);
+    const uint32_t m = meta_of(nd, j);
+    float3 lo = make_float3(CUDART_INF_F, CUDART_INF_F, CUDART_INF_F);
+    float3 hi = make_float3(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+    int ref = 0;
+    if (m != kEmpty) {
+        ref = child_ref(nd, m);
+        if (ref >= 0) {
+            float3 clo, chi;
+            child_box(nd, j, clo, chi);
+            const NodeView c = load_node(nodes, ref);
+            for (int k = 0; k < 8; ++k) {
+                if (meta_of(c, k) == kEmpty) continue;
+                float3 l, h;
+                child_box(c, k, l, h);
+                lo = make_float3(fminf(lo.x, l.x), fminf(lo.y, l.y), fminf(lo.z, l.z));
+                hi = make_float3(fmaxf(hi.x, h.x), fmaxf(hi.y, h.y), fmaxf(hi.z, h.z));
+            }
+            lo = make_float3(fmaxf(lo.x, clo.x), fmaxf(lo.y, clo.y), fmaxf(lo.z, clo.z));
+            hi = make_float3(fminf(hi.x, chi.x), fminf(hi.y, chi.y), fminf(hi.z, chi.z));
+        } else {
+            const int code = -ref - 1;
+            const int s0 = code >> 2, s1 = s0 + (code & 3) + 1;
+            for (int s = s0; s < s1; ++s) {
+                const TriV v = load_tri(tris, s);
+                lo.x = fminf(lo.x, fminf(v.a.x, fminf(v.b.x, v.c.x)));
+                lo.y = fminf(lo.y, fminf(v.a.y, fminf(v.b.y, v.c.y)));
+                lo.z = fminf(lo.z, fminf(v.a.z, fminf(v.b.z, v.c.z)));
+                hi.x = fmaxf(hi.x, fmaxf(v.a.x, fmaxf(v.b.x, v.c.x)));
+                hi.y = fmaxf(hi.y, fmaxf(v.a.y, fmaxf(v.b.y, v.c.y)));
+                hi.z = fmaxf(hi.z, fmaxf(v.a.z, fmaxf(v.b.z, v.c.z)));
+            }
+        }
+    }
+    float4* o = reinterpret_cast<float4*>(out + i);
+    o[j] = make_float4(lo.x, lo.y, lo.z, __int_as_float(ref));
+    o[8 + j] = make_float4(hi.x, hi.y, hi.z, 0.f);
+}
 
+// One thread per triangle: its frame (layout.h, WTri), in double.  A corner
+// closer to the longest edge than 1e-9 of its length counts as on it.
+__global__ void k_expand_tris(int64_t n, const CTri* __restrict__ tris, WTri* __restrict__ out) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const TriV t = load_tri(tris, (int)s);
+    float3 A = t.a, B = t.b, C = t.c;
+    const d3 eab = dsub(to_d3(B), to_d3(A)), ebc = dsub(to_d3(C), to_d3(B)), eca = dsub(to_d3(A), to_d3(C));
+    const double lab = ddot(eab, eab), lbc = ddot(ebc, ebc), lca = ddot(eca, eca);
+    d3 e = eab;
+    double l2 = lab;
+    if (lbc > lab && lbc >= lca) { A = t.b; B = t.c; C = t.a; e = ebc; l2 = lbc; }
+    else if (lca > lab) { A = t.c; B = t.a; C = t.b; e = eca; l2 = lca; }
+    const double L = sqrt(l2);
+    const d3 ex = L > 0.0 ? dscale(e, 1.0 / L) : d3{1.0, 0.0, 0.0};
+    const d3 w = dsub(to_d3(C), to_d3(A));
+    const double cx = ddot(w, ex);
+    d3 r = dsub(w, dscale(ex, cx));
+    double cy = sqrt(ddot(r, r));
+    d3 ey;
+    if (cy > 1e-9 * L) {
+        ey = dscale(r, 1.0 / cy);
+        ey = dsub(ey, dscale(ex, ddot(ey, ex)));
+    } else {
+        cy = 0.0;
+        const double ax = fabs(ex.x), ay = fabs(ex.y), az = fabs(ex.z);
+        const d3 u = ax <= ay && ax <= az ? d3{1.0, 0.0, 0.0} : (ay <= az ? d3{0.0, 1.0, 0.0} : d3{0.0, 0.0, 1.0});
+        ey = dcross(u, ex);
+    }
+    ey = dscale(ey, 1.0 / sqrt(ddot(ey, ey)));
+    const double ac = sqrt(cx * cx + cy * cy), bx = cx - L, bc = sqrt(bx * bx + cy * cy);
+    float4* o = reinterpret_cast<float4*>(out + s);
+    // a triangle without a usable plane (K >= 1e9, layout.h: the sine of an angle below 1e-8, zero area
+    // among them) is left undecided by an infinite length: the double evaluation's own rounding
+    // could pass the filter's bound there, and gives no number at all for a repeated vertex
+    o[0] = make_float4(A.x, A.y, A.z, t.k >= 1e9f ? CUDART_INF_F : (float)L);
+    o[1] = make_float4((float)ex.x, (float)ex.y, (float)ex.z, (float)ac);
+    o[2] = make_float4((float)ey.x, (float)ey.y, (float)ey.z, (float)bc);
+    o[3] = make_float4(ac > 0.0 ? (float)(cx / ac) : 1.f, ac > 0.0 ? (float)(cy / ac) : 0.f,
+                       bc > 0.0 ? (float)(bx / bc) : 1.f, bc > 0.0 ? (float)(cy / bc) : 0.f);
+}
+
+cudaError_t launch_expand(int64_t n_nodes, int64_t n_tris, const CNode* nodes, const CTri* tris, WNode* wnodes,
+                          WTri* wtris, cudaStream_t stream) {
+    if (n_nodes > 0) { k_expand_nodes<<<(unsigned)((8 * n_nodes + 255) / 256), 256, 0, stream>>>(n_nodes, nodes, tris, wnodes); count_launch(); }
+    if (n_tris > 0) { k_expand_tris<<<(unsigned)((n_tris + 127) / 128), 128, 0, stream>>>(n_tris, tris, wtris); count_launch(); }
+    return cudaGetLastError();
+}
+
+// Pairs of floats in one 64-bit register and the packed operations on them
+// (two results per issued instruction), and the three-input maximum.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2unpack(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 f2add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ f2 f2max3(f2 a, f2 b, float c) {
+    float a0, a1, b0, b1;
+    f2unpack(a, a0, a1);
+    f2unpack(b, b0, b1);
+    return f2pack(max3(a0, b0, c), max3(a1, b1, c));
+}
+
+__device__ __forceinline__ TriW make_triw(float4 w0, float4 w1, float4 w2, float4 w3) {
+    TriW t;
+    t.a = make_float3(w0.x, w0.y, w0.z); t.len = w0.w;
+    t.ex = make_float3(w1.x, w1.y, w1.z); t.lac = w1.w;
+    t.ey = make_float3(w2.x, w2.y, w2.z); t.lbc = w2.w;
+    t.vx = w3.x; t.vy = w3.y; t.ux = w3.z; t.uy = w3.w;
+    return t;
+}
+constexpr int kCand = 8;            // candidate list of a query
+constexpr int kUdfBlocks = 7;       // blocks of k_udf per SM
+
+// Lower bound of the squared distance of p to the triangle in slot s.
+__device__ __forceinline__ float tri_lower_bound(const WTri* __restrict__ wtris, int s, float3 p) {
+    const float4* tw = reinterpret_cast<const float4*>(wtris + s);
+    float err;
+    const float d2 = tri_d2_w(p, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
+    return d2 - err;
+}
+
+// A point's exact nearest triangle by a walk of its own, given an upper
+// bound U of its squared distance: every triangle whose lower bound is
+// within U is evaluated in double.  The bound k_udf ends with is all but
+// exact, so the walk meets little more than the triangles that tie.
+__device__ __noinline__ void walk_ties(const DeviceTree& tree, int root, float3 p, float U, double* bx, int* sx,
+                                       int* ix) {
+    int st[kStack];
+    int sp = 0;
+    st[sp++] = root;
+    double best = *bx;
+    int s_best = *sx, id_best = *ix;
+    const float cull = U * 1.000002f;
+    while (sp > 0) {
+        const int ref = st[--sp];
+        if (ref >= 0) {
+            const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + ref);
+            for (int j = 0; j < 8; ++j) {
+                const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
+                if (box_d2(p, make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z)) <= cull)
+                    st[sp++] = __float_as_int(lo.w);
+            }
+        } else {
+            int s0, s1;
+            leaf_range(ref, s0, s1);
+            for (int s = s0; s < s1; ++s) {
+                if (tri_lower_bound(tree.wtris, s, p) > U) continue;
+                const TriV t = load_tri(tree.tris, s);
+                const double e = dist2_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c));
+                if (e < best || (e == best && (s_best < 0 || t.id < id_best))) { best = e; s_best = s; id_best = t.id; }
+            }
+        }
+    }
+    *bx = best; *sx = s_best; *ix = id_best;
+}
 
 // Exact nearest triangle of 32 Morton-adjacent points per warp (a packet):
 // the warp walks the union of the lanes' search paths with warp-uniform
-// control flow.  A child is visited if any lane's FP32 box distance is within
-// that lane's bound (ballot), in the order of the smallest such distance
-// (warp min).  Leaves run the FP32 triangle test in every lane; each lane
+// control flow.  At an inner node, lane 8 g + j tests child j against the
+// eight points of group g (8 consecutive points of the packet, kept in the
+// registers of all the group's lanes): a child is needed when its box is
+// within the bound of some point.  So the lanes read different boxes (two
+// coalesced 16-byte loads a node) and reduce over points in registers, two
+// points an instruction: about 92 instructions a node.  With a lane per
+// point, every lane reads all eight boxes (64 cycles of the SM's load path a
+// node, which became the bound) and each child needs a warp minimum: 180
+// instructions.  Bounding the groups by boxes instead of testing their
+// points keeps ten times the leaves.  The warp's stack and the candidate
+// lists are in shared memory: 72 registers, 28 warps per SM (16 warps: 10 %
+// slower).  The lane's winner of the warp's previous packet, next to this
+// one in Morton order, gives the first bound.
+// Children are pushed farthest first (by the smallest distance of any point).
+// Leaves run the FP32 triangle test in every lane; each lane
 // keeps U, an upper bound of its squared distance (FP32 estimate + its error
 // bound), and a short list of triangles whose lower bound is within U.  At
 // the end every lane evaluates its surviving candidates in double: the
 // minimum (ties -> lowest face index) is the exact nearest triangle.
 //
-// Tail control: a packet whose walk grows past a warp's fair share of the
-// launch (the mean node + leaf visits of the packets finished so far, in
-// stats[0] / stats[1], times the packets per warp `ppw`; at least
-// kHeavyMinWork) would hold the launch's tail alone: points deep inside a
-// closed mesh or near its medial axis are about equally far from very many
-// triangles.  Such a packet stops and appends its queries to the heavy list,
-// which k_udf_heavy serves with a warp per query.  When the list is full the
-// packet finishes here instead.
+// A point that is not finite, or farther than MAX_DIST from the root's box,
+// finds nothing and takes no part in the walk.
 //
-// The check costs registers in the traversal loop, so it is compiled in
-// (TAIL) only for launches with few packets per warp (below 24): with ppw packets per
-// warp at most one packet in ppw can pass the fair share, and only such
-// launches end on a few long packets.
-template <bool UVW, bool SLOT, bool TAIL>
-__global__ void __launch_bounds__(kQBlock) k_udf(Work w, const uint32_t* __restrict__ order,
+// Bound by instruction issue and the latency of node and triangle loads.
+// Measured against the walk with a lane per point and the records of
+// layout.h's first half (call times): 1M points on 5,120 faces 1.98 -> 0.99
+// ms, 384^3 grid on 177k faces 107.5 -> 48.0 ms, 8.4M watertight points on
+// 82k faces 9.70 -> 5.52 ms, 1,000 points 1.16 -> 0.22 ms.
+//
+// Heavy queries, served afterwards with a warp each (k_udf_heavy, from the
+// bound found so far): a point whose candidate list overflows (many
+// triangles at almost the same distance), and the points of a packet that
+// is still walking after kHandOff visits when the queue is empty: deep
+// inside a closed mesh or near its medial axis points are about equally far
+// from very many triangles, and such a packet would hold the launch's end
+// alone.  When the heavy list is full both finish here instead.
+constexpr int kHandOff = 192;
+template <bool UVW, bool SLOT>
+__global__ void __launch_bounds__(kQBlock, kUdfBlocks) k_udf(Work w, const uint32_t* __restrict__ order,
                                                  const float* __restrict__ pts, float* __restrict__ dist,
                                                  int64_t* __restrict__ face_id, float* __restrict__ uvw,
-                                                 int32_t* __restrict__ slot_out, const CNode* __restrict__ nodes,
-                                                 const CTri* __restrict__ tris,
-                                                 unsigned long long* __restrict__ ctr, int64_t grab,
-                                                 uint2* __restrict__ heavy, unsigned long long* __restrict__ n_heavy,
-                                                 int64_t heavy_cap, unsigned long long* __restrict__ stats,
-                                                 float ppw, int block_grabs) {
+                                                 int32_t* __restrict__ slot_out, const DeviceTree tree,
+                                                 unsigned long long* __restrict__ ctr, RunShape shape,
+                                                 uint4* __restrict__ heavy, unsigned long long* __restrict__ n_heavy,
+                                                 int64_t heavy_cap, int block_grabs) {
+    const CTri* __restrict__ tris = tree.tris;
     const int lane = threadIdx.x & 31;
-    __shared__ __align__(16) float s_box[kQBlock / 32][64];
+    __shared__ uint2 s_cand[kQBlock / 32][kCand][32];
+    __shared__ uint2 s_stack[kQBlock / 32][kStack];
     __shared__ int s_left;
-    float* sb = s_box[threadIdx.x >> 5];
+    uint2* cand = &s_cand[threadIdx.x >> 5][0][lane];   // the lane's candidates, 32 entries apart: slot, lower bound
+    uint2* stk = s_stack[threadIdx.x >> 5];
     if (block_grabs > 0) {  // uniform: the launch's block budget
         if (threadIdx.x == 0) s_left = block_grabs;
         __syncthreads();
     }
-    PacketQueue pq(ctr, w.packets(), grab, block_grabs > 0 ? &s_left : nullptr);
+    RunQueue pq(ctr, w.packets(), shape, block_grabs > 0 ? &s_left : nullptr);
+    const unsigned long long tickets = (unsigned long long)shape.tickets(w.packets());
+    int seed = -1, seed_root = -1;   // the lane's winning slot in the warp's previous packet, and its tree
     for (int64_t pk = pq.take(); pk >= 0; pk = pq.take()) {
         int64_t start, qoff;
         int cnt, root, slot_face0;
@@ -514,104 +714,164 @@ __global__ void __launch_bounds__(kQBlock) k_udf(Work w, const uint32_t* __restr
         const bool act = lane < cnt;
         const int64_t idx = act ? (order ? (int64_t)order[qi] : qi) : 0;
         const float3 p = act ? load3(pts, idx) : make_float3(0.f, 0.f, 0.f);
+        bool near_root;              // the point can be within MAX_DIST of the mesh
+        {
+            const CNode* rn = tree.nodes + root;
+            const float3 lo = make_float3(rn->ox, rn->oy, rn->oz);
+            const float3 hi = make_float3(fmaf(255.f, exp2i(rn->ex), lo.x), fmaf(255.f, exp2i(rn->ey), lo.y),
+                                          fmaf(255.f, exp2i(rn->ez), lo.z));
+            near_root = act && isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && box_d2(p, lo, hi) <= 1e6f * 1.000002f;
+        }
         // U: upper bound of the lane's nearest squared distance (MAX_DIST^2)
-        float U = act ? 1e6f : -1.f;
-        float cull = act ? U * 1.000002f : -1.f;
-        int cs[kCand];
-        float cl[kCand];
+        float U = near_root ? 1e6f : -1.f;
+        if (root == seed_root && near_root && seed >= 0) {
+            const float4* tw = reinterpret_cast<const float4*>(tree.wtris + seed);
+            float err;
+            const float e32 = tri_d2_w(p, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
+            U = fminf(U, e32 + err);
+        }
         int nc = 0;
-        double bx = 1e6;     // exact best of flushed candidates
-        int sx = -1, ix = 0;
-        auto flush = [&](bool final_pass) {
-            for (int i = 0; i < nc; ++i) {
-                if (final_pass && cl[i] > U) continue;
-                const TriV t = load_tri(tris, cs[i]);
-                double bary[3]; d3 cp;
-                const double e = closest_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c), bary, &cp);
-                if (e < bx || (e == bx && (sx < 0 || t.id < ix))) { bx = e; sx = cs[i]; ix = t.id; }
+        // the group's points (infinitely far where there is none) and their bounds, in pairs
+        f2 gx[4], gy[4], gz[4];
+        float gc[8];
+        uint32_t cullmax;
+        {
+            const float3 q = near_root ? p : make_float3(CUDART_INF_F, CUDART_INF_F, CUDART_INF_F);
+            const int g0 = lane & 24;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                gx[i] = f2pack(__shfl_sync(kFull, q.x, g0 + 2 * i), __shfl_sync(kFull, q.x, g0 + 2 * i + 1));
+                gy[i] = f2pack(__shfl_sync(kFull, q.y, g0 + 2 * i), __shfl_sync(kFull, q.y, g0 + 2 * i + 1));
+                gz[i] = f2pack(__shfl_sync(kFull, q.z, g0 + 2 * i), __shfl_sync(kFull, q.z, g0 + 2 * i + 1));
             }
-            nc = 0;
+        }
+        auto share_bounds = [&]() {
+            const float cull = near_root ? U * 1.000002f : -1.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) gc[i] = __shfl_sync(kFull, cull, (lane & 24) + i);
+            cullmax = __reduce_max_sync(kFull, __float_as_uint(fmaxf(cull, 0.f)));
         };
-        uint32_t cullmax = __reduce_max_sync(kFull, __float_as_uint(fmaxf(cull, 0.f)));
-        WarpStack st;
+        share_bounds();
+        const f2 p2[3] = {f2pack(p.x, p.x), f2pack(p.y, p.y), f2pack(p.z, p.z)};
+        const f2 neg = f2pack(-1.f, -1.f);
+        int sp = 0;
         int cur = root;
-        bool live = __any_sync(kFull, act);
+        bool live = __any_sync(kFull, near_root);
         int work = 0;
         bool handed_off = false;
         while (live) {
-            // warp-uniform; checked every 64 visits from kHeavyMinWork on
-            if (TAIL && (++work & 63) == 0 && work >= kHeavyMinWork) {
-                unsigned long long su = 0, np = 0;
-                if (lane == 0) {
-                    su = *reinterpret_cast<volatile unsigned long long*>(stats);
-                    np = *reinterpret_cast<volatile unsigned long long*>(stats + 1);
-                }
-                su = __shfl_sync(kFull, su, 0);
-                np = __shfl_sync(kFull, np, 0);
-                if (np >= 32 && (float)work > (float)su / (float)np * ppw) {
+            if ((++work & 63) == 0 && work >= kHandOff) {   // warp-uniform
+                unsigned long long taken = 0;
+                if (lane == 0) taken = *reinterpret_cast<volatile unsigned long long*>(ctr);
+                taken = __shfl_sync(kFull, taken, 0);
+                if (taken >= tickets) {
                     unsigned long long b = 0;
                     if (lane == 0) b = atomicAdd(n_heavy, (unsigned long long)cnt);
                     b = __shfl_sync(kFull, b, 0);
                     const uint32_t mesh = w.table ? (uint32_t)w.table[pk].mesh : 0u;
-                    if (act && (int64_t)b + lane < heavy_cap) heavy[b + lane] = make_uint2((uint32_t)idx, mesh);
+                    // a list without room for all takes what fits; those queries are served twice, with the same result
+                    if (act && (int64_t)b + lane < heavy_cap) heavy[b + lane] = make_uint4((uint32_t)idx, mesh, __float_as_uint(U), 0u);
                     if ((int64_t)b + cnt <= heavy_cap) { handed_off = true; break; }
-                    // list full: finish the packet here (later checks append again; the list
-                    // length used is min(count, capacity))
                 }
             }
             if (cur >= 0) {
-                const NodeLinks nd = decode_node_warp(nodes, cur, sb);
-                uint32_t k[8];
+                const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + cur);
+                const int j = lane & 7;
+                const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
+                const f2 lx = f2pack(lo.x, lo.x), ly = f2pack(lo.y, lo.y), lz = f2pack(lo.z, lo.z);
+                const f2 hx = f2pack(-hi.x, -hi.x), hy = f2pack(-hi.y, -hi.y), hz = f2pack(-hi.z, -hi.z);
+                bool need = false;
+                float dmin = CUDART_INF_F;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    float3 lo, hi;
-                    warp_box(sb, j, lo, hi);
-                    const float d2 = box_d2(p, lo, hi);
-                    const bool need = meta_of(nd, j) != kEmpty && d2 <= cull;
-                    const uint32_t kmin = __reduce_min_sync(kFull, need ? __float_as_uint(d2) : kFull);
-                    k[j] = kmin != kFull ? ((kmin & ~7u) | (uint32_t)j) : kFull;
+                for (int i = 0; i < 4; ++i) {
+                    const f2 dx = f2max3(f2fma(gx[i], neg, lx), f2add(gx[i], hx), 0.f);
+                    const f2 dy = f2max3(f2fma(gy[i], neg, ly), f2add(gy[i], hy), 0.f);
+                    const f2 dz = f2max3(f2fma(gz[i], neg, lz), f2add(gz[i], hz), 0.f);
+                    float da, db;
+                    f2unpack(f2fma(dz, dz, f2fma(dy, dy, f2mul(dx, dx))), da, db);
+                    need |= da <= gc[2 * i];
+                    need |= db <= gc[2 * i + 1];
+                    dmin = min3(dmin, da, db);
                 }
-                sort8(k);
-#pragma unroll
-                for (int i = 7; i >= 1; --i)
-                    if (k[i] != kFull) st.push(child_ref(nd, meta_of(nd, (int)(k[i] & 7u))), k[i] & ~7u);
-                if (k[0] != kFull) cur = child_ref(nd, meta_of(nd, (int)(k[0] & 7u)));
-                else live = st.next(cullmax, cur);
+                unsigned m = __ballot_sync(kFull, need);
+                m = (m | (m >> 16));
+                m = (m | (m >> 8)) & 0xFFu;          // needed children
+                uint32_t key = __float_as_uint(dmin);
+                key = min(key, __shfl_xor_sync(kFull, key, 8));
+                key = min(key, __shfl_xor_sync(kFull, key, 16));
+                key = (m >> j) & 1u ? ((key & ~7u) | (uint32_t)j) : kFull;
+                // its place on the stack: the number of needed children farther than it, two of
+                // the eight compared by each of the four lanes with this child
+                const uint32_t ka = __shfl_sync(kFull, key, 2 * (lane >> 3)), kb = __shfl_sync(kFull, key, 2 * (lane >> 3) + 1);
+                int pos = (ka > key && ka != kFull ? 1 : 0) + (kb > key && kb != kFull ? 1 : 0);
+                pos += __shfl_xor_sync(kFull, pos, 8);
+                pos += __shfl_xor_sync(kFull, pos, 16);
+                const int kept = __popc(m);
+                __syncwarp();   // the popped entry has been read
+                if (lane < 8 && key != kFull) stk[sp + pos] = make_uint2((uint32_t)__float_as_int(lo.w), key & ~7u);
+                sp += kept;
+                __syncwarp();
             } else {
                 int s0, s1;
                 leaf_range(cur, s0, s1);
-                load_leaf_warp(tris, s0, s1, sb);
-                for (int s = s0; s < s1; ++s) {
-                    const TriV t = warp_tri(sb, s - s0);
+                const float U0 = U;
+                const float4* tw = reinterpret_cast<const float4*>(tree.wtris + s0);
+                for (int s = s0; s < s1; ++s, tw += 4) {
                     float err;
-                    const float e32 = tri_d2_f(p, t, &err);
+                    const float e32 = tri_d2_w(p, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
                     const float lb = e32 - err;
-                    if (act && lb <= U) {
+                    const bool c = near_root && !(lb > U);   // within the bound, or undecided (no number)
+                    if (c) {
                         U = fminf(U, e32 + err);
-                        if (nc == kCand) {  // keep only live candidates, else settle them exactly
+                        if (nc == kCand) {   // keep only live candidates
                             int m = 0;
-                            for (int i = 0; i < nc; ++i)
-                                if (cl[i] <= U) { cs[m] = cs[i]; cl[m] = cl[i]; ++m; }
-                            nc = m;
-                            if (nc == kCand) {
-                                flush(false);
-                                U = fminf(U, __double2float_ru(bx));
-                            }
+                            for (int k = 0; k < kCand; ++k)
+                                if (!(__uint_as_float(cand[32 * k].y) > U)) { cand[32 * m] = cand[32 * k]; ++m; }
+                            nc = m < kCand ? m : kCand + 1;
                         }
-                        cs[nc] = s; cl[nc] = lb; ++nc;
+                        if (nc < kCand) {
+                            cand[32 * nc] = make_uint2((uint32_t)s, __float_as_uint(lb));
+                            ++nc;
+                        }   // else the list has overflowed (nc = kCand + 1)
                     }
                 }
-                cull = act ? U * 1.000002f : -1.f;
-                cullmax = __reduce_max_sync(kFull, __float_as_uint(fmaxf(cull, 0.f)));
-                live = st.next(cullmax, cur);
+                if (__any_sync(kFull, U < U0)) share_bounds();
+            }
+            // the next entry that some point still needs
+            live = false;
+            while (sp > 0) {
+                const uint2 e = stk[--sp];
+                if (e.y <= cullmax) { cur = (int)e.x; live = true; break; }
             }
         }
-        if (TAIL && !handed_off && lane == 0) {
-            atomicAdd(stats, (unsigned long long)work);
-            atomicAdd(stats + 1, 1ull);
+        if (handed_off) continue;
+        bool mine = act;
+        double bx = 1e6;
+        int sx = -1, ix = 0;
+        if (nc > kCand) {
+            const unsigned long long b = atomicAdd(n_heavy, 1ull);
+            if ((int64_t)b < heavy_cap) {
+                heavy[b] = make_uint4((uint32_t)idx, w.table ? (uint32_t)w.table[pk].mesh : 0u, __float_as_uint(U), 0u);
+                mine = false;
+            } else {
+                walk_ties(tree, root, p, U, &bx, &sx, &ix);
+            }
+            nc = 0;
         }
-        if (handed_off || !act) continue;
-        flush(true);
+        // the k-th live candidates of all lanes together
+        for (int i = 0;; ++i) {
+            while (i < nc && __uint_as_float(cand[32 * i].y) > U) ++i;
+            if (!__any_sync(kFull, i < nc)) break;
+            if (i < nc) {
+                const int s = (int)cand[32 * i].x;
+                const TriV t = load_tri(tris, s);
+                const double e = dist2_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c));
+                if (e < bx || (e == bx && (sx < 0 || t.id < ix))) { bx = e; sx = s; ix = t.id; }
+            }
+        }
+        seed = sx;
+        seed_root = root;
+        if (!mine) continue;
         double d64;
         if (sx < 0) {  // nothing within MAX_DIST: distance 0 on face 0
             sx = slot_face0; d64 = 0.0;
@@ -668,8 +928,7 @@ __device__ void heavy_settle(const HeavyWarp& S, int nc, float lim, const CTri* 
         if (S.cl[i] > lim) continue;
         const int sl = S.cs[i];
         const TriV t = load_tri(tris, sl);
-        double bary[3]; d3 cp;
-        const double d = closest_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c), bary, &cp);
+        const double d = dist2_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c));
         if (d < e || (d == e && t.id < id)) { e = d; s = sl; id = t.id; }
     }
 #pragma unroll
@@ -682,14 +941,15 @@ __device__ void heavy_settle(const HeavyWarp& S, int nc, float lim, const CTri* 
 }
 
 template <bool UVW, bool SLOT>
-__global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint2* __restrict__ heavy,
+__global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint4* __restrict__ heavy,
                                                        const unsigned long long* __restrict__ n_heavy,
                                                        int64_t heavy_cap, const MeshDesc* __restrict__ meshes,
                                                        int slot_face0, const float* __restrict__ pts,
                                                        float* __restrict__ dist, int64_t* __restrict__ face_id,
                                                        float* __restrict__ uvw, int32_t* __restrict__ slot_out,
-                                                       const CNode* __restrict__ nodes, const CTri* __restrict__ tris,
+                                                       const DeviceTree tree,
                                                        unsigned long long* __restrict__ ctr) {
+    const CTri* __restrict__ tris = tree.tris;
     __shared__ HeavyWarp shw[kQBlock / 32];
     HeavyWarp& S = shw[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -701,7 +961,7 @@ __global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint2* __restrict__
         if (lane == 0) qi = atomicAdd(ctr, 1ull);
         qi = __shfl_sync(kFull, qi, 0);
         if ((int64_t)qi >= nh) break;
-        const uint2 hq = heavy[qi];
+        const uint4 hq = heavy[qi];
         const int64_t idx = hq.x;
         int root = 0, s0 = slot_face0;
         if (meshes) {
@@ -710,10 +970,11 @@ __global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint2* __restrict__
             s0 = md.slot0;
         }
         const float3 p = load3(pts, idx);
-        float U = 1e6f;  // MAX_DIST^2
+        float U = fminf(1e6f, fmaxf(__uint_as_float(hq.z), 0.f));  // the bound found so far (MAX_DIST^2)
         double bx = 1e6;
         int sx = -1, ix = 0;
-        int nc = 0, sp = 1;
+        // a point that is not finite, or too far away (U < 0), finds nothing
+        int nc = 0, sp = __uint_as_float(hq.z) >= 0.f ? 1 : 0;
         __syncwarp();  // the previous query is done with S
         if (lane == 0) { S.ref[0] = root; S.key[0] = 0u; }
         __syncwarp();
@@ -742,18 +1003,14 @@ __global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint2* __restrict__
             int cref = 0;
             uint32_t key = 0u;
             if (ni < nn) {
-                const NodeView nd = load_node(nodes, S.pop[ni]);
-                const uint32_t mm = meta_of(nd, j);
-                if (mm != kEmpty) {
-                    float3 lo, hi;
-                    child_box(nd, j, lo, hi);
-                    const float d2 = box_d2(p, lo, hi);
-                    if (d2 <= cull) {
-                        take = true;
-                        key = __float_as_uint(d2);
-                        cref = child_ref(nd, mm);
-                        leaf = cref < 0;
-                    }
+                const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + S.pop[ni]);
+                const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
+                const float d2 = box_d2(p, make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z));
+                if (d2 <= cull) {   // an unused child's box is infinitely far
+                    take = true;
+                    key = __float_as_uint(d2);
+                    cref = __float_as_int(lo.w);
+                    leaf = cref < 0;
                 }
             }
             const unsigned mi = __ballot_sync(kFull, take && !leaf);
@@ -785,18 +1042,19 @@ __global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint2* __restrict__
                 int slot = -1;
                 if (t < T) {
                     slot = S.tslot[t];
-                    e32 = tri_d2_f(p, load_tri(tris, slot), &err);
+                    const float4* tw = reinterpret_cast<const float4*>(tree.wtris + slot);
+                    e32 = tri_d2_w(p, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
                 }
                 const float ub = t < T ? e32 + err : CUDART_INF_F;
                 U = fminf(U, __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(ub))));
                 const float lb = e32 - err;
-                const bool cand = t < T && lb <= U;
+                const bool cand = t < T && !(lb > U);
                 const unsigned mc = __ballot_sync(kFull, cand);
                 if (nc + __popc(mc) > kHCand) {  // warp-uniform: drop dead candidates, else settle them
                     int keep = 0;
                     for (int i0 = 0; i0 < nc; i0 += 32) {
                         const int i = i0 + lane;
-                        const bool kp = i < nc && S.cl[i] <= U;
+                        const bool kp = i < nc && !(S.cl[i] > U);
                         const int cs_i = kp ? S.cs[i] : 0;
                         const float cl_i = kp ? S.cl[i] : 0.f;
                         const unsigned mk = __ballot_sync(kFull, kp);
@@ -1818,21 +2076,13 @@ int cell_bits(int64_t n) {
 
 }  // namespace
 
-// Heavy-query list length for n queries: a 32nd of them (at least 32768, at
-// most n); a full list only means packets finish in place.
+// Heavy-query list length for n queries: a 32nd of them, at least 262,144
+// (4 MB), at most n: a launch of few packets per warp may hand most of its
+// queries over.  A full list only means packets finish in place.
 int64_t heavy_cap_for(int64_t n) {
-    const int64_t c = n / 32 > 32768 ? n / 32 : 32768;
+    const int64_t c = n / 32 > (1 << 18) ? n / 32 : (1 << 18);
     return c < n ? c : n;
 }
-
-namespace {
-// launches with fewer packets per warp run k_udf with tail control
-constexpr float kTailPpw = 24.f;
-// packets per warp of a launch
-float packets_per_warp(int64_t packets, unsigned grid) {
-    return (float)packets / (float)((int64_t)grid * (kQBlock / 32));
-}
-}  // namespace
 
 namespace {
 // Ray launch workspace: counters (256 bytes), the unit order, a skip flag
@@ -1862,7 +2112,7 @@ size_t query_workspace_bytes(int mode, int64_t n) {
     }
     if (mode > 0) b += al(sizeof(int32_t) * n);                   // winning slots
     if (mode == 1) b += al(sizeof(uint32_t) * n);                 // watertight overflow queue
-    if (mode >= 0) b += al(sizeof(uint2) * heavy_cap_for(n));     // heavy-query list
+    if (mode >= 0) b += al(sizeof(uint4) * heavy_cap_for(n));     // heavy-query list
     if (mode == 2) b += al(sizeof(uint4) * n);                    // raystab candidates (second pass)
     if (mode == -1) b = ray_ws(n).end;                           // unit order, skip flags, incoherent packets
     return b;
@@ -1877,19 +2127,37 @@ enum : int {
     kCtArenaRs = 2,     // first raystab pass of an arena (its watertight pass takes kCtSign)
     kCtHeavyN = 6,      // heavy-query list length
     kCtHeavyNext = 7,   // k_udf_heavy queue
-    kCtStats = 8,       // k_udf tail statistics: node + leaf visits (8), packets finished (9)
     kCtOvfN = 10,       // watertight overflow queue length
     kCtCandN = 12,      // raystab second-pass candidates
     kCtLinesNext = 13,  // raystab second-pass queue
     kCtRayLanesN = 14,  // incoherent ray packets listed by k_ray
     kCtRayLanesNext = 15,  // k_ray_lanes queue
 };
-// packets per atomic grab: about 64 grabs per warp of the launch
+// packets per atomic grab: about 64 grabs per warp
 int64_t grab_for(int64_t n, unsigned grid) {
     const int64_t packets = (n + 31) / 32;
     const int64_t warps = (int64_t)grid * (kQBlock / 32);
     const int64_t g = packets / (warps * 64);
     return g < 1 ? 1 : g;
+}
+// Queue shape of k_udf: three quarters of the packets in runs of up to kRun
+// neighbouring ones, the others as grab_for (k_udf's seeds; 16 and 8 measured slower on uneven
+// work), at least about eight tickets per warp.
+constexpr int64_t kRun = 4;
+RunShape run_shape(int64_t n, unsigned grid) {
+    const int64_t packets = (n + 31) / 32;
+    const int64_t warps = (int64_t)grid * (kQBlock / 32);
+    RunShape q{0, 1, grab_for(n, grid)};
+    q.big = packets / (warps * 8);
+    if (q.big > kRun) q.big = kRun;
+    if (q.big <= q.grab) { q.big = 1; return q; }
+    q.nbig = packets * 3 / 4 / q.big;
+    return q;
+}
+// grabs that hand out the packets of n queries
+int64_t grabs_for(int64_t n, unsigned grid) {
+    const int64_t g = grab_for(n, grid);
+    return ((n + 31) / 32 + g - 1) / g;
 }
 // Launch shape of a yielding launch (PacketQueue block budget): kYieldWaves
 // times the persistent grid g, each block taking at most block_grabs grabs,
@@ -1899,9 +2167,8 @@ int64_t grab_for(int64_t n, unsigned grid) {
 // persistent launch (g blocks, no budget).
 constexpr unsigned kYieldWaves = 4;  // measured against 8 and 16
 struct LaunchShape { unsigned grid; int block_grabs; };
-LaunchShape yield_shape(unsigned g, int64_t n, int64_t grab, bool on) {
+LaunchShape yield_shape(unsigned g, int64_t grabs, bool on) {
     if (!on) return {g, 0};
-    const int64_t grabs = ((n + 31) / 32 + grab - 1) / grab;
     int64_t G = (int64_t)g * kYieldWaves;
     if (G > 2 * grabs) G = 2 * grabs > 0 ? 2 * grabs : 1;
     const int64_t bg = (2 * grabs + G - 1) / G;
@@ -1937,10 +2204,38 @@ void launch_raystab(const Work& w, int64_t n, const uint32_t* order, const float
 }
 }  // namespace
 
+namespace {
+template <bool UVW, bool SLOT>
+void launch_nearest_t(const Work& w, int64_t n, const uint32_t* order, const float* pts, float* dist, int64_t* fid,
+                      float* uvw, int32_t* slots, const DeviceTree& tree, uint4* heavy, int64_t hcap,
+                      unsigned long long* ctr, bool yield, cudaStream_t stream) {
+    const unsigned g = persistent_grid(k_udf<UVW, SLOT>, n);
+    const RunShape q = run_shape(n, g);
+    const LaunchShape y = yield_shape(g, q.tickets(w.packets()), yield);
+    k_udf<UVW, SLOT><<<y.grid, kQBlock, 0, stream>>>(w, order, pts, dist, fid, uvw, slots, tree, ctr + kCtUdf, q, heavy,
+                                                     ctr + kCtHeavyN, hcap, y.block_grabs); count_launch();
+    const unsigned gh = persistent_grid(k_udf_heavy<UVW, SLOT>, 32 * hcap);
+    k_udf_heavy<UVW, SLOT><<<gh, kQBlock, 0, stream>>>(heavy, ctr + kCtHeavyN, hcap, w.meshes, w.slot0, pts, dist, fid, uvw,
+                                                       slots, tree, ctr + kCtHeavyNext); count_launch();
+}
+// The distance search over the packets of `w` (n queries): the packets, then
+// the queries they left to k_udf_heavy.
+void launch_nearest(const Work& w, int64_t n, const uint32_t* order, const float* pts, float* dist, int64_t* fid,
+                    float* uvw, int32_t* slots, const DeviceTree& tree, uint4* heavy, int64_t hcap,
+                    unsigned long long* ctr, bool yield, cudaStream_t stream) {
+    if (uvw && slots) launch_nearest_t<true, true>(w, n, order, pts, dist, fid, uvw, slots, tree, heavy, hcap, ctr, yield, stream);
+    else if (uvw) launch_nearest_t<true, false>(w, n, order, pts, dist, fid, uvw, slots, tree, heavy, hcap, ctr, yield, stream);
+    else if (slots) launch_nearest_t<false, true>(w, n, order, pts, dist, fid, uvw, slots, tree, heavy, hcap, ctr, yield, stream);
+    else launch_nearest_t<false, false>(w, n, order, pts, dist, fid, uvw, slots, tree, heavy, hcap, ctr, yield, stream);
+}
+}  // namespace
+
 cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts, float* dist, int64_t* fid,
-                            float* uvw, const CNode* nodes, const CTri* tris, int slot_face0, NearLists near,
+                            float* uvw, const DeviceTree& tree, int slot_face0, NearLists near,
                             void* ws, cudaStream_t stream, int64_t qbase, bool yield) {
     if (n <= 0) return cudaSuccess;
+    const CNode* nodes = tree.nodes;
+    const CTri* tris = tree.tris;
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     char* w = static_cast<char*>(ws);
     unsigned long long* ctr = reinterpret_cast<unsigned long long*>(w); w += 256;
@@ -1966,34 +2261,15 @@ cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts
     if (mode != 0) w += al(sizeof(int32_t) * n);
     uint32_t* ovf = mode == 1 ? reinterpret_cast<uint32_t*>(w) : nullptr;
     if (mode == 1) w += al(sizeof(uint32_t) * n);
-    uint2* heavy = reinterpret_cast<uint2*>(w);
+    uint4* heavy = reinterpret_cast<uint4*>(w);
     const int64_t hcap = heavy_cap_for(n);
-    w += al(sizeof(uint2) * hcap);
+    w += al(sizeof(uint4) * hcap);
     const Work work{nullptr, nullptr, n, slot_face0, qbase};
-#define CUBVH_L(U, S) do { const unsigned g_ = persistent_grid(k_udf<U, S, false>, n); \
-        const float ppw_ = packets_per_warp((n + 31) / 32, g_); \
-        if (ppw_ >= kTailPpw) { \
-            const LaunchShape y_ = yield_shape(g_, n, grab_for(n, g_), yield); \
-            k_udf<U, S, false><<<y_.grid, kQBlock, 0, stream>>>(work, order, pts, dist, fid, uvw, slots, nodes, tris, \
-                                                           ctr + kCtUdf, grab_for(n, g_), heavy, ctr + kCtHeavyN, hcap, ctr + kCtStats, ppw_, \
-                                                           y_.block_grabs); count_launch(); \
-        } else { \
-            const unsigned gt_ = persistent_grid(k_udf<U, S, true>, n); \
-            const LaunchShape y_ = yield_shape(gt_, n, grab_for(n, gt_), yield); \
-            k_udf<U, S, true><<<y_.grid, kQBlock, 0, stream>>>(work, order, pts, dist, fid, uvw, slots, nodes, tris, \
-                                                           ctr + kCtUdf, grab_for(n, gt_), heavy, ctr + kCtHeavyN, hcap, ctr + kCtStats, \
-                                                           packets_per_warp((n + 31) / 32, gt_), y_.block_grabs); count_launch(); \
-            const unsigned gh_ = persistent_grid(k_udf_heavy<U, S>, 32 * hcap); \
-            k_udf_heavy<U, S><<<gh_, kQBlock, 0, stream>>>(heavy, ctr + kCtHeavyN, hcap, nullptr, slot_face0, pts, dist, \
-                                                           fid, uvw, slots, nodes, tris, ctr + kCtHeavyNext); count_launch(); \
-        } } while (0)
-    if (mode == 0) { if (want_uvw) CUBVH_L(true, false); else CUBVH_L(false, false); }
-    else { if (want_uvw) CUBVH_L(true, true); else CUBVH_L(false, true); }
-#undef CUBVH_L
+    launch_nearest(work, n, order, pts, dist, fid, want_uvw ? uvw : nullptr, slots, tree, heavy, hcap, ctr, yield, stream);
     if (mode == 1) {
         if (near.cnt) {
             const unsigned g = persistent_grid(k_sign_watertight<true>, n);
-            const LaunchShape y = yield_shape(g, n, grab_for(n, g), yield);
+            const LaunchShape y = yield_shape(g, grabs_for(n, g), yield);
             k_sign_watertight<true><<<y.grid, kQBlock, 0, stream>>>(work, order, pts, dist, slots, nodes, tris, near, ovf,
                                                                     ctr + kCtOvfN, ctr + kCtSign, grab_for(n, g),
                                                                     y.block_grabs); count_launch();
@@ -2003,7 +2279,7 @@ cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts
             }
         } else {
             const unsigned g = persistent_grid(k_sign_watertight<false>, n);
-            const LaunchShape y = yield_shape(g, n, grab_for(n, g), yield);
+            const LaunchShape y = yield_shape(g, grabs_for(n, g), yield);
             k_sign_watertight<false><<<y.grid, kQBlock, 0, stream>>>(work, order, pts, dist, slots, nodes, tris, near,
                                                                      nullptr, nullptr, ctr + kCtSign, grab_for(n, g),
                                                                      y.block_grabs); count_launch();
@@ -2097,36 +2373,18 @@ cudaError_t launch_arena_distance(const ArenaLaunch& a, const float* pts, float*
     k_arena_scatter<<<g, 256, 0, stream>>>(a.n_queries, pts, a.qoff, a.n_meshes, a.sort, a.hist, a.order); count_launch();
     const bool signed_any = a.n_wt_packets > 0 || a.n_rs_packets > 0;
     const Work all{a.packets, a.meshes, a.n_packets, 0};
-#define CUBVH_L(U, S) do { const unsigned g_ = persistent_grid(k_udf<U, S, false>, a.n_queries); \
-        const float ppw_ = packets_per_warp(a.n_packets, g_); \
-        if (ppw_ >= kTailPpw) { \
-            k_udf<U, S, false><<<g_, kQBlock, 0, stream>>>(all, a.order, pts, dist, fid, uvw, a.slots, a.nodes, \
-                                                           a.tris, a.counters + kCtUdf, grab_for(a.n_queries, g_), a.heavy, \
-                                                           a.counters + kCtHeavyN, a.heavy_cap, a.counters + kCtStats, ppw_, 0); count_launch(); \
-        } else { \
-            const unsigned gt_ = persistent_grid(k_udf<U, S, true>, a.n_queries); \
-            k_udf<U, S, true><<<gt_, kQBlock, 0, stream>>>(all, a.order, pts, dist, fid, uvw, a.slots, a.nodes, \
-                                                           a.tris, a.counters + kCtUdf, grab_for(a.n_queries, gt_), a.heavy, \
-                                                           a.counters + kCtHeavyN, a.heavy_cap, a.counters + kCtStats, \
-                                                           packets_per_warp(a.n_packets, gt_), 0); count_launch(); \
-            const unsigned gh_ = persistent_grid(k_udf_heavy<U, S>, 32 * a.heavy_cap); \
-            k_udf_heavy<U, S><<<gh_, kQBlock, 0, stream>>>(a.heavy, a.counters + kCtHeavyN, a.heavy_cap, a.meshes, 0, pts, \
-                                                           dist, fid, uvw, a.slots, a.nodes, a.tris, \
-                                                           a.counters + kCtHeavyNext); count_launch(); \
-        } } while (0)
-    if (uvw) { if (signed_any) CUBVH_L(true, true); else CUBVH_L(true, false); }
-    else { if (signed_any) CUBVH_L(false, true); else CUBVH_L(false, false); }
-#undef CUBVH_L
+    launch_nearest(all, a.n_queries, a.order, pts, dist, fid, uvw, signed_any ? a.slots : nullptr, a.tree, a.heavy,
+                   a.heavy_cap, a.counters, false, stream);
     if (a.n_wt_packets > 0) {
         const Work w{a.wt_packets, a.meshes, a.n_wt_packets, 0};
         const unsigned gw = persistent_grid(k_sign_watertight<false>, 32 * a.n_wt_packets);
-        k_sign_watertight<false><<<gw, kQBlock, 0, stream>>>(w, a.order, pts, dist, a.slots, a.nodes, a.tris,
+        k_sign_watertight<false><<<gw, kQBlock, 0, stream>>>(w, a.order, pts, dist, a.slots, a.tree.nodes, a.tree.tris,
                                                              NearLists{}, nullptr, nullptr, a.counters + kCtSign,
                                                              grab_for(32 * a.n_wt_packets, gw), 0); count_launch();
     }
     if (a.n_rs_packets > 0) {
         const Work w{a.rs_packets, a.meshes, a.n_rs_packets, 0};
-        launch_raystab(w, 32 * a.n_rs_packets, a.order, pts, dist, a.nodes, a.tris, a.counters + kCtArenaRs,
+        launch_raystab(w, 32 * a.n_rs_packets, a.order, pts, dist, a.tree.nodes, a.tree.tris, a.counters + kCtArenaRs,
                        a.rs_cand, a.counters + kCtCandN, a.counters + kCtLinesNext, stream);
     }
     return cudaGetLastError();
