@@ -46,7 +46,8 @@ struct DevCopy {
     CTri* tris = nullptr;
     WNode* wnodes = nullptr;       // expanded records (launch_expand)
     WTri* wtris = nullptr;
-    DeviceTree view() const { return DeviceTree{nodes, tris, wnodes, wtris}; }
+    int64_t n_tris = 0;
+    DeviceTree view() const { return DeviceTree{nodes, tris, wnodes, wtris, n_tris}; }
     int32_t* face_vidx = nullptr;  // [F, 3] (meshes only), uploaded on first use
     int32_t* face_slot = nullptr;  // [F] soup slot of each face id, -1 if none
     float* node_box = nullptr;     // [n_nodes, 6] refit scratch
@@ -155,6 +156,7 @@ cudaError_t expand_copy(cubvh_bvh* h, DevCopy& d, cudaStream_t s) {
         if (e != cudaSuccess) { d.wnodes = nullptr; return e; }
         d.wtris = reinterpret_cast<WTri*>(d.wnodes + nn);
     }
+    d.n_tris = (int64_t)nt;
     return launch_expand((int64_t)nn, (int64_t)nt, d.nodes, d.tris, d.wnodes, d.wtris, s);
 }
 

@@ -396,6 +396,7 @@ int cubvh_arena_set_queries(cubvh_arena* a, const int64_t* query_offsets, const 
     const size_t o_wt = off; off += al(sizeof(PacketDesc) * std::max<size_t>(wt.size(), 1));
     const size_t o_rs = off; off += al(sizeof(PacketDesc) * std::max<size_t>(rs.size(), 1));
     const size_t o_ctr = off; off += 256;
+    const size_t o_par = off; off += al(sizeof(unsigned long long) * M);
     const size_t o_order = off; off += al(sizeof(uint32_t) * std::max<int64_t>(Q, 1));
     const size_t o_hist = off; off += al(sizeof(uint32_t) * (cells + 1));
     const size_t o_bsum = off; off += al(sizeof(uint32_t) * (scan::num_chunks(cells) + 1));
@@ -420,7 +421,10 @@ int cubvh_arena_set_queries(cubvh_arena* a, const int64_t* query_offsets, const 
         (e = up(o_rs, rs.data(), sizeof(PacketDesc) * rs.size())) != cudaSuccess)
         return cuda_err(e, "arena layout upload");
     ArenaLaunch& L = a->L;
-    L.tree = DeviceTree{a->d_nodes, a->d_tris, a->d_wnodes, a->d_wtris};
+    L.tree = DeviceTree{a->d_nodes, a->d_tris, a->d_wnodes, a->d_wtris, a->n_tris};
+    L.face_off = a->d_face_off;
+    L.face_slot = a->d_gslot;
+    L.parity = reinterpret_cast<unsigned long long*>(base + o_par);
     L.n_meshes = M; L.n_queries = Q;
     L.qoff = reinterpret_cast<const int64_t*>(base + o_qoff);
     L.meshes = reinterpret_cast<const MeshDesc*>(base + o_mesh);

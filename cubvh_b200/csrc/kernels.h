@@ -44,6 +44,9 @@ struct ArenaLaunch {
     unsigned long long* counters;      // 256 bytes
     uint32_t* order; uint32_t* hist; uint32_t* bsum; int32_t* slots;
     uint4* heavy; int64_t heavy_cap;   // heavy-query list (heavy_cap_for(n_queries) entries)
+    const int64_t* face_off;           // [M + 1] first face of each mesh
+    const int32_t* face_slot;          // [faces] soup slot of each face
+    unsigned long long* parity;        // [M] edge parities (raystab)
     uint4* rs_cand;                    // raystab second-pass candidates (32 * n_rs_packets entries)
 };
 cudaError_t launch_arena_distance(const ArenaLaunch& a, const float* pts, float* dist, int64_t* fid, float* uvw,

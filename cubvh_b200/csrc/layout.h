@@ -89,6 +89,7 @@ struct DeviceTree {
     const CTri* tris = nullptr;
     const WNode* wnodes = nullptr;
     const WTri* wtris = nullptr;
+    int64_t n_tris = 0;
 };
 
 // Double operations rounded once each, on host and device alike (the device

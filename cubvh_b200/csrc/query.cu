@@ -413,6 +413,8 @@ struct Work {
     int slot0;                // implicit: face-0 slot of the single BVH
     int64_t qbase = 0;        // implicit: index of query 0 within its call (raystab streams)
     __host__ __device__ __forceinline__ int64_t packets() const { return table ? n : (n + 31) >> 5; }
+    // mesh of packet p (0: the single BVH)
+    __device__ __forceinline__ int mesh_of(int64_t p) const { return table ? table[p].mesh : 0; }
     __device__ __forceinline__ void get(int64_t p, int64_t& start, int& count, int& root, int& s0,
                                         int64_t& qoff) const {
         if (table) {
@@ -1348,21 +1350,100 @@ __global__ void __launch_bounds__(kQBlock) k_sign_watertight_ovf(const uint32_t*
 // within [0, 1000) (src/bvh.cu:408-427); the first miss ends the query.
 // Whether all rays hit does not depend on the order they are traced in.
 //
+// Closed meshes.  Where every edge of a mesh bounds an even number of its
+// triangles (k_edge_parity), the mesh is a cycle modulo two: along any ray
+// from a point that meets no edge, the number of crossings has the parity of
+// the point's winding number.  So when the crossings of one stab ray, all
+// certain by the FP32 test's error bounds, are odd in number, every ray from
+// the point crosses the mesh and all 64 hit: the point is inside after one
+// ray.  No crossing means outside; an even number, an undecided triangle, a
+// mesh that is not closed, or a point so far away that a crossing could lie
+// past t = 1000 leave the query to its other rays.  (A stab ray that the
+// rounding of the double test lets slip between two triangles at their common
+// edge, about 1e-14 of all rays, is not seen this way.)  Inside points took
+// 64 rays, bound by divergence (12.5 of 32 lanes): 2.1M points in the box of a
+// closed 82k-face mesh, 18.9 -> 4.2 ms with the faster distance search.
+
+// Hash of an undirected edge by its end points' coordinates (0 for an edge
+// of no length): mesh edges cancel in pairs under XOR.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
+    x ^= x >> 31;
+    x *= 0x7fb5d329728ea185ull;
+    x ^= x >> 27;
+    x *= 0x81dadef4bc2dd44dull;
+    return x ^ (x >> 33);
+}
+__device__ __forceinline__ unsigned long long point_hash(float3 v) {   // -0 counts as 0
+    const unsigned long long x = __float_as_uint(v.x + 0.f), y = __float_as_uint(v.y + 0.f), z = __float_as_uint(v.z + 0.f);
+    return mix64(mix64(x | (y << 32)) + z + 0x9e3779b97f4a7c15ull);
+}
+__device__ __forceinline__ unsigned long long edge_hash(unsigned long long a, unsigned long long b) {
+    if (a == b) return 0ull;
+    const unsigned long long lo = a < b ? a : b, hi = a < b ? b : a;
+    return mix64(mix64(lo) + 3ull * hi + 1ull);
+}
+// XOR of the edge hashes of every mesh's triangles into parity[m], zeroed
+// before.  Mesh m has the faces face_off[m] .. face_off[m + 1] - 1, face i the
+// soup slot face_slot[i] (both null: one mesh, every slot of nt).  The result is 0
+// for a closed mesh, and for another one with probability 2^-64.  It runs with each raystab call (82k triangles: 3 us)
+// rather than once per tree, so there is no state to keep right across
+// refits, streams and captures.
+__global__ void __launch_bounds__(256) k_edge_parity(int64_t nt, const CTri* __restrict__ tris,
+                                                     const int64_t* __restrict__ face_off,
+                                                     const int32_t* __restrict__ face_slot, int M,
+                                                     unsigned long long* __restrict__ parity) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    unsigned long long h = 0ull;
+    int mesh = -1;
+    for (int k = 0; k < 4; ++k) {   // 128 consecutive faces a warp
+        const int64_t s = warp * 128 + 32 * k + lane;
+        int m = mesh;
+        unsigned long long e = 0ull;
+        if (s < nt) {
+            const TriV t = load_tri(tris, face_slot ? face_slot[s] : (int)s);
+            const unsigned long long a = point_hash(t.a), b = point_hash(t.b), c = point_hash(t.c);
+            e = edge_hash(a, b) ^ edge_hash(b, c) ^ edge_hash(c, a);
+            m = 0;
+            if (face_off) {
+                int lo = 0, hi = M - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (face_off[mid] <= s) lo = mid; else hi = mid - 1;
+                }
+                m = lo;
+            }
+        }
+        if (m != mesh && mesh >= 0) { atomicXor(&parity[mesh], h); h = 0ull; }
+        mesh = m;
+        h ^= e;
+    }
+    const int m0 = __shfl_sync(kFull, mesh, 0);
+    if (__all_sync(kFull, mesh == m0 || mesh < 0)) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) h ^= __shfl_xor_sync(kFull, h, o);
+        if (lane == 0 && m0 >= 0) atomicXor(&parity[m0], h);
+    } else if (mesh >= 0) {
+        atomicXor(&parity[mesh], h);
+    }
+}
+
 // Work is per lane, not per warp: a warp takes a chunk of packets (queries in
 // Morton-cell order) and each lane takes the chunk's next query from a
 // shared-memory counter whenever its own query ends, and starts its next
 // stab ray as soon as the current one hits.  Stab directions differ from
 // lane to lane and inside queries need 64 rays where outside ones end after a
 // few, so lanes never wait for one another except at the end of a chunk.
-// The per-query setup (query index, stab stream offset, root) is computed by
-// the whole warp in lockstep when the chunk is taken.
+// The per-query setup (query index, stab stream offset, root, whether its
+// first ray counts crossings) is computed by the whole warp in lockstep when
+// the chunk is taken.
 //
 // With max_rays < 64 this is the first of two passes: a query whose first
 // max_rays rays all hit is not finished here but appended to `cand` (query
 // index, stab offset, root: warp-aggregated atomic on cand_n), for
 // k_sign_raystab_lines.  Outside points mostly see their first rays miss
-// and end in this pass; the candidates are mostly inside points, which need
-// every ray.
+// and end in this pass, as do the inside points of closed meshes; the
+// candidates are mostly inside points of other meshes, which need every ray.
 constexpr int kChunkMax = 2;  // packets per raystab chunk
 __global__ void __launch_bounds__(kQBlock) k_sign_raystab(Work w, const uint32_t* __restrict__ order,
                                                           const float* __restrict__ pts, float* __restrict__ dist,
@@ -1370,8 +1451,10 @@ __global__ void __launch_bounds__(kQBlock) k_sign_raystab(Work w, const uint32_t
                                                           const CTri* __restrict__ tris,
                                                           unsigned long long* __restrict__ ctr, int64_t grab,
                                                           int max_rays, uint4* __restrict__ cand,
-                                                          unsigned long long* __restrict__ cand_n) {
+                                                          unsigned long long* __restrict__ cand_n,
+                                                          const unsigned long long* __restrict__ parity) {
     __shared__ int s_next[kQBlock / 32];
+    __shared__ uint8_t s_count[kQBlock / 32][kChunkMax * 32];   // the query's first ray counts crossings
     __shared__ uint4 s_q[kQBlock / 32][kChunkMax * 32];  // query index, offset x/y bits, root (-1: none)
     const int wib = threadIdx.x >> 5;
     const float tmaxf = 1000.0f;
@@ -1391,6 +1474,18 @@ __global__ void __launch_bounds__(kQBlock) k_sign_raystab(Work w, const uint32_t
                 // the stab stream of a query is its index within its own call / mesh
                 const float2 o2 = stab_offset((uint32_t)(id - qoff));
                 e = make_uint4((uint32_t)id, __float_as_uint(o2.x), __float_as_uint(o2.y), (uint32_t)rt);
+                // closed, and the whole root box within t < 1000 of the point
+                const float3 q = load3(pts, id);
+                const CNode* rn = nodes + rt;
+                float far2 = 0.f;
+                const float lo[3] = {rn->ox, rn->oy, rn->oz}, qc[3] = {q.x, q.y, q.z};
+                const int ex[3] = {rn->ex, rn->ey, rn->ez};
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float f = fmaxf(fabsf(lo[k] - qc[k]), fabsf(fmaf(255.f, exp2i(ex[k]), lo[k]) - qc[k]));
+                    far2 = fmaf(f, f, far2);
+                }
+                s_count[wib][i] = parity[w.mesh_of(pk0 + (i >> 5))] == 0ull && far2 < 9.8e5f;
             }
             s_q[wib][i] = e;
         }
@@ -1403,6 +1498,8 @@ __global__ void __launch_bounds__(kQBlock) k_sign_raystab(Work w, const uint32_t
         float dinf = 0.f;
         bool degen = false;
         uint32_t r = 0;    // ray r: -d_{r/2} for even r, +d_{r/2} for odd r
+        bool counting = false, unsure = false, any = false;   // crossings of the first ray are counted
+        int crossings = 0;
         int st[kStack];
         int sp = 0;
         while (true) {
@@ -1414,6 +1511,7 @@ __global__ void __launch_bounds__(kQBlock) k_sign_raystab(Work w, const uint32_t
                         idx = e.x;
                         off = make_float2(__uint_as_float(e.y), __uint_as_float(e.z));
                         root = (int)e.w;
+                        counting = s_count[wib][i] != 0;
                         break;
                     }
                 }
@@ -1427,26 +1525,41 @@ __global__ void __launch_bounds__(kQBlock) k_sign_raystab(Work w, const uint32_t
                 dinf = f3inf(d);
                 sp = 0;
                 st[sp++] = root;
+                unsure = any = false;
+                crossings = 0;
             }
-            if (sp == 0) { idx = -1; continue; }  // ray r missed: outside
-            const int ref = st[--sp];
             bool hit = false;
-            if (ref >= 0) {
+            if (sp == 0) {
+                if (!counting || !any) { idx = -1; continue; }  // ray r missed: outside
+                if (!unsure && (crossings & 1)) {               // inside: every ray hits
+                    dist[idx] = -dist[idx];
+                    idx = -1;
+                    continue;
+                }
+                counting = false;                               // ray 0 hit: on with ray 1
+                hit = true;
+            }
+            const int ref = hit ? INT_MAX : st[--sp];
+            if (ref >= 0 && !hit) {
                 const NodeView nd = load_node(nodes, ref);
                 if (degen) push_ray_children<true>(nd, p, inv, cull, st, sp);
                 else push_ray_children_affine(nd, p, inv, cull, st, sp);
-            } else {
+            } else if (ref < 0) {
                 int a, b;
                 leaf_range(ref, a, b);
                 for (int s = a; s < b && !hit; ++s) {
                     const TriV t = load_tri(tris, s);
                     float tt, terr;
                     const int c = ray_tri_f(p, d, dinf, t, tmaxf, &tt, &terr);
-                    if (c == 1) hit = true;
-                    else if (c < 0) {
+                    bool on = c == 1;
+                    if (c < 0) {
                         double t64;
-                        hit = ray_tri_d(to_d3(p), to_d3(d), to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64);
+                        on = ray_tri_d(to_d3(p), to_d3(d), to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64);
+                        unsure = true;
                     }
+                    any |= on;
+                    crossings += on ? 1 : 0;
+                    hit = on && !counting;
                 }
             }
             if (hit) {
@@ -2130,6 +2243,7 @@ enum : int {
     kCtOvfN = 10,       // watertight overflow queue length
     kCtCandN = 12,      // raystab second-pass candidates
     kCtLinesNext = 13,  // raystab second-pass queue
+    kCtParity = 11,     // edge parity of a single BVH (k_edge_parity)
     kCtRayLanesN = 14,  // incoherent ray packets listed by k_ray
     kCtRayLanesNext = 15,  // k_ray_lanes queue
 };
@@ -2191,13 +2305,17 @@ namespace {
 constexpr int kRaystabFirstRays = 2;
 // The two raystab passes over the packets of `w` (n queries): counters ctr
 // (first pass), cand_n (candidates appended), lines_next (second-pass
-// queue); cand holds up to n candidates.
+// queue) and the edge parities (k_edge_parity), all zero; cand holds up to n candidates.
 void launch_raystab(const Work& w, int64_t n, const uint32_t* order, const float* pts, float* dist,
                     const CNode* nodes, const CTri* tris, unsigned long long* ctr, uint4* cand,
-                    unsigned long long* cand_n, unsigned long long* lines_next, cudaStream_t stream) {
+                    unsigned long long* cand_n, unsigned long long* lines_next, int64_t n_tris,
+                    const int64_t* face_off, const int32_t* face_slot, int n_meshes, unsigned long long* parity,
+                    cudaStream_t stream) {
+    k_edge_parity<<<(unsigned)((n_tris + 1023) / 1024), 256, 0, stream>>>(n_tris, tris, face_off, face_slot, n_meshes,
+                                                                          parity); count_launch();
     const unsigned g = persistent_grid(k_sign_raystab, n);
     k_sign_raystab<<<g, kQBlock, 0, stream>>>(w, order, pts, dist, nodes, tris, ctr, chunk_for(n, g),
-                                              kRaystabFirstRays, cand, cand_n); count_launch();
+                                              kRaystabFirstRays, cand, cand_n, parity); count_launch();
     const unsigned g2 = persistent_grid(k_sign_raystab_lines, n);
     k_sign_raystab_lines<<<g2, kQBlock, 0, stream>>>(pts, dist, nodes, tris, cand, cand_n, lines_next,
                                                      kRaystabFirstRays); count_launch();
@@ -2287,7 +2405,7 @@ cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts
     } else if (mode == 2) {
         uint4* cand = reinterpret_cast<uint4*>(w);
         launch_raystab(work, n, order, pts, dist, nodes, tris, ctr + kCtSign, cand, ctr + kCtCandN, ctr + kCtLinesNext,
-                       stream);
+                       tree.n_tris, nullptr, nullptr, 1, ctr + kCtParity, stream);
     }
     return cudaGetLastError();
 }
@@ -2384,8 +2502,10 @@ cudaError_t launch_arena_distance(const ArenaLaunch& a, const float* pts, float*
     }
     if (a.n_rs_packets > 0) {
         const Work w{a.rs_packets, a.meshes, a.n_rs_packets, 0};
+        if ((e = cudaMemsetAsync(a.parity, 0, sizeof(unsigned long long) * a.n_meshes, stream)) != cudaSuccess) return e;
         launch_raystab(w, 32 * a.n_rs_packets, a.order, pts, dist, a.tree.nodes, a.tree.tris, a.counters + kCtArenaRs,
-                       a.rs_cand, a.counters + kCtCandN, a.counters + kCtLinesNext, stream);
+                       a.rs_cand, a.counters + kCtCandN, a.counters + kCtLinesNext, a.tree.n_tris, a.face_off, a.face_slot,
+                       a.n_meshes, a.parity, stream);
     }
     return cudaGetLastError();
 }
