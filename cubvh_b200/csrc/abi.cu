@@ -592,7 +592,7 @@ int cubvh_ray_trace(cubvh_bvh* h, const float* rays_o, const float* rays_d, int6
     void* ws = nullptr;
     cudaError_t e = pool_alloc(&ws, query_workspace_bytes(-1, n), s);
     if (e != cudaSuccess) return cuda_fail(e, "ray workspace allocation");
-    e = launch_ray(n, rays_o, rays_d, positions, face_id, depth, d->nodes, d->tris, ws, s);
+    e = launch_ray(n, rays_o, rays_d, positions, face_id, depth, d->view(), ws, s);
     const cudaError_t e2 = cudaFreeAsync(ws, s);
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return cuda_fail(e, "ray kernel launch");
@@ -783,7 +783,7 @@ int cubvh_ray_trace_host(cubvh_bvh* h, const float* rays_o, const float* rays_d,
             cudaStream_t cs) {
             return launch_ray(cnt, reinterpret_cast<const float*>(in[0]), reinterpret_cast<const float*>(in[1]),
                               reinterpret_cast<float*>(out[0]), reinterpret_cast<int64_t*>(out[1]),
-                              reinterpret_cast<float*>(out[2]), d->nodes, d->tris, ws, cs);
+                              reinterpret_cast<float*>(out[2]), d->view(), ws, cs);
         });
     CUBVH_GUARD_END
 }

@@ -84,7 +84,7 @@ cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts
 cudaError_t launch_near_lists(int64_t n_tris, const CNode* nodes, const CTri* tris, int32_t* cnt, int32_t* lst,
                               double* nrm, int* any_ovf, cudaStream_t stream);
 cudaError_t launch_ray(int64_t n, const float* ro, const float* rd, float* pos, int64_t* fid, float* depth,
-                       const CNode* nodes, const CTri* tris, void* ws, cudaStream_t stream);
+                       const DeviceTree& tree, void* ws, cudaStream_t stream);
 
 // Expanded records of a tree (layout.h) from its nodes and triangles.
 cudaError_t launch_expand(int64_t n_nodes, int64_t n_tris, const CNode* nodes, const CTri* tris, WNode* wnodes,

@@ -54,11 +54,6 @@ __device__ __forceinline__ NodeView load_node(const CNode* __restrict__ nodes, i
     n.hy0 = w4.x; n.hy1 = w4.y; n.hz0 = w4.z; n.hz1 = w4.w;
     return n;
 }
-// A node's links (what a warp-uniform traversal needs besides the boxes).
-struct NodeLinks {
-    int child_base, tri_base;
-    uint32_t meta0, meta1;
-};
 template <class N>
 __device__ __forceinline__ uint32_t meta_of(const N& n, int j) {
     return ((j < 4 ? n.meta0 : n.meta1) >> (8 * (j & 3))) & 0xFFu;
@@ -83,66 +78,6 @@ template <class N>
 __device__ __forceinline__ int child_ref(const N& n, uint32_t m) {
     if (m & 0x80u) return n.child_base + (int)(m & 7u);
     return -((((n.tri_base + (int)(m & 31u)) << 2) | (int)((m >> 5) & 3u)) + 1);
-}
-
-// Cooperative decode for warp-uniform traversals (every lane visits the same
-// node): lane l < 12 loads word l of the quantised bytes (coordinate l / 2 =
-// lo x, y, z, hi x, y, z of children 4 * (l % 2) .. + 3), decodes it as
-// child_box does and stores the floats in the warp's box table s (64 floats,
-// 16-byte aligned): child j at s[8j .. 8j + 7] = lo.xyz, -, hi.xyz, -.  The
-// whole warp then reads the boxes with broadcast loads instead of decoding
-// all 48 bounds in every lane.  Called by all lanes.
-__device__ __forceinline__ NodeLinks decode_node_warp(const CNode* __restrict__ nodes, int i, float* s) {
-    const int lane = threadIdx.x & 31;
-    const uint4* p = reinterpret_cast<const uint4*>(nodes + i);
-    const uint4 l = __ldg(p + 1);
-    uint4 h = make_uint4(0u, 0u, 0u, 0u);
-    uint32_t q = 0u;
-    if (lane < 12) {  // loads first: they do not wait for the table to be free
-        h = __ldg(p);
-        q = __ldg(reinterpret_cast<const uint32_t*>(p + 2) + lane);
-    }
-    __syncwarp();  // the previous node's boxes have been read
-    if (lane < 12) {
-        const int c = lane >> 1;
-        const int ax = c < 3 ? c : c - 3;
-        const float o = __uint_as_float(ax == 0 ? h.x : (ax == 1 ? h.y : h.z));
-        const float sc = exp2i((int)(int8_t)((h.w >> (8 * ax)) & 0xFFu));
-        float* d = s + 32 * (lane & 1) + (c < 3 ? c : c + 1);
-#pragma unroll
-        for (int b = 0; b < 4; ++b) d[8 * b] = fmaf(qbyte(q, b), sc, o);
-    }
-    __syncwarp();
-    return NodeLinks{(int)l.x, (int)l.y, l.z, l.w};
-}
-// Cooperative load of a leaf's triangles (slots s0 .. s1 - 1, at most four,
-// contiguous) into the warp's table: lane l < 3 * count loads 16-byte word l,
-// so the leaf costs one memory latency instead of one per triangle.  Called
-// by all lanes; the table is the box table (the two are used in turn).
-__device__ __forceinline__ void load_leaf_warp(const CTri* __restrict__ tris, int s0, int s1, float* s) {
-    const int lane = threadIdx.x & 31;
-    const bool ld = lane < 3 * (s1 - s0);
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (ld) v = __ldg(reinterpret_cast<const float4*>(tris + s0) + lane);
-    __syncwarp();  // the previous contents have been read
-    if (ld) reinterpret_cast<float4*>(s)[lane] = v;
-    __syncwarp();
-}
-// triangle i of the leaf in the warp's table
-__device__ __forceinline__ TriV warp_tri(const float* s, int i) {
-    const float4* p = reinterpret_cast<const float4*>(s) + 3 * i;
-    const float4 w0 = p[0], w1 = p[1], w2 = p[2];
-    TriV t;
-    t.a = make_float3(w0.x, w0.y, w0.z); t.id = __float_as_int(w0.w);
-    t.b = make_float3(w1.x, w1.y, w1.z); t.ke2 = w1.w;
-    t.c = make_float3(w2.x, w2.y, w2.z); t.k = w2.w;
-    return t;
-}
-__device__ __forceinline__ void warp_box(const float* s, int j, float3& lo, float3& hi) {
-    const float4 a = *reinterpret_cast<const float4*>(s + 8 * j);
-    const float4 b = *reinterpret_cast<const float4*>(s + 8 * j + 4);
-    lo = make_float3(a.x, a.y, a.z);
-    hi = make_float3(b.x, b.y, b.z);
 }
 
 // Batcher odd-even merge sort network for 8 keys (19 comparators), ascending.
@@ -219,8 +154,6 @@ __device__ __forceinline__ void push_ray_children(const NodeView& nd, float3 o, 
     }
 }
 
-// Entry distance (as ordered bits) of the ray into each child of nd, kFull
-// where the ray does not need the child.
 // The same step for a ray without zero direction components, with the
 // node's affine decode folded into the ray: along axis a the plane of byte q
 // is met at t = (origin_a + q * s_a - o_a) * inv_a, computed as
@@ -260,20 +193,6 @@ __device__ __forceinline__ void push_ray_children_affine(const NodeView& nd, flo
     }
 }
 
-template <bool SAFE>
-__device__ __forceinline__ void ray_child_keys(const NodeLinks& nd, const float* sb, float3 o, float3 inv, float cull,
-                                               uint32_t k[8]) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        float3 lo, hi;
-        warp_box(sb, j, lo, hi);
-        float tn, tf;
-        box_ray<SAFE>(o, inv, lo, hi, tn, tf);
-        const float key = fmaxf(tn, 0.f);
-        const bool need = meta_of(nd, j) != kEmpty && tn <= tf && tf >= 0.f && key <= cull;
-        k[j] = need ? __float_as_uint(key) : kFull;
-    }
-}
 // Closest-hit step of one lane's own walk: entry distance (ordered bits of
 // max(tn, 0), child index in the low 3 bits) of the ray into each child of
 // nd that it enters within [0, cull], kFull for the others.  degen (a zero
@@ -432,31 +351,6 @@ __device__ __forceinline__ float3 load3(const float* __restrict__ a, int64_t i) 
 }
 
 // ------------------------------------------------------- unsigned distance
-// Warp-uniform stack of a packet traversal in the warp's shared memory (ref
-// and key tables of kSmemStack entries each); push / pop are called by all
-// lanes with the same arguments, lane 0 writes.
-constexpr int kSmemStack = kStack;
-struct WarpStackSmem {
-    int* ref; uint32_t* key;
-    int sp = 0;
-    __device__ __forceinline__ WarpStackSmem(int* r, uint32_t* k) : ref(r), key(k) {}
-    __device__ __forceinline__ void push(int r, uint32_t k) {
-        __syncwarp();   // earlier reads of the slot are done
-        if ((threadIdx.x & 31) == 0) { ref[sp] = r; key[sp] = k; }
-        ++sp;
-        __syncwarp();
-    }
-    __device__ __forceinline__ bool next(uint32_t cullmax, int& cur) {
-        while (sp > 0) {
-            --sp;
-            const int r = ref[sp];
-            const uint32_t k = key[sp];
-            if (k <= cullmax) { cur = r; return true; }
-        }
-        return false;
-    }
-};
-
 // ------------------------------------------------------- expanded records
 // One thread per (node, child): the child's box as floats (layout.h, WNode).
 __global__ void k_expand_nodes(int64_t n, const CNode* __restrict__ nodes, const CTri* __restrict__ tris,
@@ -1697,37 +1591,164 @@ __device__ __forceinline__ int64_t packet_ray(int64_t pk, int lane, int64_t n, c
     const int64_t slot = pk * (32 / kUnit) + lane / kUnit;
     return slot < units ? (int64_t)__ldg(order + slot) * kUnit + lane % kUnit : n;
 }
-// A packet is traced as a packet only when its rays are nearly parallel
-// (unit directions within kCohDir, max-norm, of one another's: about 6
-// degrees) and start close together (origins within kCohOrigin of the root
-// box's extent), as k_ray_order judges it; the others go to k_ray_lanes,
-// where each ray walks alone: the union of 32 unrelated walks costs far more
-// than their longest one.
-constexpr float kCohDir = 0.1f;
+// A packet is traced as a packet only when the rays of each unit are all but
+// parallel (unit directions within kCohDir, max-norm: half a degree), its
+// units' nearly so (kCohUnits) and they start close together (origins within
+// kCohOrigin of the root box's extent), as k_ray_order judges it; the others
+// go to k_ray_lanes, where each ray walks alone.  k_ray bounds a unit's rays
+// by intervals, which keep ever more nodes that no ray needs as the unit
+// spreads: 4 cameras x 1024^2 with directions jittered by 0.5 / 1 / 2 degrees
+// take 2.0 / 1.6 / 1.8 ms with the limit at 0.01 and 3.5 / 10 / 25 ms at
+// 0.1; exact cameras of 2048^2 pixels 3.11 against 3.10 ms, and 3.2 at 0.005.
+constexpr float kCohDir = 0.008f;
+constexpr float kCohUnits = 0.03f;
 constexpr float kCohOrigin = 0.01f;
+// The reciprocal of a direction component for the node tests: a component
+// that is zero, or too small for its reciprocal to be a number, counts as one
+// that moves by 1e-30 a unit.
+__device__ __forceinline__ float slab_inv(float d, float sign) {
+    return fabsf(d) > 1e-30f ? 1.0f / d : copysignf(1e30f, sign);
+}
+// One axis of the node tests of a lane's eight rays, in two halves of four
+// (a pair of values each): what the halves' origins lie within and their
+// directions' reciprocals.  kind: 0 all directions positive (or all zero), 1
+// all negative, 2 otherwise.
+struct RayAxis { f2 on, of, i0, i1; int kind; };
+// The axis of the lane's quad of rays and the other quad of its group of
+// eight, from o, d of the lane's ray (ok: the lane has one).
+__device__ __forceinline__ RayAxis ray_axis(float o, float d, bool ok) {
+    float o0 = ok ? o : CUDART_INF_F, o1 = ok ? o : -CUDART_INF_F;
+    float d0 = ok ? d : CUDART_INF_F, d1 = ok ? d : -CUDART_INF_F;
+#pragma unroll
+    for (int s = 1; s < 4; s <<= 1) {
+        o0 = fminf(o0, __shfl_xor_sync(kFull, o0, s));
+        o1 = fmaxf(o1, __shfl_xor_sync(kFull, o1, s));
+        d0 = fminf(d0, __shfl_xor_sync(kFull, d0, s));
+        d1 = fmaxf(d1, __shfl_xor_sync(kFull, d1, s));
+    }
+    const int own = d0 > 0.f || (d0 == 0.f && d1 == 0.f) ? 0 : (d1 < 0.f ? 1 : 2);
+    RayAxis r;
+    r.kind = own == __shfl_xor_sync(kFull, own, 4) ? own : 2;
+    float on, of, i0, i1;
+    if (r.kind == 2) {   // reached upwards from o1 by the largest direction, downwards from o0 by the smallest
+        on = o1; of = o0;
+        i0 = d1 > 0.f ? slab_inv(d1, 1.f) : 1e30f;
+        i1 = d0 < 0.f ? slab_inv(d0, -1.f) : -1e30f;
+    } else {
+        on = r.kind == 0 ? o1 : o0;
+        of = r.kind == 0 ? o0 : o1;
+        const float sg = r.kind == 0 ? 1.f : -1.f;
+        i0 = slab_inv(d0, sg);
+        i1 = slab_inv(d1, sg);
+    }
+    r.on = f2pack(-on, -__shfl_xor_sync(kFull, on, 4));   // negated
+    r.of = f2pack(-of, -__shfl_xor_sync(kFull, of, 4));
+    r.i0 = f2pack(i0, __shfl_xor_sync(kFull, i0, 4));
+    r.i1 = f2pack(i1, __shfl_xor_sync(kFull, i1, 4));
+    return r;
+}
+// Bounds of the parameter at which rays of either half lie between the box
+// planes lo and hi of the axis: no ray enters before tn or leaves after tf.
+// MIXED: kind 2 may occur.
+template <bool MIXED>
+__device__ __forceinline__ void axis_slab(const RayAxis& r, float lo, float hi, float tn[2], float tf[2]) {
+    const bool neg = r.kind == 1;
+    const float near = neg ? hi : lo, far = neg ? lo : hi;
+    const f2 A = f2add(f2pack(near, near), r.on), B = f2add(f2pack(far, far), r.of);
+    float p[2], q[2], u[2], v[2];
+    f2unpack(f2mul(A, r.i0), p[0], p[1]);
+    f2unpack(f2mul(A, r.i1), q[0], q[1]);
+    f2unpack(f2mul(B, r.i0), u[0], u[1]);
+    f2unpack(f2mul(B, r.i1), v[0], v[1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        tn[h] = fminf(p[h], q[h]);
+        tf[h] = fmaxf(u[h], v[h]);
+        if (MIXED && r.kind == 2) { tn[h] = fmaxf(p[h], v[h]); tf[h] = CUDART_INF_F; }
+    }
+}
+// Entry bound (ordered bits of max(tn, 0)) of the lane's eight rays into the
+// box, kFull when no half needs it within its bound c[h].  As in box_ray the
+// bounds are widened by 1e-6 relative for their roundings, here by products
+// that keep infinities: an unused child has tn = inf, tf = -inf.
+template <bool MIXED>
+__device__ __forceinline__ uint32_t group_entry(const RayAxis& X, const RayAxis& Y, const RayAxis& Z, float4 lo,
+                                                float4 hi, const float c[2]) {
+    float xn[2], xf[2], yn[2], yf[2], zn[2], zf[2];
+    axis_slab<MIXED>(X, lo.x, hi.x, xn, xf);
+    axis_slab<MIXED>(Y, lo.y, hi.y, yn, yf);
+    axis_slab<MIXED>(Z, lo.z, hi.z, zn, zf);
+    uint32_t key = kFull;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float tn = fmaxf(max3(xn[h], yn[h], zn[h]), 0.f) * 0.999999f;
+        const float tf = fminf(min3(xf[h], yf[h], zf[h]) * 1.000001f, c[h]);
+        if (tn <= tf) key = min(key, __float_as_uint(tn));
+    }
+    return key;
+}
+
+// A ray's closest hit by a walk of its own in double, given a bound U of it:
+// for a ray with more triangles at almost the same hit than its list holds.
+__device__ __noinline__ void walk_hits(const CNode* __restrict__ nodes, const CTri* __restrict__ tris, float3 o,
+                                       float3 d, float U, double* bt, int* sx, int* ix) {
+    const float3 inv = ray_inv(d);
+    const bool degen = ray_degenerate(inv);
+    const float cull = U * 1.000002f;
+    int st[kStack];
+    int sp = 0;
+    st[sp++] = 0;
+    while (sp > 0) {
+        const int ref = st[--sp];
+        if (ref >= 0) {
+            const NodeView nd = load_node(nodes, ref);
+            if (degen) push_ray_children<true>(nd, o, inv, cull, st, sp);
+            else push_ray_children<false>(nd, o, inv, cull, st, sp);
+        } else {
+            int s0, s1;
+            leaf_range(ref, s0, s1);
+            for (int s = s0; s < s1; ++s) {
+                const TriV t = load_tri(tris, s);
+                double t64;
+                if (!ray_tri_d(to_d3(o), to_d3(d), to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
+                if (t64 < *bt || (t64 == *bt && (*sx < 0 || t.id < *ix))) { *bt = t64; *sx = s; *ix = t.id; }
+            }
+        }
+    }
+}
+
+constexpr int kRayBlocks = 8;   // blocks of k_ray per SM
 // Closest hit of 32 rays per warp (a packet: the rays of 4 consecutive
 // entries of `order`, units of 8 consecutive rays sorted so that nearby ones
 // are side by side (k_ray_order); packets k_ray_order marked incoherent are
-// skipped, k_ray_lanes traces them):
-// warp-uniform walk of
-// the union of the rays' paths, children in the order of the smallest entry
-// distance of any ray that needs them.  Each lane keeps U, an upper bound of
-// its closest hit (certain FP32 hits: t + error bound), and a short list of
+// skipped, k_ray_lanes traces them, as it does packets holding a ray that is
+// not finite or has no direction, listed here): warp-uniform walk of the
+// union of the rays' paths.  At an inner node lane 8 g + j tests child j
+// against unit g in interval arithmetic: what its two halves' origins and
+// directions lie within against the box's planes (group_entry).  Eight
+// neighbouring pixels sweep nearly what they hit, so this keeps few children
+// that no ray needs, for about 100 instructions a node where a test per ray
+// and child with eight warp minima took 350 (33.5M camera rays on 82k faces:
+// 5.46 -> 3.11 ms a call; 32 warps per SM, 16 would be 20 % slower).  Children go onto the warp's
+// stack farthest entry first.  Each lane keeps U, an upper bound of its
+// closest hit (certain FP32 hits: t + error bound), and a short list of
 // triangles that may still be closer (certain or undecided hits whose lower
 // bound is within U); the list is settled in double at the end: exact t of
 // the closest hit, ties -> lowest face index.
-__global__ void __launch_bounds__(kQBlock) k_ray(int64_t n, const uint32_t* __restrict__ order,
+__global__ void __launch_bounds__(kQBlock, kRayBlocks) k_ray(int64_t n, const uint32_t* __restrict__ order,
                                                  const float* __restrict__ ro,
                                                  const float* __restrict__ rd, float* __restrict__ pos,
                                                  int64_t* __restrict__ face_id, float* __restrict__ depth,
-                                                 const CNode* __restrict__ nodes, const CTri* __restrict__ tris,
-                                                 unsigned long long* __restrict__ ctr, int64_t grab,
-                                                 const uint8_t* __restrict__ skip) {
+                                                 const DeviceTree tree, unsigned long long* __restrict__ ctr,
+                                                 int64_t grab, const uint8_t* __restrict__ skip,
+                                                 uint32_t* __restrict__ lanes,
+                                                 unsigned long long* __restrict__ lanes_n) {
+    const CTri* __restrict__ tris = tree.tris;
     const int lane = threadIdx.x & 31;
-    __shared__ __align__(16) float s_box[kQBlock / 32][64];
-    float* sb = s_box[threadIdx.x >> 5];
-    __shared__ int s_sref[kQBlock / 32][kSmemStack];
-    __shared__ uint32_t s_skey[kQBlock / 32][kSmemStack];
+    __shared__ uint2 s_stack[kQBlock / 32][kStack];
+    __shared__ uint2 s_cand[kQBlock / 32][kCand][32];
+    uint2* stk = s_stack[threadIdx.x >> 5];
+    uint2* cand = &s_cand[threadIdx.x >> 5][0][lane];   // the lane's candidates, 32 entries apart: slot, lower bound
     PacketQueue pq(ctr, (n + 31) >> 5, grab);
     for (int64_t pk = pq.take(); pk >= 0; pk = pq.take()) {
         if (__ldg(skip + pk)) continue;   // incoherent: k_ray_lanes traces it
@@ -1735,79 +1756,95 @@ __global__ void __launch_bounds__(kQBlock) k_ray(int64_t n, const uint32_t* __re
         const bool act = q < n;
         const float3 o = act ? load3(ro, q) : make_float3(0.f, 0.f, 0.f);
         const float3 d = act ? load3(rd, q) : make_float3(1.f, 1.f, 1.f);
-        const float3 inv = ray_inv(d);
-        const bool degen = __any_sync(kFull, act && ray_degenerate(inv));  // warp-uniform
         const float dinf = f3inf(d);
-        const d3 od = to_d3(o), dd = to_d3(d);
+        const bool odd = !(f3inf(o) < CUDART_INF_F && dinf > 0.f && dinf < CUDART_INF_F);   // NaN: odd
+        if (__any_sync(kFull, odd)) {
+            if (lane == 0) lanes[atomicAdd(lanes_n, 1ull)] = (uint32_t)pk;
+            continue;
+        }
+        const RayAxis X = ray_axis(o.x, d.x, act), Y = ray_axis(o.y, d.y, act), Z = ray_axis(o.z, d.z, act);
+        const bool mixed = __any_sync(kFull, X.kind == 2 || Y.kind == 2 || Z.kind == 2);
         float U = act ? 1000.0f : -1.f;             // MAX_DIST
-        float cull = act ? U * 1.000002f : -1.f;
-        int cs[kCand];
-        float cl[kCand];
-        int nc = 0;
-        double bt = 1000.0;
-        int sx = -1, ix = -1;
-        auto flush = [&](bool final_pass) {
-            for (int i = 0; i < nc; ++i) {
-                if (final_pass && cl[i] > U) continue;
-                const TriV t = load_tri(tris, cs[i]);
-                double t64;
-                if (!ray_tri_d(od, dd, to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
-                if (t64 < bt || (t64 == bt && (sx < 0 || t.id < ix))) { bt = t64; sx = cs[i]; ix = t.id; }
-            }
-            nc = 0;
+        float c[2];                                 // bounds of the lane's quad and of the other one
+        uint32_t cullmax;
+        auto share_bounds = [&]() {
+            float m = act ? U * 1.000002f : -1.f;
+            cullmax = __reduce_max_sync(kFull, __float_as_uint(fmaxf(m, 0.f)));
+            m = fmaxf(m, __shfl_xor_sync(kFull, m, 1));
+            c[0] = fmaxf(m, __shfl_xor_sync(kFull, m, 2));
+            c[1] = __shfl_xor_sync(kFull, c[0], 4);
         };
-        uint32_t cullmax = __reduce_max_sync(kFull, __float_as_uint(fmaxf(cull, 0.f)));
-        WarpStackSmem st(s_sref[threadIdx.x >> 5], s_skey[threadIdx.x >> 5]);
-        int cur = 0;
-        bool live = __any_sync(kFull, act);
+        share_bounds();
+        int nc = 0, sp = 0, cur = 0;
+        bool live = true;
         while (live) {
             if (cur >= 0) {
-                const NodeLinks nd = decode_node_warp(nodes, cur, sb);
-                uint32_t k[8];
-                if (degen) ray_child_keys<true>(nd, sb, o, inv, cull, k);
-                else ray_child_keys<false>(nd, sb, o, inv, cull, k);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint32_t kmin = __reduce_min_sync(kFull, k[j]);
-                    k[j] = kmin != kFull ? ((kmin & ~7u) | (uint32_t)j) : kFull;
-                }
-                sort8(k);
-#pragma unroll
-                for (int i = 7; i >= 1; --i)
-                    if (k[i] != kFull) st.push(child_ref(nd, meta_of(nd, (int)(k[i] & 7u))), k[i] & ~7u);
-                if (k[0] != kFull) cur = child_ref(nd, meta_of(nd, (int)(k[0] & 7u)));
-                else live = st.next(cullmax, cur);
+                const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + cur);
+                const int j = lane & 7;
+                const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
+                uint32_t key = mixed ? group_entry<true>(X, Y, Z, lo, hi, c) : group_entry<false>(X, Y, Z, lo, hi, c);
+                key = min(key, __shfl_xor_sync(kFull, key, 8));
+                key = min(key, __shfl_xor_sync(kFull, key, 16));
+                if (key != kFull) key = (key & ~7u) | (uint32_t)j;
+                // its place on the stack: the number of needed children farther than it, two of
+                // the eight compared by each of the four lanes with this child
+                const uint32_t ka = __shfl_sync(kFull, key, 2 * (lane >> 3)), kb = __shfl_sync(kFull, key, 2 * (lane >> 3) + 1);
+                int place = (ka > key && ka != kFull ? 1 : 0) + (kb > key && kb != kFull ? 1 : 0);
+                place += __shfl_xor_sync(kFull, place, 8);
+                place += __shfl_xor_sync(kFull, place, 16);
+                const int kept = __popc(__ballot_sync(kFull, key != kFull) & 0xFFu);
+                __syncwarp();   // the popped entry has been read
+                if (lane < 8 && key != kFull) stk[sp + place] = make_uint2((uint32_t)__float_as_int(lo.w), key & ~7u);
+                sp += kept;
+                __syncwarp();
             } else {
                 int s0, s1;
                 leaf_range(cur, s0, s1);
-                load_leaf_warp(tris, s0, s1, sb);
+                const float U0 = U;
                 for (int s = s0; s < s1; ++s) {
-                    const TriV t = warp_tri(sb, s - s0);
+                    const TriV t = load_tri(tris, s);
                     float tt, terr;
                     const int r = ray_tri_f(o, d, dinf, t, 1000.0f, &tt, &terr);
                     const float lb = tt - terr;
                     if (act && r != 0 && lb <= U) {
                         if (r == 1) U = fminf(U, tt + terr);
-                        if (nc == kCand) {
+                        if (nc == kCand) {   // keep only live candidates
                             int m = 0;
-                            for (int i = 0; i < nc; ++i)
-                                if (cl[i] <= U) { cs[m] = cs[i]; cl[m] = cl[i]; ++m; }
-                            nc = m;
-                            if (nc == kCand) {
-                                flush(false);
-                                if (sx >= 0) U = fminf(U, __double2float_ru(bt));
-                            }
+                            for (int i = 0; i < kCand; ++i)
+                                if (__uint_as_float(cand[32 * i].y) <= U) { cand[32 * m] = cand[32 * i]; ++m; }
+                            nc = m < kCand ? m : kCand + 1;
                         }
-                        cs[nc] = s; cl[nc] = lb; ++nc;
+                        if (nc < kCand) {
+                            cand[32 * nc] = make_uint2((uint32_t)s, __float_as_uint(lb));
+                            ++nc;
+                        }   // else the list has overflowed (nc = kCand + 1)
                     }
                 }
-                cull = act ? U * 1.000002f : -1.f;
-                cullmax = __reduce_max_sync(kFull, __float_as_uint(fmaxf(cull, 0.f)));
-                live = st.next(cullmax, cur);
+                if (__any_sync(kFull, U < U0)) share_bounds();
+            }
+            // the next entry that some ray still needs
+            live = false;
+            while (sp > 0) {
+                const uint2 e = stk[--sp];
+                if (e.y <= cullmax) { cur = (int)e.x; live = true; break; }
             }
         }
         if (!act) continue;
-        flush(true);
+        double bt = 1000.0;
+        int sx = -1, ix = -1;
+        if (nc > kCand) {
+            walk_hits(tree.nodes, tris, o, d, U, &bt, &sx, &ix);
+            nc = 0;
+        }
+        const d3 od = to_d3(o), dd = to_d3(d);
+        for (int i = 0; i < nc; ++i) {
+            const uint2 e = cand[32 * i];
+            if (__uint_as_float(e.y) > U) continue;
+            const TriV t = load_tri(tris, (int)e.x);
+            double t64;
+            if (!ray_tri_d(od, dd, to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
+            if (t64 < bt || (t64 == bt && (sx < 0 || t.id < ix))) { bt = t64; sx = (int)e.x; ix = t.id; }
+        }
         depth[q] = __double2float_rn(bt);
         pos[3 * q] = __double2float_rn(dA((double)o.x, dM(bt, (double)d.x)));
         pos[3 * q + 1] = __double2float_rn(dA((double)o.y, dM(bt, (double)d.y)));
@@ -2042,7 +2079,7 @@ __device__ __forceinline__ int ray_entry(float3 o, float3 d, const float lo[3], 
 // window (4 consecutive sorted units) is judged: coherent when each unit's
 // first and last rays lie within kCohDir (unit directions, max-norm) and
 // kCohOrigin (origins) of the unit's fourth ray, and each unit's fourth ray
-// within the same of the first unit's.  skip[p] = 1 marks the others for
+// within kCohUnits and kCohOrigin of the first unit's.  skip[p] = 1 marks the others for
 // k_ray, and they are listed for k_ray_lanes.
 __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const float* __restrict__ ro,
                                                            const float* __restrict__ rd,
@@ -2149,7 +2186,7 @@ __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const floa
                 dv = fmaxf(dv, fabsf(s_ray[v][k] - s_ray[f][k]));
                 dov = fmaxf(dov, fabsf(s_ray[v][3 + k] - s_ray[f][3 + k]));
             }
-            inc |= s_bad[v] || !(dv <= kCohDir && dov <= spread_max);
+            inc |= s_bad[v] || !(dv <= kCohUnits && dov <= spread_max);
         }
         skip[pk] = inc ? 1 : 0;
     }
@@ -2421,8 +2458,10 @@ cudaError_t launch_near_lists(int64_t n_tris, const CNode* nodes, const CTri* tr
 }
 
 cudaError_t launch_ray(int64_t n, const float* ro, const float* rd, float* pos, int64_t* fid, float* depth,
-                       const CNode* nodes, const CTri* tris, void* ws, cudaStream_t stream) {
+                       const DeviceTree& tree, void* ws, cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
+    const CNode* nodes = tree.nodes;
+    const CTri* tris = tree.tris;
     unsigned long long* ctr = reinterpret_cast<unsigned long long*>(ws);
     cudaError_t e = cudaMemsetAsync(ctr, 0, 256, stream);
     if (e != cudaSuccess) return e;
@@ -2435,8 +2474,8 @@ cudaError_t launch_ray(int64_t n, const float* ro, const float* rd, float* pos, 
     k_ray_order<<<(unsigned)((units + kOrdUnits - 1) / kOrdUnits), kOrdThreads, 0, stream>>>(
         n, ro, rd, nodes, order, skip, lanes, ctr + kCtRayLanesN); count_launch();
     const unsigned g = persistent_grid(k_ray, n);
-    k_ray<<<g, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, nodes, tris, ctr + kCtUdf, grab_for(n, g),
-                                     skip); count_launch();
+    k_ray<<<g, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, tree, ctr + kCtUdf, grab_for(n, g), skip, lanes,
+                                     ctr + kCtRayLanesN); count_launch();
     const unsigned gl = persistent_grid(k_ray_lanes, n);
     k_ray_lanes<<<gl, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, nodes, tris, lanes,
                                             ctr + kCtRayLanesN, ctr + kCtRayLanesNext); count_launch();
