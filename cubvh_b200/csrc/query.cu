@@ -58,9 +58,56 @@ template <class N>
 __device__ __forceinline__ uint32_t meta_of(const N& n, int j) {
     return ((j < 4 ? n.meta0 : n.meta1) >> (8 * (j & 3))) & 0xFFu;
 }
+// Pairs of floats in one 64-bit register and the packed operations on them
+// (two results per issued instruction), and the three-input maximum.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2unpack(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 f2add(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2mul(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 f2fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ f2 f2max3(f2 a, f2 b, float c) {
+    float a0, a1, b0, b1;
+    f2unpack(a, a0, a1);
+    f2unpack(b, b0, b1);
+    return f2pack(max3(a0, b0, c), max3(a1, b1, c));
+}
+
 // byte k of w as a float: 0x4B0000qq is 2^23 + q, minus 2^23 is q exactly
 __device__ __forceinline__ float qbyte(uint32_t w, int k) {
     return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u + (unsigned)k)) - 8388608.0f;
+}
+// bytes k and k + 1 of w as floats
+__device__ __forceinline__ f2 qpair(uint32_t w, int k) {
+    const f2 q = f2pack(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u + (unsigned)k)),
+                        __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7541u + (unsigned)k)));
+    return f2add(q, f2pack(-8388608.0f, -8388608.0f));
 }
 // origin + q * 2^e: exact product, one rounding (same as the host check)
 __device__ __forceinline__ void child_box(const NodeView& n, int j, float3& lo, float3& hi) {
@@ -164,32 +211,56 @@ __device__ __forceinline__ void push_ray_children(const NodeView& nd, float3 o, 
 // with B_a - E_a and exits with B_a + E_a, E_a = 1e-6 * S_a (about 16 * 2^-24
 // * S_a).  The ray's direction signs fix which of a child's two planes is
 // the near one on each axis, so no per-child min / max is needed.
-__device__ __forceinline__ void push_ray_children_affine(const NodeView& nd, float3 o, float3 inv, float cull,
-                                                         int* st, int& sp) {
+struct AffineNode { f2 ax, ay, az, nbx, fbx, nby, fby, nbz, fbz; uint32_t nx[2], fx[2], ny[2], fy[2], nz[2], fz[2]; };
+__device__ __forceinline__ AffineNode affine_node(const NodeView& nd, float3 o, float3 inv) {
     const float ax = nd.sx * inv.x, ay = nd.sy * inv.y, az = nd.sz * inv.z;
     const float bx = (nd.ox - o.x) * inv.x, by = (nd.oy - o.y) * inv.y, bz = (nd.oz - o.z) * inv.z;
     const float ex = 1e-6f * (fabsf(nd.ox * inv.x) + 255.f * fabsf(ax) + fabsf(bx));
     const float ey = 1e-6f * (fabsf(nd.oy * inv.y) + 255.f * fabsf(ay) + fabsf(by));
     const float ez = 1e-6f * (fabsf(nd.oz * inv.z) + 255.f * fabsf(az) + fabsf(bz));
-    const float nbx = bx - ex, fbx = bx + ex, nby = by - ey, fby = by + ey, nbz = bz - ez, fbz = bz + ez;
     const bool px = inv.x >= 0.f, py = inv.y >= 0.f, pz = inv.z >= 0.f;
+    AffineNode a;
+    a.ax = f2pack(ax, ax); a.ay = f2pack(ay, ay); a.az = f2pack(az, az);
+    a.nbx = f2pack(bx - ex, bx - ex); a.fbx = f2pack(bx + ex, bx + ex);
+    a.nby = f2pack(by - ey, by - ey); a.fby = f2pack(by + ey, by + ey);
+    a.nbz = f2pack(bz - ez, bz - ez); a.fbz = f2pack(bz + ez, bz + ez);
     // near / far quantised words per axis (children 0-3, 4-7)
-    const uint32_t nx0 = px ? nd.lx0 : nd.hx0, nx1 = px ? nd.lx1 : nd.hx1;
-    const uint32_t fx0 = px ? nd.hx0 : nd.lx0, fx1 = px ? nd.hx1 : nd.lx1;
-    const uint32_t ny0 = py ? nd.ly0 : nd.hy0, ny1 = py ? nd.ly1 : nd.hy1;
-    const uint32_t fy0 = py ? nd.hy0 : nd.ly0, fy1 = py ? nd.hy1 : nd.ly1;
-    const uint32_t nz0 = pz ? nd.lz0 : nd.hz0, nz1 = pz ? nd.lz1 : nd.hz1;
-    const uint32_t fz0 = pz ? nd.hz0 : nd.lz0, fz1 = pz ? nd.hz1 : nd.lz1;
+    a.nx[0] = px ? nd.lx0 : nd.hx0; a.nx[1] = px ? nd.lx1 : nd.hx1;
+    a.fx[0] = px ? nd.hx0 : nd.lx0; a.fx[1] = px ? nd.hx1 : nd.lx1;
+    a.ny[0] = py ? nd.ly0 : nd.hy0; a.ny[1] = py ? nd.ly1 : nd.hy1;
+    a.fy[0] = py ? nd.hy0 : nd.ly0; a.fy[1] = py ? nd.hy1 : nd.ly1;
+    a.nz[0] = pz ? nd.lz0 : nd.hz0; a.nz[1] = pz ? nd.lz1 : nd.hz1;
+    a.fz[0] = pz ? nd.hz0 : nd.lz0; a.fz[1] = pz ? nd.hz1 : nd.lz1;
+    return a;
+}
+// Entry and exit (at most cull) of the ray in children 2 c and 2 c + 1:
+// entered where entry <= exit and 0 <= exit (never by a ray that is no number).
+__device__ __forceinline__ void affine_pair(const AffineNode& a, int c, float cull, float tn[2], float tf[2]) {
+    const int h = c >> 1, b = 2 * (c & 1);
+    float x0, x1, y0, y1, z0, z1;
+    f2unpack(f2fma(qpair(a.nx[h], b), a.ax, a.nbx), x0, x1);
+    f2unpack(f2fma(qpair(a.ny[h], b), a.ay, a.nby), y0, y1);
+    f2unpack(f2fma(qpair(a.nz[h], b), a.az, a.nbz), z0, z1);
+    tn[0] = max3(x0, y0, z0);
+    tn[1] = max3(x1, y1, z1);
+    f2unpack(f2fma(qpair(a.fx[h], b), a.ax, a.fbx), x0, x1);
+    f2unpack(f2fma(qpair(a.fy[h], b), a.ay, a.fby), y0, y1);
+    f2unpack(f2fma(qpair(a.fz[h], b), a.az, a.fbz), z0, z1);
+    tf[0] = fminf(min3(x0, y0, z0), cull);
+    tf[1] = fminf(min3(x1, y1, z1), cull);
+}
+__device__ __forceinline__ void push_ray_children_affine(const NodeView& nd, float3 o, float3 inv, float cull,
+                                                         int* st, int& sp) {
+    const AffineNode a = affine_node(nd, o, inv);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const uint32_t m = meta_of(nd, j);
-        const int b = j & 3;
-        const bool h = j >= 4;
-        const float tn = fmaxf(fmaxf(fmaf(qbyte(h ? nx1 : nx0, b), ax, nbx), fmaf(qbyte(h ? ny1 : ny0, b), ay, nby)),
-                               fmaf(qbyte(h ? nz1 : nz0, b), az, nbz));
-        const float tf = fminf(fminf(fmaf(qbyte(h ? fx1 : fx0, b), ax, fbx), fmaf(qbyte(h ? fy1 : fy0, b), ay, fby)),
-                               fmaf(qbyte(h ? fz1 : fz0, b), az, fbz));
-        if (m != kEmpty && tn <= tf && tf >= 0.f && tn <= cull) st[sp++] = child_ref(nd, m);
+    for (int c = 0; c < 4; ++c) {
+        float tn[2], tf[2];
+        affine_pair(a, c, cull, tn, tf);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t m = meta_of(nd, 2 * c + i);
+            if (m != kEmpty && tn[i] <= tf[i] && tf[i] >= 0.f) st[sp++] = child_ref(nd, m);
+        }
     }
 }
 
@@ -213,30 +284,17 @@ __device__ __forceinline__ void lane_child_keys(const NodeView& nd, float3 o, fl
         }
         return;
     }
-    const float ax = nd.sx * inv.x, ay = nd.sy * inv.y, az = nd.sz * inv.z;
-    const float bx = (nd.ox - o.x) * inv.x, by = (nd.oy - o.y) * inv.y, bz = (nd.oz - o.z) * inv.z;
-    const float ex = 1e-6f * (fabsf(nd.ox * inv.x) + 255.f * fabsf(ax) + fabsf(bx));
-    const float ey = 1e-6f * (fabsf(nd.oy * inv.y) + 255.f * fabsf(ay) + fabsf(by));
-    const float ez = 1e-6f * (fabsf(nd.oz * inv.z) + 255.f * fabsf(az) + fabsf(bz));
-    const float nbx = bx - ex, fbx = bx + ex, nby = by - ey, fby = by + ey, nbz = bz - ez, fbz = bz + ez;
-    const bool px = inv.x >= 0.f, py = inv.y >= 0.f, pz = inv.z >= 0.f;
-    const uint32_t nx0 = px ? nd.lx0 : nd.hx0, nx1 = px ? nd.lx1 : nd.hx1;
-    const uint32_t fx0 = px ? nd.hx0 : nd.lx0, fx1 = px ? nd.hx1 : nd.lx1;
-    const uint32_t ny0 = py ? nd.ly0 : nd.hy0, ny1 = py ? nd.ly1 : nd.hy1;
-    const uint32_t fy0 = py ? nd.hy0 : nd.ly0, fy1 = py ? nd.hy1 : nd.ly1;
-    const uint32_t nz0 = pz ? nd.lz0 : nd.hz0, nz1 = pz ? nd.lz1 : nd.hz1;
-    const uint32_t fz0 = pz ? nd.hz0 : nd.lz0, fz1 = pz ? nd.hz1 : nd.lz1;
+    const AffineNode a = affine_node(nd, o, inv);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int b = j & 3;
-        const bool h = j >= 4;
-        const float tn = fmaxf(fmaxf(fmaf(qbyte(h ? nx1 : nx0, b), ax, nbx), fmaf(qbyte(h ? ny1 : ny0, b), ay, nby)),
-                               fmaf(qbyte(h ? nz1 : nz0, b), az, nbz));
-        const float tf = fminf(fminf(fmaf(qbyte(h ? fx1 : fx0, b), ax, fbx), fmaf(qbyte(h ? fy1 : fy0, b), ay, fby)),
-                               fmaf(qbyte(h ? fz1 : fz0, b), az, fbz));
-        const float key = fmaxf(tn, 0.f);
-        const bool need = meta_of(nd, j) != kEmpty && tn <= tf && tf >= 0.f && key <= cull;
-        k[j] = need ? ((__float_as_uint(key) & ~7u) | (uint32_t)j) : kFull;
+    for (int c = 0; c < 4; ++c) {
+        float tn[2], tf[2];
+        affine_pair(a, c, cull, tn, tf);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int j = 2 * c + i;
+            const bool need = meta_of(nd, j) != kEmpty && tn[i] <= tf[i] && tf[i] >= 0.f;
+            k[j] = need ? ((__float_as_uint(fmaxf(tn[i], 0.f)) & ~7u) | (uint32_t)j) : kFull;
+        }
     }
 }
 __device__ __forceinline__ float cull_of(double best) { return __double2float_ru(dM(best, 1.000001)); }
@@ -444,47 +502,6 @@ cudaError_t launch_expand(int64_t n_nodes, int64_t n_tris, const CNode* nodes, c
     if (n_nodes > 0) { k_expand_nodes<<<(unsigned)((8 * n_nodes + 255) / 256), 256, 0, stream>>>(n_nodes, nodes, tris, wnodes); count_launch(); }
     if (n_tris > 0) { k_expand_tris<<<(unsigned)((n_tris + 127) / 128), 128, 0, stream>>>(n_tris, tris, wtris); count_launch(); }
     return cudaGetLastError();
-}
-
-// Pairs of floats in one 64-bit register and the packed operations on them
-// (two results per issued instruction), and the three-input maximum.
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 f2pack(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2unpack(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f2 f2add(f2 a, f2 b) {
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2mul(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2fma(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-__device__ __forceinline__ float min3(float a, float b, float c) {
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-}
-__device__ __forceinline__ f2 f2max3(f2 a, f2 b, float c) {
-    float a0, a1, b0, b1;
-    f2unpack(a, a0, a1);
-    f2unpack(b, b0, b1);
-    return f2pack(max3(a0, b0, c), max3(a1, b1, c));
 }
 
 __device__ __forceinline__ TriW make_triw(float4 w0, float4 w1, float4 w2, float4 w3) {
@@ -1923,13 +1940,24 @@ __global__ void k_cell_scatter(int64_t n, const float* __restrict__ pts, const u
         order[atomicAdd(&offs[cell_of(load3(pts, i), box, bits)], 1u)] = (uint32_t)i;
 }
 
-// Closest hit of the rays of the incoherent packets k_ray listed: a warp
-// takes a packet, and each lane walks its own ray alone (own stack in local
-// memory, children nearest first, a child popped only while its entry
-// distance is within the lane's bound U).  A step is one node or one leaf.
-// Filters, candidate list and the FP64 settlement are k_ray's, so every
-// result is the one k_ray would give.
-__global__ void __launch_bounds__(kQBlock) k_ray_lanes(int64_t n, const uint32_t* __restrict__ order,
+constexpr int kLaneBlocks = 6;    // blocks of k_ray_lanes per SM
+constexpr int kLaneRefill = 16;   // idle lanes that make a warp finish them and take new rays
+constexpr int kLaneInner = 12;    // fewer lanes at inner nodes than this wait for those at leaves
+// Closest hit of the rays of the incoherent packets (k_ray_order and k_ray
+// list them): each lane walks its own ray alone (own stack in local memory,
+// children nearest first, a child popped only while its entry distance is
+// within the lane's bound U).  The warp keeps its lanes on the same kind of
+// step, inner nodes until few lanes are at one, then leaves; rays that ended
+// wait until kLaneRefill lanes are idle, which settle their hits in double
+// together and take the next rays of the warp's packet.  A warp that walked
+// its 32 rays to the longest one's end had 6.8 lanes active and took 497
+// instructions a ray; now 11.3 and 287, with two children an instruction in
+// affine_pair: 5M random rays on 82k faces 3.36 -> 2.32 ms a call (refill at
+// 8 or 4 idle lanes 3 and 9 % slower, leaves at once 13 %; what is left is
+// load latency and divergence).  Filters,
+// candidate list and the FP64 settlement are k_ray's, so every result is the
+// one k_ray would give.
+__global__ void __launch_bounds__(kQBlock, kLaneBlocks) k_ray_lanes(int64_t n, const uint32_t* __restrict__ order,
                                                        const float* __restrict__ ro, const float* __restrict__ rd,
                                                        float* __restrict__ pos, int64_t* __restrict__ face_id,
                                                        float* __restrict__ depth, const CNode* __restrict__ nodes,
@@ -1938,89 +1966,132 @@ __global__ void __launch_bounds__(kQBlock) k_ray_lanes(int64_t n, const uint32_t
                                                        const unsigned long long* __restrict__ lanes_n,
                                                        unsigned long long* __restrict__ next) {
     const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    __shared__ uint2 s_cand[kQBlock / 32][kCand][32];
+    uint2* cand = &s_cand[threadIdx.x >> 5][0][lane];   // the lane's candidates, 32 entries apart: slot, lower bound
     const unsigned long long count = *lanes_n;
-    int st_ref[kStack];
-    uint32_t st_key[kStack];
+    uint2 st[kStack];
+    int sp = 0, cur = 0, nc = 0;
+    bool live = false;                       // the lane's walk goes on
+    int64_t q = -1;                          // the lane's ray, -1: none
+    float3 o = make_float3(0.f, 0.f, 0.f), d = o, inv = o;
+    float dinf = 0.f, U = 0.f;
+    bool degen = false;
+    int64_t packet = -1;                     // the warp's packet, its next ray (32: used up), more may come
+    int from = 32;
+    bool more = true;
     while (true) {
-        unsigned long long c = 0;
-        if (lane == 0) c = atomicAdd(next, 1ull);
-        c = __shfl_sync(kFull, c, 0);
-        if (c >= count) break;
-        const int64_t q = packet_ray((int64_t)lanes[c], lane, n, order);
-        const bool act = q < n;
-        const float3 o = act ? load3(ro, q) : make_float3(0.f, 0.f, 0.f);
-        const float3 d = act ? load3(rd, q) : make_float3(1.f, 1.f, 1.f);
-        const float3 inv = ray_inv(d);
-        const bool degen = ray_degenerate(inv);
-        const float dinf = f3inf(d);
-        const d3 od = to_d3(o), dd = to_d3(d);
-        float U = 1000.0f;                          // MAX_DIST
-        float cull = U * 1.000002f;
-        int cs[kCand];
-        float cl[kCand];
-        int nc = 0;
-        double bt = 1000.0;
-        int sx = -1, ix = -1;
-        auto flush = [&](bool final_pass) {
-            for (int i = 0; i < nc; ++i) {
-                if (final_pass && cl[i] > U) continue;
-                const TriV t = load_tri(tris, cs[i]);
-                double t64;
-                if (!ray_tri_d(od, dd, to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
-                if (t64 < bt || (t64 == bt && (sx < 0 || t.id < ix))) { bt = t64; sx = cs[i]; ix = t.id; }
+        const unsigned idle = __ballot_sync(kFull, !live);
+        if (idle == kFull || (more && __popc(idle) >= kLaneRefill)) {
+            if (!live && q >= 0) {           // settle and write
+                double bt = 1000.0;
+                int sx = -1, ix = -1;
+                if (nc > kCand) {
+                    walk_hits(nodes, tris, o, d, U, &bt, &sx, &ix);
+                    nc = 0;
+                }
+                const d3 od = to_d3(o), dd = to_d3(d);
+                for (int i = 0; i < nc; ++i) {
+                    const uint2 e = cand[32 * i];
+                    if (__uint_as_float(e.y) > U) continue;
+                    const TriV t = load_tri(tris, (int)e.x);
+                    double t64;
+                    if (!ray_tri_d(od, dd, to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
+                    if (t64 < bt || (t64 == bt && (sx < 0 || t.id < ix))) { bt = t64; sx = (int)e.x; ix = t.id; }
+                }
+                depth[q] = __double2float_rn(bt);
+                pos[3 * q] = __double2float_rn(dA((double)o.x, dM(bt, (double)d.x)));
+                pos[3 * q + 1] = __double2float_rn(dA((double)o.y, dM(bt, (double)d.y)));
+                pos[3 * q + 2] = __double2float_rn(dA((double)o.z, dM(bt, (double)d.z)));
+                face_id[q] = sx >= 0 ? (int64_t)ix : (int64_t)-1;
+                q = -1;
             }
-            nc = 0;
-        };
-        int sp = 0, cur = 0;
-        bool live = act;
-        while (live) {
-            if (cur >= 0) {
+            __syncwarp();
+            if (from >= 32 && more) {        // the warp's next packet
+                unsigned long long c = 0;
+                if (lane == 0) c = atomicAdd(next, 1ull);
+                c = __shfl_sync(kFull, c, 0);
+                more = c < count;
+                if (more) { packet = (int64_t)__ldg(lanes + c); from = 0; }
+            }
+            if (from < 32) {
+                const int k = from + __popc(idle & lt);
+                if (!live && k < 32) {
+                    q = packet_ray(packet, k, n, order);
+                    if (q >= n) q = -1;
+                    if (q >= 0) {
+                        o = load3(ro, q);
+                        d = load3(rd, q);
+                        inv = ray_inv(d);
+                        degen = ray_degenerate(inv);
+                        dinf = f3inf(d);
+                        U = 1000.0f;         // MAX_DIST
+                        nc = sp = cur = 0;
+                        live = true;
+                    }
+                }
+                from = min(32, from + __popc(idle));
+            } else if (idle == kFull) {
+                break;                       // no ray left
+            }
+            continue;
+        }
+        // inner nodes
+        while (true) {
+            const unsigned in = __ballot_sync(kFull, live && cur >= 0);
+            if (!in || (__popc(in) < kLaneInner && __any_sync(kFull, live && cur < 0))) break;
+            if (live && cur >= 0) {
+                const float cull = U * 1.000002f;
                 const NodeView nd = load_node(nodes, cur);
                 uint32_t k[8];
                 lane_child_keys(nd, o, inv, degen, cull, k);
                 sort8(k);
 #pragma unroll
                 for (int i = 7; i >= 1; --i)
-                    if (k[i] != kFull) { st_ref[sp] = child_ref(nd, meta_of(nd, (int)(k[i] & 7u))); st_key[sp] = k[i] & ~7u; ++sp; }
-                if (k[0] != kFull) { cur = child_ref(nd, meta_of(nd, (int)(k[0] & 7u))); continue; }
-            } else {
-                int s0, s1;
-                leaf_range(cur, s0, s1);
-                for (int s = s0; s < s1; ++s) {
-                    const TriV t = load_tri(tris, s);
-                    float tt, terr;
-                    const int r = ray_tri_f(o, d, dinf, t, 1000.0f, &tt, &terr);
-                    const float lb = tt - terr;
-                    if (r != 0 && lb <= U) {
-                        if (r == 1) U = fminf(U, tt + terr);
-                        if (nc == kCand) {
-                            int m = 0;
-                            for (int i = 0; i < nc; ++i)
-                                if (cl[i] <= U) { cs[m] = cs[i]; cl[m] = cl[i]; ++m; }
-                            nc = m;
-                            if (nc == kCand) {
-                                flush(false);
-                                if (sx >= 0) U = fminf(U, __double2float_ru(bt));
-                            }
-                        }
-                        cs[nc] = s; cl[nc] = lb; ++nc;
+                    if (k[i] != kFull) st[sp++] = make_uint2((uint32_t)child_ref(nd, meta_of(nd, (int)(k[i] & 7u))), k[i] & ~7u);
+                if (k[0] != kFull) {
+                    cur = child_ref(nd, meta_of(nd, (int)(k[0] & 7u)));
+                } else {                     // the next entry whose box is still within the bound
+                    live = false;
+                    while (sp > 0) {
+                        const uint2 e = st[--sp];
+                        if (__uint_as_float(e.y) <= cull) { cur = (int)e.x; live = true; break; }
                     }
                 }
-                cull = U * 1.000002f;
             }
-            live = false;             // the next entry whose box is still within the bound
+            if (more && __popc(__ballot_sync(kFull, !live)) >= kLaneRefill) break;
+        }
+        // leaves
+        if (live && cur < 0) {
+            int s0, s1;
+            leaf_range(cur, s0, s1);
+            for (int s = s0; s < s1; ++s) {
+                const TriV t = load_tri(tris, s);
+                float tt, terr;
+                const int r = ray_tri_f(o, d, dinf, t, 1000.0f, &tt, &terr);
+                const float lb = tt - terr;
+                if (r != 0 && lb <= U) {
+                    if (r == 1) U = fminf(U, tt + terr);
+                    if (nc == kCand) {   // keep only live candidates
+                        int m = 0;
+                        for (int i = 0; i < kCand; ++i)
+                            if (__uint_as_float(cand[32 * i].y) <= U) { cand[32 * m] = cand[32 * i]; ++m; }
+                        nc = m < kCand ? m : kCand + 1;
+                    }
+                    if (nc < kCand) {
+                        cand[32 * nc] = make_uint2((uint32_t)s, __float_as_uint(lb));
+                        ++nc;
+                    }   // else the list has overflowed (nc = kCand + 1)
+                }
+            }
+            const float cull = U * 1.000002f;
+            live = false;
             while (sp > 0) {
-                --sp;
-                if (__uint_as_float(st_key[sp]) <= cull) { cur = st_ref[sp]; live = true; break; }
+                const uint2 e = st[--sp];
+                if (__uint_as_float(e.y) <= cull) { cur = (int)e.x; live = true; break; }
             }
         }
-        if (!act) continue;
-        flush(true);
-        depth[q] = __double2float_rn(bt);
-        pos[3 * q] = __double2float_rn(dA((double)o.x, dM(bt, (double)d.x)));
-        pos[3 * q + 1] = __double2float_rn(dA((double)o.y, dM(bt, (double)d.y)));
-        pos[3 * q + 2] = __double2float_rn(dA((double)o.z, dM(bt, (double)d.z)));
-        face_id[q] = sx >= 0 ? (int64_t)ix : (int64_t)-1;
+        __syncwarp();
     }
 }
 
