@@ -54,8 +54,9 @@ cudaError_t launch_arena_distance(const ArenaLaunch& a, const float* pts, float*
 int cell_bits_for(int64_t n);
 int64_t heavy_cap_for(int64_t n);
 
-// Point queries at least this many are visited in Morton-cell order.
-constexpr int64_t kSortMinQueries = 2048;
+// Calls with fewer point queries than this run eight lanes per query in their
+// own order (k_udf_few); the others visit packets in Morton-cell order.
+constexpr int64_t kFewQueries = 65536;
 
 // Device scratch bytes of a query launch: launch_distance (mode 0..2) or
 // launch_ray (mode -1) for n queries.

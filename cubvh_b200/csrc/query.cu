@@ -853,6 +853,156 @@ __device__ void heavy_settle(const HeavyWarp& S, int nc, float lim, const CTri* 
     if (s >= 0 && (e < bx || (e == bx && (sx < 0 || id < ix)))) { bx = e; sx = s; ix = id; }
 }
 
+// The walk of one query by the whole warp: the exact nearest triangle of p
+// under `root` into (bx, sx, ix), the same in every lane.  U: a bound of its
+// squared distance (negative: nothing can be found).
+__device__ void heavy_walk(HeavyWarp& S, const DeviceTree& tree, int root, float3 p, float U, double& bx, int& sx,
+                           int& ix) {
+    const CTri* __restrict__ tris = tree.tris;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    int nc = 0, sp = U >= 0.f ? 1 : 0;
+    U = fminf(1e6f, fmaxf(U, 0.f));   // MAX_DIST^2
+    bx = 1e6;
+    sx = -1;
+    ix = 0;
+    __syncwarp();  // the previous query is done with S
+    if (lane == 0) { S.ref[0] = root; S.key[0] = 0u; }
+    __syncwarp();
+    while (sp > 0) {
+        const float cull = U * 1.000002f;
+        // pop: of the top 32 entries, the first four (from the top) whose
+        // key is within the bound; the culled ones above them go too
+        const int pos = sp - 1 - lane;
+        const bool alive = pos >= 0 && S.key[pos] <= __float_as_uint(cull);
+        const unsigned m = __ballot_sync(kFull, alive);
+        int nn = __popc(m), used = sp < 32 ? sp : 32;
+        if (nn >= 4) {  // up to and including the fourth live entry
+            unsigned m4 = m;
+            m4 &= m4 - 1u;
+            m4 &= m4 - 1u;
+            m4 &= m4 - 1u;
+            used = __ffs(m4);
+            nn = 4;
+        }
+        if (alive && __popc(m & lt) < 4) S.pop[__popc(m & lt)] = S.ref[pos];
+        sp -= used;
+        __syncwarp();
+        // children of the popped nodes
+        const int ni = lane >> 3, j = lane & 7;
+        bool take = false, leaf = false;
+        int cref = 0;
+        uint32_t key = 0u;
+        if (ni < nn) {
+            const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + S.pop[ni]);
+            const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
+            const float d2 = box_d2(p, make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z));
+            if (d2 <= cull) {   // an unused child's box is infinitely far
+                take = true;
+                key = __float_as_uint(d2);
+                cref = __float_as_int(lo.w);
+                leaf = cref < 0;
+            }
+        }
+        const unsigned mi = __ballot_sync(kFull, take && !leaf);
+        if (take && !leaf) {
+            const int q = sp + __popc(mi & lt);
+            S.ref[q] = cref;
+            S.key[q] = key;
+        }
+        sp += __popc(mi);
+        // the leaf children's triangles, 32 per round
+        int c = 0, a = 0;
+        if (take && leaf) {
+            int b;
+            leaf_range(cref, a, b);
+            c = b - a;
+        }
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const int T = __shfl_sync(kFull, incl, 31);
+        for (int i = 0; i < c; ++i) S.tslot[incl - c + i] = a + i;
+        __syncwarp();
+        for (int base = 0; base < T; base += 32) {
+            const int t = base + lane;
+            float e32 = 0.f, err = 0.f;
+            int slot = -1;
+            if (t < T) {
+                slot = S.tslot[t];
+                const float4* tw = reinterpret_cast<const float4*>(tree.wtris + slot);
+                e32 = tri_d2_w(p, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
+            }
+            const float ub = t < T ? e32 + err : CUDART_INF_F;
+            U = fminf(U, __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(ub))));
+            const float lb = e32 - err;
+            const bool cand = t < T && !(lb > U);
+            const unsigned mc = __ballot_sync(kFull, cand);
+            if (nc + __popc(mc) > kHCand) {  // warp-uniform: drop dead candidates, else settle them
+                int keep = 0;
+                for (int i0 = 0; i0 < nc; i0 += 32) {
+                    const int i = i0 + lane;
+                    const bool kp = i < nc && !(S.cl[i] > U);
+                    const int cs_i = kp ? S.cs[i] : 0;
+                    const float cl_i = kp ? S.cl[i] : 0.f;
+                    const unsigned mk = __ballot_sync(kFull, kp);
+                    __syncwarp();  // every lane has read its entry
+                    if (kp) {
+                        S.cs[keep + __popc(mk & lt)] = cs_i;
+                        S.cl[keep + __popc(mk & lt)] = cl_i;
+                    }
+                    keep += __popc(mk);
+                    __syncwarp();
+                }
+                nc = keep;
+                if (nc + __popc(mc) > kHCand) {
+                    heavy_settle(S, nc, CUDART_INF_F, tris, p, bx, sx, ix);
+                    U = fminf(U, __double2float_ru(bx));
+                    nc = 0;
+                    __syncwarp();
+                }
+            }
+            if (cand) {
+                S.cs[nc + __popc(mc & lt)] = slot;
+                S.cl[nc + __popc(mc & lt)] = lb;
+            }
+            nc += __popc(mc);
+            __syncwarp();
+        }
+    }
+    heavy_settle(S, nc, U, tris, p, bx, sx, ix);
+}
+
+// Writes a query's result from its exact nearest triangle (sx < 0: none).
+template <bool UVW, bool SLOT>
+__device__ __forceinline__ void write_nearest(const CTri* __restrict__ tris, int64_t idx, float3 p, double bx, int sx,
+                                              int ix, int slot_face0, float* __restrict__ dist,
+                                              int64_t* __restrict__ face_id, float* __restrict__ uvw,
+                                              int32_t* __restrict__ slot_out) {
+    double d64;
+    if (sx < 0) {  // nothing within MAX_DIST: distance 0 on face 0
+        sx = slot_face0;
+        d64 = 0.0;
+        ix = load_tri(tris, sx).id;
+    } else {
+        d64 = __dsqrt_rn(bx);
+    }
+    dist[idx] = __double2float_rn(d64);
+    face_id[idx] = (int64_t)ix;
+    if (SLOT) slot_out[idx] = sx;
+    if (UVW) {
+        const TriV t = load_tri(tris, sx);
+        double bary[3]; d3 cp;
+        closest_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c), bary, &cp);
+        uvw[3 * idx] = __double2float_rn(bary[0]);
+        uvw[3 * idx + 1] = __double2float_rn(bary[1]);
+        uvw[3 * idx + 2] = __double2float_rn(bary[2]);
+    }
+}
+
 template <bool UVW, bool SLOT>
 __global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint4* __restrict__ heavy,
                                                        const unsigned long long* __restrict__ n_heavy,
@@ -862,11 +1012,9 @@ __global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint4* __restrict__
                                                        float* __restrict__ uvw, int32_t* __restrict__ slot_out,
                                                        const DeviceTree tree,
                                                        unsigned long long* __restrict__ ctr) {
-    const CTri* __restrict__ tris = tree.tris;
     __shared__ HeavyWarp shw[kQBlock / 32];
     HeavyWarp& S = shw[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
     const int64_t nh_all = (int64_t)*n_heavy;
     const int64_t nh = nh_all < heavy_cap ? nh_all : heavy_cap;
     while (true) {
@@ -883,140 +1031,167 @@ __global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint4* __restrict__
             s0 = md.slot0;
         }
         const float3 p = load3(pts, idx);
-        float U = fminf(1e6f, fmaxf(__uint_as_float(hq.z), 0.f));  // the bound found so far (MAX_DIST^2)
-        double bx = 1e6;
-        int sx = -1, ix = 0;
-        // a point that is not finite, or too far away (U < 0), finds nothing
-        int nc = 0, sp = __uint_as_float(hq.z) >= 0.f ? 1 : 0;
-        __syncwarp();  // the previous query is done with S
-        if (lane == 0) { S.ref[0] = root; S.key[0] = 0u; }
-        __syncwarp();
+        double bx;
+        int sx, ix;
+        heavy_walk(S, tree, root, p, __uint_as_float(hq.z), bx, sx, ix);
+        if (lane == 0) write_nearest<UVW, SLOT>(tree.tris, idx, p, bx, sx, ix, s0, dist, face_id, uvw, slot_out);
+    }
+}
+
+// -------------------------------------------------------------- few queries
+// Eight lanes per query, four queries a warp, for calls with too few queries
+// to make packets of near neighbours or to fill the chip with packets: lane j
+// of a group tests child j of the query's node, and the leaf's triangles are
+// spread over the lanes.  The walk is the query's own, nearest child first,
+// so its length is a few node latencies, and the call is this one launch: no
+// bucketing, no queue.  Once the walk has a bound from its first leaf and
+// kFewVisits nodes behind it, a query that needs more is finished by the
+// whole warp, four nodes a step (heavy_walk), as is one whose candidate list
+// overflows; so few queries get a warp each, more of them two or four.
+// Against unsorted packets (100 to 1,000 points on 82k faces 2.7 ms) 22 to 36
+// us; 16,000 points 544 -> 111 us, sorted packets of today 316.  The lines:
+// 32 and 96 visits are up to 1.5 and 2.5 times slower, fewer than the tree is
+// deep up to 3 times; at 64k queries packets draw level (82k-face mesh 376
+// against 302 us, 5,120 faces 389 against 396, 177k open tori 726 against 641).
+constexpr int kFewVisits = 8;
+constexpr int kFewWarps = 16;      // warps of k_udf_few on an SM at a time
+constexpr int kFewCand = 32;
+struct FewGroup {
+    uint2 stack[kStack];           // reference, key
+    uint2 cand[kFewCand];          // slot, lower bound
+};
+union FewWarp { FewGroup g[4]; HeavyWarp h; };
+template <bool UVW, bool SLOT>
+__global__ void __launch_bounds__(kQBlock) k_udf_few(int64_t n, const float* __restrict__ pts,
+                                                     float* __restrict__ dist, int64_t* __restrict__ face_id,
+                                                     float* __restrict__ uvw, int32_t* __restrict__ slot_out,
+                                                     const DeviceTree tree, const MeshDesc* __restrict__ meshes,
+                                                     const int64_t* __restrict__ qoff, int n_meshes, int slot_face0,
+                                                     int per_warp) {
+    __shared__ FewWarp s_few[kQBlock / 32];
+    FewWarp& W = s_few[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, j = lane & 7, g = lane >> 3;
+    FewGroup& S = W.g[g];
+    const CTri* __restrict__ tris = tree.tris;
+    const int64_t w0 = (((int64_t)blockIdx.x * kQBlock + threadIdx.x) >> 5) * per_warp;
+    if (w0 >= n) return;                       // the whole warp
+    const int64_t idx = w0 + g;
+    const bool act = g < per_warp && idx < n;
+    int root = 0, face0 = slot_face0;
+    if (meshes && act) {
+        int lo = 0, hi = n_meshes - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (qoff[mid] <= idx) lo = mid; else hi = mid - 1;
+        }
+        root = meshes[lo].root;
+        face0 = meshes[lo].slot0;
+    }
+    const float3 p = act ? load3(pts, idx) : make_float3(0.f, 0.f, 0.f);
+    const bool reach = act && isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+    float U = reach ? 1e6f : -1.f;             // bound of the squared distance (MAX_DIST^2), the group's
+    int nc = 0, sp = 0, cur = root, visits = 0;
+    bool live = reach, heavy = false;
+    // the next entry within the bound
+    auto pop = [&](float cull) {
+        live = false;
         while (sp > 0) {
+            const uint2 e = S.stack[--sp];
+            if (__uint_as_float(e.y) <= cull) { cur = (int)e.x; live = true; break; }
+        }
+    };
+    while (__any_sync(kFull, live)) {
+        const bool inner = live && cur >= 0;
+        if (__any_sync(kFull, inner)) {
             const float cull = U * 1.000002f;
-            // pop: of the top 32 entries, the first four (from the top) whose
-            // key is within the bound; the culled ones above them go too
-            const int pos = sp - 1 - lane;
-            const bool alive = pos >= 0 && S.key[pos] <= __float_as_uint(cull);
-            const unsigned m = __ballot_sync(kFull, alive);
-            int nn = __popc(m), used = sp < 32 ? sp : 32;
-            if (nn >= 4) {  // up to and including the fourth live entry
-                unsigned m4 = m;
-                m4 &= m4 - 1u;
-                m4 &= m4 - 1u;
-                m4 &= m4 - 1u;
-                used = __ffs(m4);
-                nn = 4;
-            }
-            if (alive && __popc(m & lt) < 4) S.pop[__popc(m & lt)] = S.ref[pos];
-            sp -= used;
-            __syncwarp();
-            // children of the popped nodes
-            const int ni = lane >> 3, j = lane & 7;
-            bool take = false, leaf = false;
-            int cref = 0;
-            uint32_t key = 0u;
-            if (ni < nn) {
-                const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + S.pop[ni]);
+            uint32_t key = kFull;
+            int ref = 0;
+            if (inner) {
+                const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + cur);
                 const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
                 const float d2 = box_d2(p, make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z));
-                if (d2 <= cull) {   // an unused child's box is infinitely far
-                    take = true;
-                    key = __float_as_uint(d2);
-                    cref = __float_as_int(lo.w);
-                    leaf = cref < 0;
-                }
+                if (d2 <= cull) key = (__float_as_uint(d2) & ~7u) | (uint32_t)j;
+                ref = __float_as_int(lo.w);
             }
-            const unsigned mi = __ballot_sync(kFull, take && !leaf);
-            if (take && !leaf) {
-                const int q = sp + __popc(mi & lt);
-                S.ref[q] = cref;
-                S.key[q] = key;
-            }
-            sp += __popc(mi);
-            // the leaf children's triangles, 32 per round
-            int c = 0, a = 0;
-            if (take && leaf) {
-                int b;
-                leaf_range(cref, a, b);
-                c = b - a;
-            }
-            int incl = c;
+            int pos = 0;                       // entries farther than this one
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(kFull, incl, o);
-                if (lane >= o) incl += v;
+            for (int x = 1; x < 8; ++x) {
+                const uint32_t k = __shfl_xor_sync(kFull, key, x);
+                pos += k > key && k != kFull ? 1 : 0;
             }
-            const int T = __shfl_sync(kFull, incl, 31);
-            for (int i = 0; i < c; ++i) S.tslot[incl - c + i] = a + i;
+            const int kept = __popc((__ballot_sync(kFull, key != kFull) >> (lane & 24)) & 0xFFu);
+            if (key != kFull) S.stack[sp + pos] = make_uint2((uint32_t)ref, key & ~7u);
             __syncwarp();
-            for (int base = 0; base < T; base += 32) {
-                const int t = base + lane;
-                float e32 = 0.f, err = 0.f;
-                int slot = -1;
-                if (t < T) {
-                    slot = S.tslot[t];
-                    const float4* tw = reinterpret_cast<const float4*>(tree.wtris + slot);
-                    e32 = tri_d2_w(p, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
-                }
-                const float ub = t < T ? e32 + err : CUDART_INF_F;
-                U = fminf(U, __uint_as_float(__reduce_min_sync(kFull, __float_as_uint(ub))));
-                const float lb = e32 - err;
-                const bool cand = t < T && !(lb > U);
-                const unsigned mc = __ballot_sync(kFull, cand);
-                if (nc + __popc(mc) > kHCand) {  // warp-uniform: drop dead candidates, else settle them
-                    int keep = 0;
-                    for (int i0 = 0; i0 < nc; i0 += 32) {
-                        const int i = i0 + lane;
-                        const bool kp = i < nc && !(S.cl[i] > U);
-                        const int cs_i = kp ? S.cs[i] : 0;
-                        const float cl_i = kp ? S.cl[i] : 0.f;
-                        const unsigned mk = __ballot_sync(kFull, kp);
-                        __syncwarp();  // every lane has read its entry
-                        if (kp) {
-                            S.cs[keep + __popc(mk & lt)] = cs_i;
-                            S.cl[keep + __popc(mk & lt)] = cl_i;
-                        }
-                        keep += __popc(mk);
-                        __syncwarp();
-                    }
-                    nc = keep;
-                    if (nc + __popc(mc) > kHCand) {
-                        heavy_settle(S, nc, CUDART_INF_F, tris, p, bx, sx, ix);
-                        U = fminf(U, __double2float_ru(bx));
-                        nc = 0;
-                        __syncwarp();
-                    }
-                }
-                if (cand) {
-                    S.cs[nc + __popc(mc & lt)] = slot;
-                    S.cl[nc + __popc(mc & lt)] = lb;
-                }
-                nc += __popc(mc);
-                __syncwarp();
+            if (inner) {
+                sp += kept;
+                pop(cull);
+                if (++visits >= kFewVisits && U < 1e6f && live) { live = false; heavy = true; }
             }
+            __syncwarp();                      // the entries have been read
         }
-        heavy_settle(S, nc, U, tris, p, bx, sx, ix);
-        if (lane == 0) {
-            double d64;
-            if (sx < 0) {  // nothing within MAX_DIST: distance 0 on face 0
-                sx = s0;
-                d64 = 0.0;
-                ix = load_tri(tris, sx).id;
-            } else {
-                d64 = __dsqrt_rn(bx);
+        const bool leaf = live && cur < 0;
+        if (__any_sync(kFull, leaf)) {
+            float lb = 0.f, ub = CUDART_INF_F;
+            int s = 0;
+            bool on = false;
+            if (leaf) {
+                int s0, s1;
+                leaf_range(cur, s0, s1);
+                s = s0 + j;
+                on = s < s1;
+                if (on) {
+                    const float4* tw = reinterpret_cast<const float4*>(tree.wtris + s);
+                    float err;
+                    const float d2 = tri_d2_w(p, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
+                    lb = d2 - err;
+                    ub = d2 + err;
+                }
             }
-            dist[idx] = __double2float_rn(d64);
-            face_id[idx] = (int64_t)ix;
-            if (SLOT) slot_out[idx] = sx;
-            if (UVW) {
-                const TriV t = load_tri(tris, sx);
-                double bary[3]; d3 cp;
-                closest_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c), bary, &cp);
-                uvw[3 * idx] = __double2float_rn(bary[0]);
-                uvw[3 * idx + 1] = __double2float_rn(bary[1]);
-                uvw[3 * idx + 2] = __double2float_rn(bary[2]);
+#pragma unroll
+            for (int x = 1; x < 4; x <<= 1) ub = fminf(ub, __shfl_xor_sync(kFull, ub, x));   // lanes 0 - 3 hold the leaf
+            ub = __shfl_sync(kFull, ub, lane & 24);
+            if (leaf) U = fminf(U, ub);
+            const bool c = on && !(lb > U);    // within the bound, or undecided (no number)
+            const unsigned m = (__ballot_sync(kFull, c) >> (lane & 24)) & 0xFFu;
+            if (leaf) {
+                const int at = nc + __popc(m & ((1u << j) - 1u));
+                if (c && at < kFewCand) S.cand[at] = make_uint2((uint32_t)s, __float_as_uint(lb));
+                nc += __popc(m);
+                pop(U * 1.000002f);
+                if (nc > kFewCand) { live = false; heavy = true; }
             }
+            __syncwarp();
         }
+    }
+    // exact minimum (ties -> lowest face index) of the group's candidates
+    double bx = CUDART_INF;
+    int sx = -1, ix = INT_MAX;
+    __syncwarp();
+    if (!heavy) {
+        for (int i = j; i < nc; i += 8) {
+            const uint2 e = S.cand[i];
+            if (__uint_as_float(e.y) > U) continue;
+            const TriV t = load_tri(tris, (int)e.x);
+            const double d = dist2_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c));
+            if (d <= 1e6 && (d < bx || (d == bx && t.id < ix))) { bx = d; sx = (int)e.x; ix = t.id; }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int x = 1; x < 8; x <<= 1) {
+        const double b2 = __shfl_xor_sync(kFull, bx, x);
+        const int s2 = __shfl_xor_sync(kFull, sx, x), i2 = __shfl_xor_sync(kFull, ix, x);
+        if (s2 >= 0 && (b2 < bx || (b2 == bx && i2 < ix))) { bx = b2; sx = s2; ix = i2; }
+    }
+    if (act && !heavy && j == 0) write_nearest<UVW, SLOT>(tris, idx, p, bx, sx, ix, face0, dist, face_id, uvw, slot_out);
+    // the long ones, one after the other, by the whole warp
+    for (unsigned hm = __ballot_sync(kFull, heavy && j == 0); hm; hm &= hm - 1u) {
+        const int src = __ffs(hm) - 1;
+        const float3 q = make_float3(__shfl_sync(kFull, p.x, src), __shfl_sync(kFull, p.y, src), __shfl_sync(kFull, p.z, src));
+        const float u = __shfl_sync(kFull, U, src);
+        const int r = __shfl_sync(kFull, root, src), f0 = __shfl_sync(kFull, face0, src);
+        heavy_walk(W.h, tree, r, q, u, bx, sx, ix);
+        if (lane == 0) write_nearest<UVW, SLOT>(tris, w0 + (src >> 3), q, bx, sx, ix, f0, dist, face_id, uvw, slot_out);
     }
 }
 
@@ -2324,7 +2499,7 @@ RayWs ray_ws(int64_t n) {
 size_t query_workspace_bytes(int mode, int64_t n) {
     size_t b = 256;                                               // packet counters
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    if (mode >= 0 && n >= kSortMinQueries) {
+    if (mode >= 0 && n >= kFewQueries) {
         const int64_t cells = (int64_t)1 << (3 * cell_bits(n));
         b += al(sizeof(uint32_t) * n);                            // order
         b += al(sizeof(uint32_t) * (cells + 1));                  // cell counts / offsets
@@ -2432,6 +2607,24 @@ void launch_raystab(const Work& w, int64_t n, const uint32_t* order, const float
 
 namespace {
 template <bool UVW, bool SLOT>
+void launch_few_t(int64_t n, const float* pts, float* dist, int64_t* fid, float* uvw, int32_t* slots,
+                  const DeviceTree& tree, const MeshDesc* meshes, const int64_t* qoff, int n_meshes, int slot0,
+                  cudaStream_t stream) {
+    const int64_t room = (int64_t)sm_count() * kFewWarps;
+    const int q = n <= room ? 1 : (n <= 2 * room ? 2 : 4);   // queries per warp
+    const int64_t warps = (n + q - 1) / q;
+    k_udf_few<UVW, SLOT><<<(unsigned)((warps + 3) / 4), kQBlock, 0, stream>>>(n, pts, dist, fid, uvw, slots, tree, meshes,
+                                                                              qoff, n_meshes, slot0, q); count_launch();
+}
+void launch_few(int64_t n, const float* pts, float* dist, int64_t* fid, float* uvw, int32_t* slots,
+                const DeviceTree& tree, const MeshDesc* meshes, const int64_t* qoff, int n_meshes, int slot0,
+                cudaStream_t stream) {
+    if (uvw && slots) launch_few_t<true, true>(n, pts, dist, fid, uvw, slots, tree, meshes, qoff, n_meshes, slot0, stream);
+    else if (uvw) launch_few_t<true, false>(n, pts, dist, fid, uvw, slots, tree, meshes, qoff, n_meshes, slot0, stream);
+    else if (slots) launch_few_t<false, true>(n, pts, dist, fid, uvw, slots, tree, meshes, qoff, n_meshes, slot0, stream);
+    else launch_few_t<false, false>(n, pts, dist, fid, uvw, slots, tree, meshes, qoff, n_meshes, slot0, stream);
+}
+template <bool UVW, bool SLOT>
 void launch_nearest_t(const Work& w, int64_t n, const uint32_t* order, const float* pts, float* dist, int64_t* fid,
                       float* uvw, int32_t* slots, const DeviceTree& tree, uint4* heavy, int64_t hcap,
                       unsigned long long* ctr, bool yield, cudaStream_t stream) {
@@ -2465,10 +2658,11 @@ cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     char* w = static_cast<char*>(ws);
     unsigned long long* ctr = reinterpret_cast<unsigned long long*>(w); w += 256;
-    cudaError_t e = cudaMemsetAsync(ctr, 0, 256, stream);
-    if (e != cudaSuccess) return e;
+    const bool few = n < kFewQueries;
+    cudaError_t e = cudaSuccess;
+    if (!(few && mode == 0) && (e = cudaMemsetAsync(ctr, 0, 256, stream)) != cudaSuccess) return e;
     uint32_t* order = nullptr;
-    if (n >= kSortMinQueries) {
+    if (!few) {
         const int bits = cell_bits(n);
         const int64_t cells = (int64_t)1 << (3 * bits);
         order = reinterpret_cast<uint32_t*>(w); w += al(sizeof(uint32_t) * n);
@@ -2491,7 +2685,10 @@ cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts
     const int64_t hcap = heavy_cap_for(n);
     w += al(sizeof(uint4) * hcap);
     const Work work{nullptr, nullptr, n, slot_face0, qbase};
-    launch_nearest(work, n, order, pts, dist, fid, want_uvw ? uvw : nullptr, slots, tree, heavy, hcap, ctr, yield, stream);
+    if (few)
+        launch_few(n, pts, dist, fid, want_uvw ? uvw : nullptr, slots, tree, nullptr, nullptr, 0, slot_face0, stream);
+    else
+        launch_nearest(work, n, order, pts, dist, fid, want_uvw ? uvw : nullptr, slots, tree, heavy, hcap, ctr, yield, stream);
     if (mode == 1) {
         if (near.cnt) {
             const unsigned g = persistent_grid(k_sign_watertight<true>, n);
@@ -2592,28 +2789,36 @@ __global__ void k_arena_scatter(int64_t n, const float* __restrict__ pts, const 
 cudaError_t launch_arena_distance(const ArenaLaunch& a, const float* pts, float* dist, int64_t* fid, float* uvw,
                                   cudaStream_t stream) {
     if (a.n_queries <= 0) return cudaSuccess;
+    const bool few = a.n_queries < kFewQueries;
+    uint32_t* const order = few ? nullptr : a.order;
     cudaError_t e = cudaMemsetAsync(a.counters, 0, 256, stream);
     if (e != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(a.hist, 0, sizeof(uint32_t) * (a.n_cells + 1), stream)) != cudaSuccess) return e;
-    const unsigned g = (unsigned)sm_count() * 8;
-    k_arena_hist<<<g, 256, 0, stream>>>(a.n_queries, pts, a.qoff, a.n_meshes, a.sort, a.hist); count_launch();
-    scan::exclusive(a.hist, a.bsum, a.n_cells, stream);
-    k_arena_scatter<<<g, 256, 0, stream>>>(a.n_queries, pts, a.qoff, a.n_meshes, a.sort, a.hist, a.order); count_launch();
+    if (!few) {
+        if ((e = cudaMemsetAsync(a.hist, 0, sizeof(uint32_t) * (a.n_cells + 1), stream)) != cudaSuccess) return e;
+        const unsigned g = (unsigned)sm_count() * 8;
+        k_arena_hist<<<g, 256, 0, stream>>>(a.n_queries, pts, a.qoff, a.n_meshes, a.sort, a.hist); count_launch();
+        scan::exclusive(a.hist, a.bsum, a.n_cells, stream);
+        k_arena_scatter<<<g, 256, 0, stream>>>(a.n_queries, pts, a.qoff, a.n_meshes, a.sort, a.hist, a.order); count_launch();
+    }
     const bool signed_any = a.n_wt_packets > 0 || a.n_rs_packets > 0;
     const Work all{a.packets, a.meshes, a.n_packets, 0};
-    launch_nearest(all, a.n_queries, a.order, pts, dist, fid, uvw, signed_any ? a.slots : nullptr, a.tree, a.heavy,
-                   a.heavy_cap, a.counters, false, stream);
+    int32_t* const slots = signed_any ? a.slots : nullptr;
+    if (few)
+        launch_few(a.n_queries, pts, dist, fid, uvw, slots, a.tree, a.meshes, a.qoff, a.n_meshes, 0, stream);
+    else
+        launch_nearest(all, a.n_queries, order, pts, dist, fid, uvw, slots, a.tree, a.heavy, a.heavy_cap, a.counters, false,
+                       stream);
     if (a.n_wt_packets > 0) {
         const Work w{a.wt_packets, a.meshes, a.n_wt_packets, 0};
         const unsigned gw = persistent_grid(k_sign_watertight<false>, 32 * a.n_wt_packets);
-        k_sign_watertight<false><<<gw, kQBlock, 0, stream>>>(w, a.order, pts, dist, a.slots, a.tree.nodes, a.tree.tris,
+        k_sign_watertight<false><<<gw, kQBlock, 0, stream>>>(w, order, pts, dist, a.slots, a.tree.nodes, a.tree.tris,
                                                              NearLists{}, nullptr, nullptr, a.counters + kCtSign,
                                                              grab_for(32 * a.n_wt_packets, gw), 0); count_launch();
     }
     if (a.n_rs_packets > 0) {
         const Work w{a.rs_packets, a.meshes, a.n_rs_packets, 0};
         if ((e = cudaMemsetAsync(a.parity, 0, sizeof(unsigned long long) * a.n_meshes, stream)) != cudaSuccess) return e;
-        launch_raystab(w, 32 * a.n_rs_packets, a.order, pts, dist, a.tree.nodes, a.tree.tris, a.counters + kCtArenaRs,
+        launch_raystab(w, 32 * a.n_rs_packets, order, pts, dist, a.tree.nodes, a.tree.tris, a.counters + kCtArenaRs,
                        a.rs_cand, a.counters + kCtCandN, a.counters + kCtLinesNext, a.tree.n_tris, a.face_off, a.face_slot,
                        a.n_meshes, a.parity, stream);
     }

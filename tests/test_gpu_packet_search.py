@@ -20,9 +20,10 @@ def _check(oracle, v, f, pts, dev):
     assert np.array_equal(uvw.cpu().numpy(), ouvw.astype(np.float32))
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 31, 32, 33, 65, 2047, 2048, 2049, 6001])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 31, 32, 33, 2367, 2368, 2369, 4737, 65535, 65536, 65567])
 def test_packet_edges(oracle, dev, n):
-    v, f = W.displaced_icosphere(3, 2)
+    """Below 65,536 points eight lanes a query, one, two or four queries a warp; above, packets of 32."""
+    v, f = W.displaced_icosphere(2, 2)
     _check(oracle, v, f, W.uniform_points(n, n), dev)
 
 
@@ -35,7 +36,7 @@ def _fan(valence, copies):
 
 
 @pytest.mark.parametrize("valence,copies", [(40, 1), (8, 12), (200, 2)])
-@pytest.mark.parametrize("n", [40, 5000])
+@pytest.mark.parametrize("n", [40, 5000, 70000])
 def test_candidate_overflow(oracle, dev, valence, copies, n):
     """Points above the apex tie on every triangle of the fan."""
     v, f = _fan(valence, copies)
@@ -45,16 +46,38 @@ def test_candidate_overflow(oracle, dev, valence, copies, n):
     _check(oracle, v, f, pts, dev)
 
 
+@pytest.mark.parametrize("counts", [[1, 0, 300, 7], [40000, 0, 25536, 3]])
+def test_small_and_large_arenas(oracle, dev, counts):
+    """Queries of several meshes, one of them without any, on both sides of the split."""
+    meshes = [W.icosphere(2, 0.8), W.displaced_icosphere(2, 1), W.displaced_icosphere(3, 3), W.icosphere(1, 0.5)]
+    arena = cubvh.BVHArena(meshes)
+    arena.set_queries(counts, ["unsigned", "watertight", "watertight", "raystab"])
+    qs = [W.uniform_points(n, i) for i, n in enumerate(counts)]
+    d, fid, uvw = arena.distance(torch.from_numpy(np.concatenate(qs)).to(dev), return_uvw=True)
+    at = 0
+    for (v, f), q, mode in zip(meshes, qs, ["unsigned", "watertight", "watertight", "raystab"]):
+        if len(q):
+            bvh, p = cubvh.cuBVH(v, f), torch.from_numpy(q).to(dev)
+            want = (bvh.unsigned_distance(p, return_uvw=True) if mode == "unsigned"
+                    else bvh.signed_distance(p, return_uvw=True, mode=mode))
+            for a, b in zip((d, fid, uvw), want):
+                assert torch.equal(a[at:at + len(q)], b)
+            od, ofid, _, _, _ = oracle.udf64(v, f, q[:2000])
+            assert np.array_equal(fid[at:at + len(q)][:2000].cpu().numpy(), ofid)
+            assert np.array_equal(d[at:at + len(q)][:2000].abs().cpu().numpy(), od.astype(np.float32))
+        at += len(q)
+
+
 def test_idle_points(oracle, dev):
     """Points that are no number, infinite or out of reach, between ordinary ones in the same packets."""
     v, f = W.displaced_icosphere(3, 2)
-    pts = W.uniform_points(4096, 5)
+    pts = W.uniform_points(70016, 5)
     odd = np.array([[np.nan, 0, 0], [np.inf, 0, 0], [0, -np.inf, 0], [3e38, 0, 0], [2000, 0, 0], [0, 1.5e3, 0]], np.float32)
-    at = np.arange(0, 4096, 37)
+    at = np.arange(0, len(pts), 37)
     mixed = pts.copy()
     mixed[at] = odd[np.arange(len(at)) % len(odd)]
     bvh = cubvh.cuBVH(v, f)
-    for n in (4096, 300):
+    for n in (len(pts), 4096, 300):
         want = bvh.unsigned_distance(torch.from_numpy(pts[:n]).to(dev))
         d, fid, _ = bvh.unsigned_distance(torch.from_numpy(mixed[:n]).to(dev))
         keep = np.ones(n, bool)
