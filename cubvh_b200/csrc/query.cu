@@ -1370,8 +1370,9 @@ __global__ void __launch_bounds__(kQBlock) k_near_lists(int64_t nt, const CNode*
 // point of the query's nearest triangle (soup slot `own`).  LIST: the normal
 // sum over own's candidate list; a query whose list overflowed is queued in
 // ovf for k_sign_watertight_ovf (single BVH).  !LIST: the walk (arenas).
+constexpr int kSignBlocks = 5;   // blocks per SM (8.4M points, whole call: 4 5.41 ms, 5 5.23, 6 5.31)
 template <bool LIST>
-__global__ void __launch_bounds__(kQBlock)
+__global__ void __launch_bounds__(kQBlock, LIST ? kSignBlocks : 1)
 k_sign_watertight(Work w, const uint32_t* __restrict__ order, const float* __restrict__ pts, float* __restrict__ dist,
                   const int32_t* __restrict__ slots, const CNode* __restrict__ nodes, const CTri* __restrict__ tris,
                   const NearLists near, uint32_t* __restrict__ ovf, unsigned long long* __restrict__ ovf_n,
@@ -1514,163 +1515,176 @@ __global__ void __launch_bounds__(256) k_edge_parity(int64_t nt, const CTri* __r
     }
 }
 
-// Work is per lane, not per warp: a warp takes a chunk of packets (queries in
-// Morton-cell order) and each lane takes the chunk's next query from a
-// shared-memory counter whenever its own query ends, and starts its next
-// stab ray as soon as the current one hits.  Stab directions differ from
-// lane to lane and inside queries need 64 rays where outside ones end after a
-// few, so lanes never wait for one another except at the end of a chunk.
-// The per-query setup (query index, stab stream offset, root, whether its
-// first ray counts crossings) is computed by the whole warp in lockstep when
-// the chunk is taken.
+// First raystab pass: each lane traces one query's first stab line, ray 0 =
+// -d_0 and, when that hits (or its count decides nothing), ray 1 = +d_0.  A
+// query whose rays both hit is appended to `cand` (query index, stab offset,
+// root: warp-aggregated atomic on cand_n), for k_sign_raystab_lines.  Outside
+// points mostly see a ray miss and end in this pass, as do the inside points
+// of closed meshes; the candidates are mostly inside points of other meshes,
+// which need every ray.
 //
-// With max_rays < 64 this is the first of two passes: a query whose first
-// max_rays rays all hit is not finished here but appended to `cand` (query
-// index, stab offset, root: warp-aggregated atomic on cand_n), for
-// k_sign_raystab_lines.  Outside points mostly see their first rays miss
-// and end in this pass, as do the inside points of closed meshes; the
-// candidates are mostly inside points of other meshes, which need every ray.
-constexpr int kChunkMax = 2;  // packets per raystab chunk
-__global__ void __launch_bounds__(kQBlock) k_sign_raystab(Work w, const uint32_t* __restrict__ order,
+// Work is per lane, as in k_ray_lanes: a warp takes a chunk of packets (queries
+// in Morton-cell order), prepares its queries in lockstep (position, stab
+// offset, d_0, root, whether ray 0 counts crossings), and hands them to lanes
+// whenever kStabRefill are idle; its lanes stay on the same kind of step, inner
+// nodes until few are at one, then leaves.  Lanes refilled one by one, each on
+// its own step, took 2.2 of the 4.1 ms of 2.1M points on a closed 82k-face
+// mesh; now the call takes 3.0 (refill at 12 and 20 idle lanes 3.2 and 3.5).
+constexpr int kChunkMax = 2;      // packets per raystab chunk
+constexpr int kStabRefill = 6;   // idle lanes that take new queries
+constexpr int kStabInner = 12;    // fewer lanes at inner nodes than this wait for those at leaves
+constexpr int kStabBlocks = 6;    // blocks per SM
+struct StabQuery { float px, py, pz, dx, dy, dz, ox, oy; uint32_t idx; int root; };   // d_0, stab offset; root -1: none, -2 - root: counting
+__global__ void __launch_bounds__(kQBlock, kStabBlocks) k_sign_raystab(Work w, const uint32_t* __restrict__ order,
                                                           const float* __restrict__ pts, float* __restrict__ dist,
                                                           const CNode* __restrict__ nodes,
                                                           const CTri* __restrict__ tris,
                                                           unsigned long long* __restrict__ ctr, int64_t grab,
-                                                          int max_rays, uint4* __restrict__ cand,
+                                                          uint4* __restrict__ cand,
                                                           unsigned long long* __restrict__ cand_n,
                                                           const unsigned long long* __restrict__ parity) {
-    __shared__ int s_next[kQBlock / 32];
-    __shared__ uint8_t s_count[kQBlock / 32][kChunkMax * 32];   // the query's first ray counts crossings
-    __shared__ uint4 s_q[kQBlock / 32][kChunkMax * 32];  // query index, offset x/y bits, root (-1: none)
-    const int wib = threadIdx.x >> 5;
+    __shared__ StabQuery s_q[kQBlock / 32][kChunkMax * 32];
+    StabQuery* sq = s_q[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
     const float tmaxf = 1000.0f;
     const float cull = cull_of(1000.0);
     PacketQueue pq(ctr, w.packets(), grab);
-    int64_t pk0, pk1;
-    while (pq.take_range(pk0, pk1)) {
-        const int total = (int)(pk1 - pk0) * 32;
-        for (int i = threadIdx.x & 31; i < total; i += 32) {
-            int64_t start, qoff;
-            int cnt, rt, s0;
-            w.get(pk0 + (i >> 5), start, cnt, rt, s0, qoff);
-            uint4 e = make_uint4(0u, 0u, 0u, 0xFFFFFFFFu);
-            if ((i & 31) < cnt) {
-                const int64_t qi = start + (i & 31);
-                const int64_t id = order ? (int64_t)order[qi] : qi;
-                // the stab stream of a query is its index within its own call / mesh
-                const float2 o2 = stab_offset((uint32_t)(id - qoff));
-                e = make_uint4((uint32_t)id, __float_as_uint(o2.x), __float_as_uint(o2.y), (uint32_t)rt);
-                // closed, and the whole root box within t < 1000 of the point
-                const float3 q = load3(pts, id);
-                const CNode* rn = nodes + rt;
-                float far2 = 0.f;
-                const float lo[3] = {rn->ox, rn->oy, rn->oz}, qc[3] = {q.x, q.y, q.z};
-                const int ex[3] = {rn->ex, rn->ey, rn->ez};
+    int next = 0, total = 0;                 // the chunk's queries: next to hand out, number
+    bool more = true;                        // more chunks may come
+    bool live = false, second = false, counting = false, unsure = false, any = false, degen = false;
+    int crossings = 0, root = 0, cur = 0, sp = 0;
+    int64_t idx = -1;
+    float3 p = make_float3(0.f, 0.f, 0.f), d = p, inv = p;
+    float2 off = make_float2(0.f, 0.f);
+    float dinf = 0.f;
+    int st[kStack];
+    auto start_ray = [&]() {
+        inv = ray_inv_approx(d);
+        degen = ray_degenerate(inv);
+        dinf = f3inf(d);
+        sp = 0;
+        cur = root;
+    };
+    while (true) {
+        const unsigned idle = __ballot_sync(kFull, !live);
+        if (idle == kFull || ((more || next < total) && __popc(idle) >= kStabRefill)) {
+            if (next >= total && more) {     // the next chunk
+                int64_t pk0, pk1;
+                more = pq.take_range(pk0, pk1);
+                total = more ? (int)(pk1 - pk0) * 32 : 0;
+                next = 0;
+                __syncwarp();                // the last chunk's queries have been read
+                for (int i = lane; i < total; i += 32) {
+                    int64_t start, qoff;
+                    int cnt, rt, s0;
+                    w.get(pk0 + (i >> 5), start, cnt, rt, s0, qoff);
+                    StabQuery q;
+                    q.root = -1;
+                    if ((i & 31) < cnt) {
+                        const int64_t qi = start + (i & 31);
+                        const int64_t id = order ? (int64_t)order[qi] : qi;
+                        // the stab stream of a query is its index within its own call / mesh
+                        const float2 o2 = stab_offset((uint32_t)(id - qoff));
+                        const float3 v = load3(pts, id), sd = stab_dir(0, o2);
+                        // closed, and the whole root box within t < 1000 of the point
+                        const CNode* rn = nodes + rt;
+                        float far2 = 0.f;
+                        const float lo[3] = {rn->ox, rn->oy, rn->oz}, qc[3] = {v.x, v.y, v.z};
+                        const int ex[3] = {rn->ex, rn->ey, rn->ez};
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float f = fmaxf(fabsf(lo[k] - qc[k]), fabsf(fmaf(255.f, exp2i(ex[k]), lo[k]) - qc[k]));
-                    far2 = fmaf(f, f, far2);
-                }
-                s_count[wib][i] = parity[w.mesh_of(pk0 + (i >> 5))] == 0ull && far2 < 9.8e5f;
-            }
-            s_q[wib][i] = e;
-        }
-        if ((threadIdx.x & 31) == 0) s_next[wib] = 0;
-        __syncwarp();
-        int64_t idx = -1;  // current query, -1: none
-        int root = 0;
-        float3 p = make_float3(0.f, 0.f, 0.f), sd = p, d = p, inv = p;
-        float2 off = make_float2(0.f, 0.f);
-        float dinf = 0.f;
-        bool degen = false;
-        uint32_t r = 0;    // ray r: -d_{r/2} for even r, +d_{r/2} for odd r
-        bool counting = false, unsure = false, any = false;   // crossings of the first ray are counted
-        int crossings = 0;
-        int st[kStack];
-        int sp = 0;
-        while (true) {
-            if (idx < 0) {
-                int i;
-                while ((i = atomicAdd(&s_next[wib], 1)) < total) {
-                    const uint4 e = s_q[wib][i];
-                    if (e.w != 0xFFFFFFFFu) {
-                        idx = e.x;
-                        off = make_float2(__uint_as_float(e.y), __uint_as_float(e.z));
-                        root = (int)e.w;
-                        counting = s_count[wib][i] != 0;
-                        break;
+                        for (int k = 0; k < 3; ++k) {
+                            const float f = fmaxf(fabsf(lo[k] - qc[k]), fabsf(fmaf(255.f, exp2i(ex[k]), lo[k]) - qc[k]));
+                            far2 = fmaf(f, f, far2);
+                        }
+                        const bool count = parity[w.mesh_of(pk0 + (i >> 5))] == 0ull && far2 < 9.8e5f;
+                        q = StabQuery{v.x, v.y, v.z, sd.x, sd.y, sd.z, o2.x, o2.y, (uint32_t)id, count ? -2 - rt : rt};
                     }
+                    sq[i] = q;
                 }
-                if (idx < 0) break;
-                p = load3(pts, idx);
-                r = 0;
-                sd = stab_dir(0, off);
-                d = make_float3(-sd.x, -sd.y, -sd.z);
-                inv = ray_inv_approx(d);
-                degen = ray_degenerate(inv);
-                dinf = f3inf(d);
-                sp = 0;
-                st[sp++] = root;
-                unsure = any = false;
-                crossings = 0;
+                __syncwarp();
             }
-            bool hit = false;
-            if (sp == 0) {
-                if (!counting || !any) { idx = -1; continue; }  // ray r missed: outside
-                if (!unsure && (crossings & 1)) {               // inside: every ray hits
-                    dist[idx] = -dist[idx];
-                    idx = -1;
-                    continue;
+            if (next < total) {
+                const int k = next + __popc(idle & lt);
+                if (!live && k < total && sq[k].root != -1) {
+                    const StabQuery q = sq[k];
+                    counting = q.root < 0;
+                    root = counting ? -2 - q.root : q.root;
+                    idx = q.idx;
+                    p = make_float3(q.px, q.py, q.pz);
+                    d = make_float3(-q.dx, -q.dy, -q.dz);
+                    off = make_float2(q.ox, q.oy);
+                    second = unsure = any = false;
+                    crossings = 0;
+                    live = true;
+                    start_ray();
                 }
-                counting = false;                               // ray 0 hit: on with ray 1
-                hit = true;
+                next += __popc(idle);
+            } else if (idle == kFull && !more) {
+                break;
             }
-            const int ref = hit ? INT_MAX : st[--sp];
-            if (ref >= 0 && !hit) {
-                const NodeView nd = load_node(nodes, ref);
+            continue;
+        }
+        bool ended = false, hit = false;
+        // inner nodes
+        while (true) {
+            const bool inner = live && !ended && cur >= 0;
+            const unsigned in = __ballot_sync(kFull, inner);
+            if (!in || (__popc(in) < kStabInner && __any_sync(kFull, live && !ended && cur < 0))) break;
+            if (inner) {
+                const NodeView nd = load_node(nodes, cur);
                 if (degen) push_ray_children<true>(nd, p, inv, cull, st, sp);
                 else push_ray_children_affine(nd, p, inv, cull, st, sp);
-            } else if (ref < 0) {
-                int a, b;
-                leaf_range(ref, a, b);
-                for (int s = a; s < b && !hit; ++s) {
-                    const TriV t = load_tri(tris, s);
-                    float tt, terr;
-                    const int c = ray_tri_f(p, d, dinf, t, tmaxf, &tt, &terr);
-                    bool on = c == 1;
-                    if (c < 0) {
-                        double t64;
-                        on = ray_tri_d(to_d3(p), to_d3(d), to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64);
-                        unsure = true;
-                    }
-                    any |= on;
-                    crossings += on ? 1 : 0;
-                    hit = on && !counting;
-                }
+                if (sp > 0) cur = st[--sp];
+                else ended = true;
             }
-            if (hit) {
-                if (++r == 64) {  // every ray hit: inside
-                    dist[idx] = -dist[idx];
-                    idx = -1;
-                    continue;
+            if (__popc(__ballot_sync(kFull, !live || ended)) >= kStabRefill) break;
+        }
+        // leaves
+        if (live && !ended && cur < 0) {
+            int a, b;
+            leaf_range(cur, a, b);
+            for (int s = a; s < b && !hit; ++s) {
+                const TriV t = load_tri(tris, s);
+                float tt, terr;
+                const int c = ray_tri_f(p, d, dinf, t, tmaxf, &tt, &terr);
+                bool on = c == 1;
+                if (c < 0) {
+                    double t64;
+                    on = ray_tri_d(to_d3(p), to_d3(d), to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64);
+                    unsure = true;
                 }
-                if ((int)r == max_rays) {  // first pass: the rest goes to k_sign_raystab_lines
-                    const cooperative_groups::coalesced_group g = cooperative_groups::coalesced_threads();
-                    unsigned long long b = 0;
-                    if (g.thread_rank() == 0) b = atomicAdd(cand_n, (unsigned long long)g.size());
-                    b = g.shfl(b, 0) + g.thread_rank();
-                    cand[b] = make_uint4((uint32_t)idx, __float_as_uint(off.x), __float_as_uint(off.y),
-                                         (uint32_t)root);
-                    idx = -1;
-                    continue;
-                }
-                if (r & 1) d = sd;
-                else { sd = stab_dir(r >> 1, off); d = make_float3(-sd.x, -sd.y, -sd.z); }
-                inv = ray_inv_approx(d);
-                degen = ray_degenerate(inv);
-                dinf = f3inf(d);
-                sp = 0;
-                st[sp++] = root;
+                any |= on;
+                crossings += on ? 1 : 0;
+                hit = on && !counting;
+            }
+            if (!hit) {
+                if (sp > 0) cur = st[--sp];
+                else ended = true;
+            }
+        }
+        __syncwarp();
+        // rays that came to their end
+        if (ended) {
+            if (counting && any && (unsure || !(crossings & 1))) hit = true;   // ray 0 hits, no more is known
+            else {
+                if (counting && any) dist[idx] = -dist[idx];                   // inside: every ray hits
+                live = false;                                                  // else a ray missed: outside
+            }
+            counting = false;
+        }
+        if (hit) {
+            if (!second) {
+                second = true;
+                d = make_float3(-d.x, -d.y, -d.z);
+                start_ray();
+            } else {
+                const cooperative_groups::coalesced_group g = cooperative_groups::coalesced_threads();
+                unsigned long long b = 0;
+                if (g.thread_rank() == 0) b = atomicAdd(cand_n, (unsigned long long)g.size());
+                b = g.shfl(b, 0) + g.thread_rank();
+                cand[b] = make_uint4((uint32_t)idx, __float_as_uint(off.x), __float_as_uint(off.y), (uint32_t)root);
+                live = false;
             }
         }
         __syncwarp();
@@ -2079,6 +2093,11 @@ __global__ void k_box(int64_t n, const float* __restrict__ pts, uint32_t* __rest
         for (int k = 0; k < 3; ++k)
             if (isfinite(c[k])) { lo[k] = min(lo[k], f2o(c[k])); hi[k] = max(hi[k], f2o(c[k])); }
     }
+    // one set of atomics a block: a set per warp, 57,000 atomics on six words,
+    // took 41 us of 1M points' bucketing
+    __shared__ uint32_t s_box[6];
+    if (threadIdx.x < 6) s_box[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         lo[k] = __reduce_min_sync(kFull, lo[k]);
@@ -2086,8 +2105,11 @@ __global__ void k_box(int64_t n, const float* __restrict__ pts, uint32_t* __rest
     }
     if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) { atomicMin(&box[k], lo[k]); atomicMax(&box[3 + k], hi[k]); }
+        for (int k = 0; k < 3; ++k) { atomicMin(&s_box[k], lo[k]); atomicMax(&s_box[3 + k], hi[k]); }
     }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(&box[threadIdx.x], s_box[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(&box[threadIdx.x], s_box[threadIdx.x]);
 }
 __device__ __forceinline__ uint32_t cell_of(float3 p, const uint32_t* __restrict__ box, int bits) {
     const float side = (float)(1 << bits), m = side - 1.f;
@@ -2571,10 +2593,7 @@ LaunchShape yield_shape(unsigned g, int64_t grabs, bool on) {
     const int64_t bg = (2 * grabs + G - 1) / G;
     return {(unsigned)G, (int)(bg > 0 ? bg : 1)};
 }
-// raystab chunk: kChunkMax packets (64 queries for 32 lanes: a lane whose
-// query ends early takes another one; larger chunks cost more in lane-by-lane
-// query setup than they save), one packet when the launch has fewer than two
-// packets per warp
+// raystab chunk: kChunkMax packets, one packet when the launch has few per warp
 int64_t chunk_for(int64_t n, unsigned grid) {
     const int64_t packets = (n + 31) / 32;
     const int64_t warps = (int64_t)grid * (kQBlock / 32);
@@ -2597,8 +2616,8 @@ void launch_raystab(const Work& w, int64_t n, const uint32_t* order, const float
     k_edge_parity<<<(unsigned)((n_tris + 1023) / 1024), 256, 0, stream>>>(n_tris, tris, face_off, face_slot, n_meshes,
                                                                           parity); count_launch();
     const unsigned g = persistent_grid(k_sign_raystab, n);
-    k_sign_raystab<<<g, kQBlock, 0, stream>>>(w, order, pts, dist, nodes, tris, ctr, chunk_for(n, g),
-                                              kRaystabFirstRays, cand, cand_n, parity); count_launch();
+    k_sign_raystab<<<g, kQBlock, 0, stream>>>(w, order, pts, dist, nodes, tris, ctr, chunk_for(n, g), cand, cand_n, parity);
+    count_launch();
     const unsigned g2 = persistent_grid(k_sign_raystab_lines, n);
     k_sign_raystab_lines<<<g2, kQBlock, 0, stream>>>(pts, dist, nodes, tris, cand, cand_n, lines_next,
                                                      kRaystabFirstRays); count_launch();
