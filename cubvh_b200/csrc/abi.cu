@@ -47,6 +47,7 @@ struct DevCopy {
     WNode* wnodes = nullptr;       // expanded records (launch_expand)
     WTri* wtris = nullptr;
     int64_t n_tris = 0;
+    bool one_block = false;        // tris, wnodes and wtris lie in the block at nodes
     DeviceTree view() const { return DeviceTree{nodes, tris, wnodes, wtris, n_tris}; }
     int32_t* face_vidx = nullptr;  // [F, 3] (meshes only), uploaded on first use
     int32_t* face_slot = nullptr;  // [F] soup slot of each face id, -1 if none
@@ -171,14 +172,23 @@ int device_copy(cubvh_bvh* h, DevCopy** out) {
     if ((e = ensure_constants(device)) != cudaSuccess) return cuda_fail(e, "constant upload");
     DevCopy d;
     d.device = device;
-    const size_t nb = h->host.nodes.size() * sizeof(CNode), tb = h->host.tris.size() * sizeof(CTri);
-    if ((e = cudaMalloc(&d.nodes, nb)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(nodes)");
-    if ((e = cudaMalloc(&d.tris, tb)) != cudaSuccess) { cudaFree(d.nodes); return cuda_fail(e, "cudaMalloc(triangles)"); }
+    // one block for the uploaded and the expanded records: each cudaMalloc and
+    // cudaFree costs a first call 0.1 to 0.2 ms
+    const size_t nn = h->host.nodes.size(), nt = h->host.tris.size();
+    const size_t nb = nn * sizeof(CNode), tb = nt * sizeof(CTri);
+    auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    char* block = nullptr;
+    if ((e = cudaMalloc(reinterpret_cast<void**>(&block), al(nb) + al(tb) + nn * sizeof(WNode) + nt * sizeof(WTri))) != cudaSuccess)
+        return cuda_fail(e, "cudaMalloc(BVH)");
+    d.nodes = reinterpret_cast<CNode*>(block);
+    d.tris = reinterpret_cast<CTri*>(block + al(nb));
+    d.wnodes = reinterpret_cast<WNode*>(block + al(nb) + al(tb));
+    d.wtris = reinterpret_cast<WTri*>(d.wnodes + nn);
+    d.one_block = true;
     if ((e = cudaMemcpy(d.nodes, h->host.nodes.data(), nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(d.tris, h->host.tris.data(), tb, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = expand_copy(h, d, 0)) != cudaSuccess || (e = cudaStreamSynchronize(0)) != cudaSuccess) {
-        cudaFree(d.nodes); cudaFree(d.tris);
-        if (d.wnodes) cudaFree(d.wnodes);
+        cudaFree(block);
         return cuda_fail(e, "BVH upload");
     }
     h->dev.push_back(d);
@@ -458,8 +468,11 @@ int cubvh_bvh_destroy(cubvh_bvh* h) {
     const bool have = cudaGetDevice(&cur) == cudaSuccess;
     for (auto& d : h->dev) {
         if (cudaSetDevice(d.device) == cudaSuccess) {
-            cudaFree(d.nodes); cudaFree(d.tris);
-            if (d.wnodes) cudaFree(d.wnodes);
+            cudaFree(d.nodes);
+            if (!d.one_block) {
+                cudaFree(d.tris);
+                if (d.wnodes) cudaFree(d.wnodes);
+            }
             if (d.face_vidx) cudaFree(d.face_vidx);
             if (d.face_slot) cudaFree(d.face_slot);
             if (d.node_box) cudaFree(d.node_box);
