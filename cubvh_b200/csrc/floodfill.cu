@@ -10,7 +10,7 @@
 // a C-order [D][H][W] array; this implementation uses the same neighbourhood
 // (identical to [H][W][D] when H = W = D).
 //
-// Algorithm (four kernels, no host round trip).  A row is W consecutive
+// Algorithm (three kernels, no host round trip).  A row is W consecutive
 // voxels of memory; a run is a maximal stretch of free voxels in a row.
 //   1. tile     one block per tile of T consecutive rows of one z-slice,
 //               four bitmask words per thread: packs the tile's free-voxel
@@ -28,19 +28,14 @@
 //               above; lock-free union-find on the global roots that always
 //               links the larger root under the smaller, so every root is
 //               its component's smallest run id, i.e. smallest voxel index
-//   3. resolve  every run's label = its root's first voxel (for the tiles
-//               the label writer does not stage)
-//   4. label    one block per tile: the tile's run labels (each run's
+//   3. label    one block per tile: the tile's run labels (each run's
 //               root's first voxel), start marks and run bases staged in
 //               shared memory, then the int32 labels (or the signed
-//               distances of udf_to_sdf) written with 16-byte streaming
-//               stores; rows of W % 32 != 0 voxels: a warp per 32 words
-//               over the resolved labels
-// The tile kernel keeps the bitmask and every row's first run id (rowid);
-// for the row-wise label writer (rows of W % 32 != 0 voxels) also per word
-// its run starts (starts) and the id of the last run that starts before it
-// (wbase: the run covering bit x of word w is wbase[w] + popc(starts[w] &
-// bits 0..x) - 1).  The tile label writer recomputes both from the bitmask.
+//               distances of udf_to_sdf) written: 16-byte streaming stores,
+//               or for rows of W % 32 != 0 voxels and unaligned arrays a warp
+//               per word, 128 bytes a store
+// The tile kernel keeps the bitmask and every row's first run id (rowid); the
+// label writer recomputes run starts and bases from the bitmask.
 #include <algorithm>
 #include <climits>
 #include <cstdint>
@@ -67,11 +62,11 @@ constexpr int kSmemRuns = 12 * kTileThreads;   // a tile's runs unite (and are l
 struct FFPlan {
     int64_t rows, wpr, words, ntot;
     int H, W;
-    int wpr_shift;                     // log2(wpr) when wpr is a power of two, else -1
+    uint32_t wpr_magic;                // ceil(2^32 / wpr): word -> row of its tile (word_pos)
     int tile_rows;                     // T: rows per tile; a tile never spans two z-slices
     int64_t tiles_per_slice, ntiles;
     int64_t cap;                       // run ids per tile: T * ceil(W / 2)
-    size_t off_bits, off_starts, off_wbase, off_rowid, off_tcount, off_start, off_parent, off_status, total;
+    size_t off_bits, off_rowid, off_tcount, off_start, off_parent, off_status, total;
 };
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -83,9 +78,7 @@ FFPlan make_plan(int B, int H, int W, int D) {
     p.wpr = (W + 31) / 32;
     p.words = p.rows * p.wpr;
     p.ntot = p.rows * W;
-    p.wpr_shift = -1;
-    for (int k = 0; k < 31; ++k)
-        if (((int64_t)1 << k) == p.wpr) p.wpr_shift = k;
+    p.wpr_magic = p.wpr > 1 ? (uint32_t)((((uint64_t)1 << 32) + p.wpr - 1) / p.wpr) : 0u;
     // rows per tile: about kTileWords words (one chunk), the slice split evenly;
     // rows of more than kTileWords words: one row per tile, in several chunks
     const int64_t tmax = std::max<int64_t>(1, std::min<int64_t>(H, kTileWords / std::max<int64_t>(p.wpr, 1)));
@@ -101,8 +94,6 @@ FFPlan make_plan(int B, int H, int W, int D) {
     p.ntiles = (int64_t)B * D * p.tiles_per_slice;
     size_t o = 0;
     p.off_bits = o; o = align256(o + sizeof(uint32_t) * p.words);
-    p.off_starts = o; o = align256(o + sizeof(uint32_t) * p.words);
-    p.off_wbase = o; o = align256(o + sizeof(uint32_t) * p.words);
     p.off_rowid = o; o = align256(o + sizeof(uint32_t) * p.rows);
     p.off_tcount = o; o = align256(o + sizeof(uint32_t) * p.ntiles);
     p.off_start = o; o = align256(o + sizeof(int32_t) * p.ntiles * p.cap);
@@ -112,10 +103,13 @@ FFPlan make_plan(int B, int H, int W, int D) {
     return p;
 }
 
-// Row and position in the row of bitmask word w.
-__device__ __forceinline__ void word_pos(int64_t w, int64_t wpr, int shift, int64_t& row, int64_t& wi) {
-    if (shift >= 0) { row = w >> shift; wi = w & (wpr - 1); }
-    else { row = w / wpr; wi = w - row * wpr; }
+// Row in its tile and position in the row of the tile's word w.  A tile of
+// several rows has at most kTileWords words, so w * wpr < 2^20 and the product
+// with ceil(2^32 / wpr) gives the quotient exactly (a 64-bit division per word
+// made ragged grids' tile kernel three times slower).
+__device__ __forceinline__ void word_pos(int w, int T, int wpr, uint32_t magic, int& row, int& wi) {
+    row = T == 1 ? 0 : (wpr == 1 ? w : (int)__umulhi((uint32_t)w, magic));
+    wi = w - row * wpr;
 }
 
 __device__ __forceinline__ uint32_t starts_of(uint32_t f, uint32_t prev_word) {
@@ -160,21 +154,53 @@ __device__ __forceinline__ int32_t uf_root(const int32_t* parent, int32_t x, int
     return x;
 }
 
+// uf_root of x[0 .. 3] (negative: none), the four walks side by side: a walk
+// is a chain of dependent loads.
+__device__ __forceinline__ void uf_root4(const int32_t* parent, int32_t x[4], int* status) {
+    int32_t p[4];
+    bool go = false;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = x[j] >= 0 ? parent[x[j]] : x[j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) go |= p[j] != x[j];
+    int steps = 0;
+    while (go) {
+        go = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const bool up = p[j] != x[j];
+            x[j] = p[j];
+            if (up) p[j] = parent[x[j]];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) go |= p[j] != x[j];
+        if (++steps > kStepLimit) { atomicExch(status, 1); break; }
+    }
+}
+
 // Free-voxel sources of the tile kernel: a bool grid (free = 0) or an
 // unsigned-distance grid thresholded at eps (free = !(udf < eps), so a NaN
 // distance is free).  vec: W % 32 == 0 and a 16-byte aligned array, so a
-// tile's voxels are whole words and are read 16 bytes per load.
+// tile's voxels are whole words and are read 16 bytes per load; else a lane
+// loads voxel i and takes its value.
 struct GridSrc {
     const uint8_t* g;
     bool vec;
-    __device__ __forceinline__ bool free_at(int64_t i) const { return g[i] == 0; }
+    typedef uint8_t Value;
+    __device__ __forceinline__ uint8_t load(int64_t i) const { return __ldcs(g + i); }
+    __device__ __forceinline__ bool take(int64_t, uint8_t v) const { return v == 0; }
 };
 struct UdfSrc {
     const float* u;
     float eps;
     bool vec;
-    float* d;   // vec: receives udf - eps (the unsigned part of the signed grid) as the udf is read
-    __device__ __forceinline__ bool free_at(int64_t i) const { return !(__ldg(u + i) < eps); }
+    float* d;   // receives udf - eps (the unsigned part of the signed grid) as the udf is read
+    typedef float Value;
+    __device__ __forceinline__ float load(int64_t i) const { return __ldcs(u + i); }
+    __device__ __forceinline__ bool take(int64_t i, float v) const {
+        __stcs(d + i, __fsub_rn(v, eps));
+        return !(v < eps);
+    }
 };
 
 // Packs voxels [v0, v0 + 32 * nwords) (whole rows, W % 32 == 0) into nwords
@@ -236,6 +262,33 @@ __device__ __forceinline__ void pack_vec(const UdfSrc& s, int64_t v0, int nwords
     }
 }
 
+// The same for any W and alignment: words k of the tile chunk (rows from r0,
+// tile-relative word of k: c0 + k) by a warp each, a lane a voxel, four words'
+// loads in flight.
+template <class Src>
+__device__ __forceinline__ void pack_rows(const Src& s, int64_t r0, int c0, int nw, int W, int T, int wpr, uint32_t magic,
+                                          uint32_t* sout, uint32_t* gout) {
+    const int lane = threadIdx.x & 31;
+    for (int k0 = 4 * (threadIdx.x >> 5); k0 < nw; k0 += 4 * kTileWarps) {
+        typename Src::Value v[4];
+        int64_t at[4];
+        bool in[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            int row, wi;
+            word_pos(c0 + k0 + j, T, wpr, magic, row, wi);
+            in[j] = k0 + j < nw && wi * 32 + lane < W;
+            at[j] = (r0 + row) * W + wi * 32 + lane;
+            v[j] = in[j] ? s.load(at[j]) : typename Src::Value(0);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, in[j] && s.take(at[j], v[j]));
+            if (lane == 0 && k0 + j < nw) put_word(sout, gout, k0 + j, m);
+        }
+    }
+}
+
 // Exclusive scan of one value per thread over the block (kTileThreads
 // threads); *total receives the block's sum.  Called by all threads; wsum:
 // kTileWarps + 1 words of shared memory, free again after the next barrier.
@@ -271,9 +324,8 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* wsum, 
 // Thread t owns words 4t .. 4t + 3 of the chunk.
 template <class Src>
 __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSM)
-k_ff_tile(Src src, int W, int64_t wpr, int shift, int T, int64_t tiles_per_slice, int H, int64_t cap,
-          bool store_words, uint32_t* __restrict__ bits, uint32_t* __restrict__ starts, uint32_t* __restrict__ wbase,
-          uint32_t* __restrict__ rowid,
+k_ff_tile(Src src, int W, int wpr, uint32_t magic, int T, int64_t tiles_per_slice, int H, int64_t cap,
+          uint32_t* __restrict__ bits, uint32_t* __restrict__ rowid,
           uint32_t* __restrict__ tcount, int32_t* __restrict__ start, int32_t* __restrict__ parent,
           int* __restrict__ status) {
     __shared__ __align__(16) uint32_t sbits[kTileWords];
@@ -299,15 +351,7 @@ k_ff_tile(Src src, int W, int64_t wpr, int shift, int T, int64_t tiles_per_slice
         if (src.vec) {
             pack_vec(src, g0 * 32, nw, sbits, bits + g0);
         } else {
-            const int lane = threadIdx.x & 31;
-            for (int k = threadIdx.x >> 5; k < nw; k += kTileWarps) {
-                int64_t row, wi;
-                word_pos(g0 + k, wpr, shift, row, wi);
-                const int x = (int)wi * 32 + lane;
-                const bool fr = x < W && src.free_at(row * W + x);
-                const uint32_t m = __ballot_sync(0xFFFFFFFFu, fr);
-                if (lane == 0) put_word(sbits, bits + g0, k, m);
-            }
+            pack_rows(src, r0, (int)c0, nw, W, T, wpr, magic, sbits, bits + g0);
         }
         __syncthreads();
         // run starts of the thread's words, their counts scanned over the block
@@ -317,8 +361,8 @@ k_ff_tile(Src src, int W, int64_t wpr, int shift, int T, int64_t tiles_per_slice
             const int w = t4 + j;
             st[j] = 0u;
             if (w < nw) {
-                int64_t row, wi;
-                word_pos(g0 + w, wpr, shift, row, wi);
+                int row, wi;
+                word_pos((int)c0 + w, T, wpr, magic, row, wi);
                 const uint32_t prev = wi == 0 ? 0u : (w > 0 ? sbits[w - 1] : bits[g0 - 1]);
                 st[j] = starts_of(sbits[w], prev);
             }
@@ -334,15 +378,11 @@ k_ff_tile(Src src, int W, int64_t wpr, int shift, int T, int64_t tiles_per_slice
             const int w = t4 + j;
             if (w < nw) {
                 sw[w] = run;
-                if (store_words) {
-                    starts[g0 + w] = st[j];
-                    wbase[g0 + w] = (uint32_t)(tbase + run);
-                }
-                int64_t row, wi;
-                word_pos(g0 + w, wpr, shift, row, wi);
-                if (wi == 0) rowid[row] = (uint32_t)(tbase + run);   // the row's first run
+                int row, wi;
+                word_pos((int)c0 + w, T, wpr, magic, row, wi);
+                if (wi == 0) rowid[r0 + row] = (uint32_t)(tbase + run);   // the row's first run
                 if (st[j]) {
-                    const int64_t v0 = row * W + wi * 32;   // < 2^31 voxels (host check)
+                    const int64_t v0 = (r0 + row) * W + wi * 32;   // < 2^31 voxels (host check)
                     uint32_t sj = st[j];
                     int32_t id = (int32_t)run;
                     while (sj) {
@@ -371,9 +411,9 @@ k_ff_tile(Src src, int W, int64_t wpr, int shift, int T, int64_t tiles_per_slice
         for (int j = 0; j < 4; ++j) {
             const int w = t4 + j;
             if (w < wpr || w >= nwords) continue;
-            const int q = w - (int)wpr;
-            int64_t row, wi;
-            word_pos(w0 + w, wpr, shift, row, wi);
+            const int q = w - wpr;
+            int row, wi;
+            word_pos(w, T, wpr, magic, row, wi);
             const uint32_t pw = wi ? sbits[w - 1] : 0u, pq = wi ? sbits[q - 1] : 0u;
             const uint32_t f = sbits[w], fq = sbits[q];
             const uint32_t sr = starts_of(f, pw), sq = starts_of(fq, pq);
@@ -479,43 +519,24 @@ __global__ void k_ff_merge(const uint32_t* __restrict__ bits, const uint32_t* __
     }
 }
 
-// 3. start[run] := start[root] for every run of the tiles with more than
-// `skip_upto` runs (a root's own entry is already its label, and only
-// non-root entries are written, so concurrent readers of roots' entries see
-// final values).  The tile label writer resolves the runs of the tiles it
-// stages in shared memory itself (skip_upto = kSmemRuns).
-__global__ void k_ff_resolve(const uint32_t* __restrict__ tcount, int64_t ntiles, int64_t cap,
-                             const int32_t* __restrict__ parent, int32_t* __restrict__ start,
-                             int* __restrict__ status, uint32_t skip_upto) {
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int32_t n = (int32_t)tcount[tile];
-        if ((uint32_t)n <= skip_upto) continue;
-        const int32_t base = (int32_t)(tile * cap);
-        for (int32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const int32_t g = base + i;
-            const int32_t root = uf_root(parent, g, status);
-            if (root != g) start[g] = start[root];
-        }
-    }
-}
-
-// 4 (W % 32 == 0, 16-byte aligned output).  One block per tile: the tile's
-// run labels (up to kSmemRuns) and its words' free bits are staged in shared
-// memory with coalesced loads, the words' run starts and run bases
-// (tile-relative) recomputed from the bits with one block-wide scan, then
+// 3. One block per tile: the tile's run labels (up to kSmemRuns) and its
+// words' free bits are staged in shared memory with coalesced loads, the
+// words' run starts and run bases (tile-relative) recomputed from the bits
+// with one block-wide scan, then (VEC: W % 32 == 0, 16-byte aligned output)
 // each thread writes groups of 4 voxels (bits 4k .. 4k + 3 of a word) with
-// 16-byte streaming stores, consecutive threads consecutive groups.
+// 16-byte streaming stores, consecutive threads consecutive groups; else a
+// warp writes a word's voxels, a lane each.
 // SDF: the signed distance s = udf - eps instead of the label, negated where
 // the voxel's label (-1 when occupied) differs from the label of its
 // volume's first voxel (b, 0, 0, 0) and s > 0; the tile kernel has already
 // stored s (reading the udf once), so only groups holding a voxel to negate
 // are read and rewritten.
-template <bool SDF>
+template <bool SDF, bool VEC>
 __global__ void __launch_bounds__(kTileThreads)
 k_write_tile(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ rowid,
-             const uint32_t* __restrict__ tcount, const int32_t* __restrict__ runlab,
-             const int32_t* __restrict__ parent, int* __restrict__ status, int64_t wpr, int shift, int T,
-             int64_t tiles_per_slice, int H, int64_t cap, int4* __restrict__ labels, float4* __restrict__ sdf,
+             const uint32_t* __restrict__ tcount, int32_t* __restrict__ runlab,
+             const int32_t* __restrict__ parent, int* __restrict__ status, int W, int wpr, uint32_t magic, int T,
+             int64_t tiles_per_slice, int H, int64_t cap, int32_t* __restrict__ labels, float* __restrict__ sdf,
              int64_t rows_per_volume) {
     __shared__ int32_t slab[kSmemRuns];
     __shared__ __align__(16) uint32_t sf[kTileWords], ss[kTileWords], sb[kTileWords];
@@ -535,15 +556,33 @@ k_write_tile(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ row
         const int64_t rv = (r0 / rows_per_volume) * rows_per_volume;
         if (bits[rv * wpr] & 1u) empty = runlab[uf_root(parent, (int32_t)rowid[rv], status)];
     }
-    // staged tiles: each run's label is its root's first voxel (k_ff_resolve
-    // skipped these tiles); other tiles' labels were resolved in place
+    // each run's label is its root's first voxel: staged, or for a tile with
+    // more runs than fit resolved in place.  A root's own entry is its label
+    // already and stays as it is, so other blocks reading roots see final values.
     bool other = !inl;   // SDF: the tile may hold a run whose label differs from empty
-    if (inl)
-        for (uint32_t i = threadIdx.x; i < n; i += kTileThreads) {
-            const int32_t l = runlab[uf_root(parent, (int32_t)(tbase + i), status)];
-            slab[i] = l;
-            other |= l != empty;
+    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 4 * kTileThreads) {
+        int32_t root[4], l[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t i = i0 + j * kTileThreads;
+            root[j] = i < n ? (int32_t)(tbase + i) : -1;
         }
+        uf_root4(parent, root, status);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) l[j] = root[j] >= 0 ? runlab[root[j]] : -1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t i = i0 + j * kTileThreads;
+            if (i >= n) continue;
+            if (inl) {
+                slab[i] = l[j];
+                other |= l[j] != empty;
+            } else if (root[j] != (int32_t)(tbase + i)) {
+                runlab[tbase + i] = l[j];
+            }
+        }
+    }
+    if (!inl) __syncthreads();
     // SDF: sdf already holds udf - eps, and only free voxels of runs labelled
     // differently from the volume's first voxel can flip; a tile with none
     // is done
@@ -565,8 +604,8 @@ k_write_tile(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ row
             const int w = t4 + j;
             stw[j] = 0u;
             if (w < nw) {
-                int64_t k, wi;
-                word_pos(c0 + w, wpr, shift, k, wi);
+                int k, wi;
+                word_pos((int)c0 + w, T, wpr, magic, k, wi);
                 const uint32_t prev = wi == 0 ? 0u : (w > 0 ? sf[w - 1] : bits[g0 - 1]);
                 stw[j] = starts_of(sf[w], prev);
             }
@@ -581,7 +620,35 @@ k_write_tile(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ row
         }
         carry += total;
         __syncthreads();
-        for (int g = threadIdx.x; g < 8 * nw; g += kTileThreads) {
+        if (!VEC) {
+            const int lane = threadIdx.x & 31;
+            const uint32_t upto = lane == 31 ? 0xFFFFFFFFu : ((2u << lane) - 1u);
+            for (int k0 = 4 * (threadIdx.x >> 5); k0 < nw; k0 += 4 * kTileWarps) {   // four words in flight
+                int64_t i[4];
+                int32_t l[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int k = min(k0 + j, nw - 1);
+                    int row, wi;
+                    word_pos((int)c0 + k, T, wpr, magic, row, wi);
+                    const int x = wi * 32 + lane;
+                    i[j] = k0 + j < nw && x < W ? (r0 + row) * W + x : -1;
+                    l[j] = ((sf[k] >> lane) & 1u) ? lab[sb[k] + __popc(ss[k] & upto) - 1] : -1;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (i[j] < 0) continue;
+                    if (SDF) {   // a voxel flips as below
+                        if (l[j] >= 0 && l[j] != empty) {
+                            const float v = sdf[i[j]];
+                            if (v > 0.f) __stcs(sdf + i[j], -v);
+                        }
+                    } else {
+                        __stcs(labels + i[j], l[j]);
+                    }
+                }
+            }
+        } else for (int g = threadIdx.x; g < 8 * nw; g += kTileThreads) {
             const size_t i4 = (size_t)g0 * 8 + g;     // 16-byte group of the whole grid
             const int k = g >> 3;
             const uint32_t q = (uint32_t)(g & 7) * 4;
@@ -603,112 +670,61 @@ k_write_tile(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ row
 #pragma unroll
                 for (int j = 0; j < 4; ++j) any |= o[j] >= 0 && o[j] != empty;
                 if (any) {
-                    const float4 v = sdf[i4];
+                    float4* const s4 = reinterpret_cast<float4*>(sdf) + i4;
+                    const float4 v = *s4;
                     float d[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         if (o[j] != empty && d[j] > 0.f) d[j] = -d[j];
-                    __stcs(sdf + i4, make_float4(d[0], d[1], d[2], d[3]));
+                    __stcs(s4, make_float4(d[0], d[1], d[2], d[3]));
                 }
             } else {
-                __stcs(labels + i4, make_int4(o[0], o[1], o[2], o[3]));
+                __stcs(reinterpret_cast<int4*>(labels) + i4, make_int4(o[0], o[1], o[2], o[3]));
             }
         }
         __syncthreads();
     }
 }
 
-// 4 (rows of W % 32 != 0 voxels): one warp writes 32 consecutive voxels per
-// store (128 B).  Lane k of the warp decodes word w0 + k once (its row, its
-// first voxel and how many of its 32 bits lie inside the row); the loop over
-// the 32 words then only shuffles those values.  SDF as k_write_tile.
-template <bool SDF>
-__global__ void k_write_rows(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ starts,
-                             const uint32_t* __restrict__ wbase, const int32_t* __restrict__ runlab,
-                             int32_t* __restrict__ labels, const float* __restrict__ udf, float* __restrict__ sdf,
-                             int64_t rows, int64_t wpr, int W, int64_t rows_per_volume, float eps) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t words = rows * wpr;
-    const uint32_t below = (lane == 31) ? 0xFFFFFFFFu : ((2u << lane) - 1u);
-    for (int64_t w0 = warp * 32; w0 < words; w0 += nwarps * 32) {
-        const int64_t wk = w0 + lane;
-        uint32_t f = 0, s = 0, base = 0, vb = 0;
-        int nval = 0;
-        int32_t empty = -1;
-        if (wk < words) {
-            const int64_t r = wk / wpr, wi = wk - r * wpr;
-            f = bits[wk];
-            s = starts[wk];
-            base = wbase[wk];
-            vb = (uint32_t)(r * W + wi * 32);   // < 2^31 voxels (checked on the host)
-            nval = min(32, W - (int)wi * 32);
-            if (SDF) {
-                const int64_t rv = (r / rows_per_volume) * rows_per_volume;
-                if (bits[rv * wpr] & 1u) empty = __ldg(runlab + wbase[rv * wpr]);
-            }
-        }
-        const int nw = (int)min((int64_t)32, words - w0);
-        for (int k = 0; k < nw; ++k) {
-            const uint32_t fk = __shfl_sync(0xFFFFFFFFu, f, k);
-            const uint32_t sk = __shfl_sync(0xFFFFFFFFu, s, k);
-            const uint32_t bk = __shfl_sync(0xFFFFFFFFu, base, k);
-            const uint32_t vk = __shfl_sync(0xFFFFFFFFu, vb, k);
-            const int nk = __shfl_sync(0xFFFFFFFFu, nval, k);
-            const int32_t ek = SDF ? __shfl_sync(0xFFFFFFFFu, empty, k) : -1;
-            if (lane < nk) {
-                int32_t lab = -1;
-                if ((fk >> lane) & 1u) lab = __ldg(runlab + (bk + __popc(sk & below) - 1));
-                if (SDF) {
-                    const float d = __fsub_rn(__ldcs(udf + vk + lane), eps);
-                    __stcs(sdf + vk + lane, (lab != ek && d > 0.f) ? -d : d);
-                } else {
-                    __stcs(labels + vk + lane, lab);
-                }
-            }
-        }
-    }
-}
-
 __global__ void k_zero(int* p) { *p = 0; }
 
 struct FFBufs {
-    uint32_t *bits, *starts, *wbase, *rowid, *tcount;
+    uint32_t *bits, *rowid, *tcount;
     int32_t *start, *parent;
     int* status;
 };
 FFBufs carve(const FFPlan& p, void* ws) {
     char* base = static_cast<char*>(ws);
-    return FFBufs{reinterpret_cast<uint32_t*>(base + p.off_bits), reinterpret_cast<uint32_t*>(base + p.off_starts),
-                  reinterpret_cast<uint32_t*>(base + p.off_wbase), reinterpret_cast<uint32_t*>(base + p.off_rowid),
+    return FFBufs{reinterpret_cast<uint32_t*>(base + p.off_bits), reinterpret_cast<uint32_t*>(base + p.off_rowid),
                   reinterpret_cast<uint32_t*>(base + p.off_tcount),
                   reinterpret_cast<int32_t*>(base + p.off_start), reinterpret_cast<int32_t*>(base + p.off_parent),
                   reinterpret_cast<int*>(base + p.off_status)};
 }
 
-// 1-3: tiles, cross-tile unions, run labels (start[] := label of each run)
-// tile_writer: the labels are written by k_write_tile, which resolves the
-// runs of the tiles it stages itself.
+// 1-2: tiles, cross-tile unions
 template <class Src>
-void label_runs(const FFPlan& p, int D, const Src& src, const FFBufs& b, unsigned sgrid, bool tile_writer,
-                cudaStream_t stream) {
+void label_runs(const FFPlan& p, int D, const Src& src, const FFBufs& b, cudaStream_t stream) {
     k_zero<<<1, 1, 0, stream>>>(b.status); count_launch();
     k_ff_tile<Src><<<(unsigned)p.ntiles, kTileThreads, 0, stream>>>(
-        src, p.W, p.wpr, p.wpr_shift, p.tile_rows, p.tiles_per_slice, p.H, p.cap, !tile_writer, b.bits, b.starts,
-        b.wbase, b.rowid, b.tcount, b.start, b.parent, b.status); count_launch();
+        src, p.W, (int)p.wpr, p.wpr_magic, p.tile_rows, p.tiles_per_slice, p.H, p.cap, b.bits, b.rowid, b.tcount, b.start,
+        b.parent, b.status); count_launch();
     const unsigned mgrid = (unsigned)((2 * p.rows + 255) / 256);
     k_ff_merge<<<mgrid, 256, 0, stream>>>(b.bits, b.rowid, b.parent, b.status, p.rows, p.wpr, p.H, D,
                                           p.tile_rows); count_launch();
-    k_ff_resolve<<<sgrid, 256, 0, stream>>>(b.tcount, p.ntiles, p.cap, b.parent, b.start, b.status,
-                                            tile_writer ? (uint32_t)kSmemRuns : 0u); count_launch();
 }
-
-unsigned stream_grid() {
-    int dev = 0, nsm = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    return (unsigned)nsm * 8;
+// 3
+template <bool SDF>
+void write_tiles(const FFPlan& p, const FFBufs& b, bool vec, int32_t* labels, float* sdf, int64_t rows_per_volume,
+                 cudaStream_t stream) {
+    if (vec)
+        k_write_tile<SDF, true><<<(unsigned)p.ntiles, kTileThreads, 0, stream>>>(
+            b.bits, b.rowid, b.tcount, b.start, b.parent, b.status, p.W, (int)p.wpr, p.wpr_magic, p.tile_rows,
+            p.tiles_per_slice, p.H, p.cap, labels, sdf, rows_per_volume);
+    else
+        k_write_tile<SDF, false><<<(unsigned)p.ntiles, kTileThreads, 0, stream>>>(
+            b.bits, b.rowid, b.tcount, b.start, b.parent, b.status, p.W, (int)p.wpr, p.wpr_magic, p.tile_rows,
+            p.tiles_per_slice, p.H, p.cap, labels, sdf, rows_per_volume);
+    count_launch();
 }
 
 }  // namespace
@@ -721,18 +737,9 @@ cudaError_t launch_floodfill(const uint8_t* grid, int B, int H, int W, int D, in
     const FFPlan p = make_plan(B, H, W, D);
     if (p.ntot <= 0) return cudaSuccess;
     const FFBufs b = carve(p, ws);
-    const unsigned sgrid = stream_grid();
     const GridSrc src{grid, W % 32 == 0 && (reinterpret_cast<uintptr_t>(grid) & 15) == 0};
-    const bool tile_writer = W % 32 == 0 && (reinterpret_cast<uintptr_t>(labels) & 15) == 0;
-    label_runs(p, D, src, b, sgrid, tile_writer, stream);
-    if (tile_writer) {
-        k_write_tile<false><<<(unsigned)p.ntiles, kTileThreads, 0, stream>>>(
-            b.bits, b.rowid, b.tcount, b.start, b.parent, b.status, p.wpr, p.wpr_shift, p.tile_rows,
-            p.tiles_per_slice, p.H, p.cap, reinterpret_cast<int4*>(labels), nullptr, 1); count_launch();
-    } else {
-        k_write_rows<false><<<sgrid, 256, 0, stream>>>(b.bits, b.starts, b.wbase, b.start, labels, nullptr, nullptr,
-                                                       p.rows, p.wpr, W, 1, 0.f); count_launch();
-    }
+    label_runs(p, D, src, b, stream);
+    write_tiles<false>(p, b, W % 32 == 0 && (reinterpret_cast<uintptr_t>(labels) & 15) == 0, labels, nullptr, 1, stream);
     return cudaGetLastError();
 }
 
@@ -741,19 +748,10 @@ cudaError_t launch_udf_to_sdf(const float* udf, int B, int H, int W, int D, floa
     const FFPlan p = make_plan(B, H, W, D);
     if (p.ntot <= 0) return cudaSuccess;
     const FFBufs b = carve(p, ws);
-    const unsigned sgrid = stream_grid();
     const bool vec = W % 32 == 0 && ((reinterpret_cast<uintptr_t>(udf) | reinterpret_cast<uintptr_t>(sdf)) & 15) == 0;
     const UdfSrc src{udf, eps, vec, sdf};
-    label_runs(p, D, src, b, sgrid, vec, stream);
-    if (vec) {
-        k_write_tile<true><<<(unsigned)p.ntiles, kTileThreads, 0, stream>>>(
-            b.bits, b.rowid, b.tcount, b.start, b.parent, b.status, p.wpr, p.wpr_shift, p.tile_rows,
-            p.tiles_per_slice, p.H, p.cap, nullptr, reinterpret_cast<float4*>(sdf), (int64_t)D * H);
-        count_launch();
-    } else {
-        k_write_rows<true><<<sgrid, 256, 0, stream>>>(b.bits, b.starts, b.wbase, b.start, nullptr, udf, sdf, p.rows,
-                                                      p.wpr, W, (int64_t)D * H, eps); count_launch();
-    }
+    label_runs(p, D, src, b, stream);
+    write_tiles<true>(p, b, vec, nullptr, sdf, (int64_t)D * H, stream);
     return cudaGetLastError();
 }
 
