@@ -165,13 +165,118 @@ __device__ __forceinline__ int n_table_triangles(uint32_t inside) {
     return t;
 }
 
-__global__ void k_smc_count(int64_t n, const float* __restrict__ corners, float iso, bool table,
-                            uint32_t* __restrict__ nv, uint32_t* __restrict__ nt) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const Cube c = load_cube(corners, i, iso);
-        nv[i] = __popc(c.cut);
-        nt[i] = (uint32_t)(table ? n_table_triangles(c.inside) : n_triangles(c, iso));
+// Bound: launches and host round trips.  The surface voxels of a 192^3 grid
+// (22 MB of inputs and results: 3.4 us of memory time) take about 105 us of
+// kernels, 52 of them the radix sort's, and three waits (the counts, the
+// merged vertices, the release).  So few launches: the count kernel takes the
+// coordinate bounds along, count and emit scan their own block's counts (a
+// prefix over all voxels is one small launch between them), emit writes the
+// sort's values, merge scans its own run starts; two workspaces instead of
+// twenty allocations; and keys of the smallest type and bit count that hold
+// the range.  213 us a call against 333 with separate bounds, scans, index
+// and head passes and 26-bit keys in 64 bits.
+constexpr int kSmcBlock = 256;
+struct SmcTotals { int32_t lo[3], hi[3]; uint32_t nv, nt; };   // coordinate bounds, vertices, triangles
+
+// Exclusive prefix of v over the block's threads; every thread gets the total.
+__device__ __forceinline__ uint32_t smc_block_scan(uint32_t v, uint32_t* total) {
+    __shared__ uint32_t s_warp[kSmcBlock / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if (lane >= o) inc += t;
     }
+    if (lane == 31) s_warp[w] = inc;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < kSmcBlock / 32; ++k) {
+        before += k < w ? s_warp[k] : 0u;
+        all += s_warp[k];
+    }
+    *total = all;
+    return before + inc - v;
+}
+
+// Per voxel its vertices (low byte) and triangles (high byte); per block their
+// sums and the coordinate bounds.
+__global__ void __launch_bounds__(kSmcBlock) k_smc_count(int64_t n, const int32_t* __restrict__ coords,
+                                                         const float* __restrict__ corners, float iso, bool table,
+                                                         uint16_t* __restrict__ counts, uint2* __restrict__ bsum,
+                                                         int32_t* __restrict__ bbox) {
+    const int64_t i = (int64_t)blockIdx.x * kSmcBlock + threadIdx.x;
+    int lo[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, hi[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
+    uint32_t nv = 0, nt = 0;
+    if (i < n) {
+        const Cube c = load_cube(corners, i, iso);
+        nv = __popc(c.cut);
+        nt = (uint32_t)(table ? n_table_triangles(c.inside) : n_triangles(c, iso));
+        counts[i] = (uint16_t)(nv | (nt << 8));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) lo[k] = hi[k] = coords[3 * i + k];
+    }
+    __shared__ int32_t sb[6];
+    if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? INT32_MAX : INT32_MIN;
+    uint32_t total;
+    smc_block_scan(nv | (nt << 16), &total);   // at most 12 * 256 each
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = __reduce_min_sync(0xFFFFFFFFu, lo[k]);
+        hi[k] = __reduce_max_sync(0xFFFFFFFFu, hi[k]);
+    }
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { atomicMin(&sb[k], lo[k]); atomicMax(&sb[3 + k], hi[k]); }
+    __syncthreads();
+    if (threadIdx.x == 0) bsum[blockIdx.x] = make_uint2(total & 0xFFFFu, total >> 16);
+    if (threadIdx.x < 6) bbox[6 * (int64_t)blockIdx.x + threadIdx.x] = sb[threadIdx.x];
+}
+// One block: exclusive prefixes of the block sums, totals and bounds.
+__global__ void __launch_bounds__(1024) k_smc_top(int64_t nblk, const uint2* __restrict__ bsum,
+                                                  const int32_t* __restrict__ bbox, uint2* __restrict__ bpre,
+                                                  SmcTotals* __restrict__ out) {
+    __shared__ uint2 sh[1024];
+    __shared__ int32_t sb[6];
+    if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? INT32_MAX : INT32_MIN;
+    __syncthreads();
+    const int64_t per = (nblk + 1023) / 1024;
+    const int64_t b0 = threadIdx.x * per, b1 = min(b0 + per, nblk);
+    uint2 s = make_uint2(0u, 0u);
+#pragma unroll 8
+    for (int64_t i = b0; i < b1; ++i) { s.x += bsum[i].x; s.y += bsum[i].y; }
+    int v[6] = {INT32_MAX, INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN, INT32_MIN};
+    for (int64_t i = threadIdx.x; i < nblk; i += 1024)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { v[k] = min(v[k], bbox[6 * i + k]); v[3 + k] = max(v[3 + k], bbox[6 * i + 3 + k]); }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        v[k] = __reduce_min_sync(0xFFFFFFFFu, v[k]);
+        v[3 + k] = __reduce_max_sync(0xFFFFFFFFu, v[3 + k]);
+    }
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { atomicMin(&sb[k], v[k]); atomicMax(&sb[3 + k], v[3 + k]); }
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 1; o < 1024; o <<= 1) {
+        const uint2 t = threadIdx.x >= (unsigned)o ? sh[threadIdx.x - o] : make_uint2(0u, 0u);
+        __syncthreads();
+        sh[threadIdx.x].x += t.x;
+        sh[threadIdx.x].y += t.y;
+        __syncthreads();
+    }
+    uint2 run = threadIdx.x ? sh[threadIdx.x - 1] : make_uint2(0u, 0u);
+#pragma unroll 8
+    for (int64_t i = b0; i < b1; ++i) {
+        const uint2 t = bsum[i];
+        bpre[i] = run;
+        run.x += t.x;
+        run.y += t.y;
+    }
+    if (threadIdx.x < 3) { out->lo[threadIdx.x] = sb[threadIdx.x]; out->hi[threadIdx.x] = sb[3 + threadIdx.x]; }
+    if (threadIdx.x == 1023) { out->nv = sh[1023].x; out->nt = sh[1023].y; }
 }
 
 struct KeyPack {
@@ -185,15 +290,21 @@ __device__ __forceinline__ uint64_t pack_point(int x, int y, int z, const KeyPac
 
 // Vertices (position, edge key) in edge order and triangles (indices into
 // this launch's vertex list, before merging) of every voxel.
-__global__ void k_smc_emit(int64_t n, const int32_t* __restrict__ coords, const float* __restrict__ corners,
-                           float iso, bool table, const uint32_t* __restrict__ vpre, const uint32_t* __restrict__ tpre,
-                           KeyPack kp, float* __restrict__ pos, uint64_t* __restrict__ key,
+template <class Key>
+__global__ void __launch_bounds__(kSmcBlock, 4) k_smc_emit(int64_t n, const int32_t* __restrict__ coords,
+                           const float* __restrict__ corners, float iso, bool table,
+                           const uint16_t* __restrict__ counts, const uint2* __restrict__ bpre, KeyPack kp,
+                           float* __restrict__ pos, Key* __restrict__ key, int32_t* __restrict__ ord,
                            int32_t* __restrict__ tri) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = (int64_t)blockIdx.x * kSmcBlock + threadIdx.x;
+    const uint32_t mine = i < n ? counts[i] : 0u;
+    uint32_t total;
+    const uint32_t before = smc_block_scan((mine & 0xFFu) | ((mine >> 8) << 16), &total);
+    if (mine) {
+        const uint2 base = bpre[blockIdx.x];
         const Cube c = load_cube(corners, i, iso);
-        if (!c.cut) continue;
         const int x = coords[3 * i], y = coords[3 * i + 1], z = coords[3 * i + 2];
-        const uint32_t vb = vpre[i];
+        const uint32_t vb = base.x + (before & 0xFFFFu);
         uint32_t k = vb;
         for (int e = 0; e < 12; ++e) {
             if (!((c.cut >> e) & 1u)) continue;
@@ -213,11 +324,12 @@ __global__ void k_smc_emit(int64_t n, const int32_t* __restrict__ coords, const 
             pos[3 * k + 1] = __fmaf_rn(t, __fsub_rn((float)by, (float)ay), (float)ay);
             pos[3 * k + 2] = __fmaf_rn(t, __fsub_rn((float)bz, (float)az), (float)az);
             const int axis = ax != bx ? 0 : (ay != by ? 1 : 2);
-            key[k] = pack_point(min(ax, bx), min(ay, by), min(az, bz), kp) * 3u + (uint64_t)axis;
+            key[k] = (Key)(pack_point(min(ax, bx), min(ay, by), min(az, bz), kp) * 3u + (uint64_t)axis);
+            ord[k] = (int32_t)k;
             ++k;
         }
-        uint32_t t_out = tpre[i];
-        const uint32_t t_end = tpre[i + 1];  // the count pass's triangles: never write past them
+        uint32_t t_out = base.y + (before >> 16);
+        const uint32_t t_end = t_out + (mine >> 8);  // the count pass's triangles: never write past them
         auto vid = [&](int e) { return (int32_t)(vb + __popc(c.cut & ((1u << e) - 1u))); };
         if (table) {
             // the case table's triangles, written (e0, e2, e1) as the reference does
@@ -229,7 +341,7 @@ __global__ void k_smc_emit(int64_t n, const int32_t* __restrict__ coords, const 
                 tri[3 * t_out + 2] = vid(c_mc_tri[c.inside][3 * t + 1]);
                 ++t_out;
             }
-            continue;
+            return;
         }
         int8_t nxt[12];
         surface_links(c, iso, nxt);
@@ -312,30 +424,33 @@ __global__ void k_smc_emit(int64_t n, const int32_t* __restrict__ coords, const 
     }
 }
 
-__global__ void k_smc_iota(int64_t m, int32_t* __restrict__ a) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
-        a[i] = (int32_t)i;
-}
 
-// sorted keys: head[i] = first of its run; unique id = inclusive scan - 1
-__global__ void k_smc_heads(int64_t m, const uint64_t* __restrict__ key, uint32_t* __restrict__ head) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
-        head[i] = (i == 0 || key[i] != key[i - 1]) ? 1u : 0u;
+// sorted keys: the runs that start in each block
+template <class Key>
+__global__ void __launch_bounds__(kSmcBlock) k_smc_heads(int64_t m, const Key* __restrict__ key,
+                                                         uint32_t* __restrict__ hsum) {
+    const int64_t i = (int64_t)blockIdx.x * kSmcBlock + threadIdx.x;
+    const int c = __syncthreads_count(i < m && (i == 0 || key[i] != key[i - 1]));
+    if (threadIdx.x == 0) hsum[blockIdx.x] = (uint32_t)c;
 }
-// ids: exclusive scan of heads; the run's first (lowest emission index, the
-// sort being stable) supplies the merged vertex's position
-__global__ void k_smc_merge(int64_t m, const uint32_t* __restrict__ head, const uint32_t* __restrict__ ids,
-                            const int32_t* __restrict__ order, const float* __restrict__ pos,
-                            int32_t* __restrict__ map, float* __restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t id = (int32_t)(ids[i] + head[i]) - 1;
-        const int32_t src = order[i];
-        map[src] = id;
-        if (head[i]) {
-            out[3 * id] = pos[3 * src];
-            out[3 * id + 1] = pos[3 * src + 1];
-            out[3 * id + 2] = pos[3 * src + 2];
-        }
+// hsum: exclusive prefixes of the blocks' run starts; the run's first (lowest
+// emission index, the sort being stable) supplies the merged vertex's position
+template <class Key>
+__global__ void __launch_bounds__(kSmcBlock) k_smc_merge(int64_t m, const Key* __restrict__ key,
+                            const uint32_t* __restrict__ hsum, const int32_t* __restrict__ order,
+                            const float* __restrict__ pos, int32_t* __restrict__ map, float* __restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * kSmcBlock + threadIdx.x;
+    const uint32_t head = i < m && (i == 0 || key[i] != key[i - 1]) ? 1u : 0u;
+    uint32_t total;
+    const uint32_t before = smc_block_scan(head, &total);
+    if (i >= m) return;
+    const int32_t id = (int32_t)(hsum[blockIdx.x] + before + head) - 1;
+    const int32_t src = order[i];
+    map[src] = id;
+    if (head) {
+        out[3 * id] = pos[3 * src];
+        out[3 * id + 1] = pos[3 * src + 1];
+        out[3 * id + 2] = pos[3 * src + 2];
     }
 }
 __global__ void k_smc_remap(int64_t n3, const int32_t* __restrict__ map, int32_t* __restrict__ tri) {
@@ -344,19 +459,21 @@ __global__ void k_smc_remap(int64_t n3, const int32_t* __restrict__ map, int32_t
 }
 
 // corner averaging: keys of the 8 corners of every voxel
-__global__ void k_smc_corner_keys(int64_t n, const int32_t* __restrict__ coords, KeyPack kp,
-                                  uint64_t* __restrict__ key, int32_t* __restrict__ idx) {
+template <class Key>
+__global__ void k_smc_corner_keys(int64_t n, const int32_t* __restrict__ coords, KeyPack kp, Key* __restrict__ key,
+                                  int32_t* __restrict__ idx) {
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < 8 * n; j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = j >> 3;
         const int c = (int)(j & 7);
-        key[j] = pack_point(coords[3 * i] + c_corner_off[c][0], coords[3 * i + 1] + c_corner_off[c][1],
-                            coords[3 * i + 2] + c_corner_off[c][2], kp);
+        key[j] = (Key)pack_point(coords[3 * i] + c_corner_off[c][0], coords[3 * i + 1] + c_corner_off[c][1],
+                                 coords[3 * i + 2] + c_corner_off[c][2], kp);
         idx[j] = (int32_t)j;
     }
 }
 // one thread per run of equal corner keys: the mean of the run's values, in
 // run order (voxel order), written back to every member
-__global__ void k_smc_corner_mean(int64_t m, const uint64_t* __restrict__ key, const int32_t* __restrict__ idx,
+template <class Key>
+__global__ void k_smc_corner_mean(int64_t m, const Key* __restrict__ key, const int32_t* __restrict__ idx,
                                   const float* __restrict__ in, float* __restrict__ out) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
         if (i > 0 && key[i] == key[i - 1]) continue;
@@ -367,34 +484,6 @@ __global__ void k_smc_corner_mean(int64_t m, const uint64_t* __restrict__ key, c
         const float mean = __fdiv_rn(sum, (float)cnt);
         for (int64_t q = i; q < j; ++q) out[idx[q]] = mean;
     }
-}
-
-__global__ void k_smc_bounds(int64_t n, const int32_t* __restrict__ coords, int32_t* __restrict__ b) {
-    int lo[3] = {INT32_MAX, INT32_MAX, INT32_MAX}, hi[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) { lo[k] = min(lo[k], coords[3 * i + k]); hi[k] = max(hi[k], coords[3 * i + k]); }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = __reduce_min_sync(0xFFFFFFFFu, lo[k]);
-        hi[k] = __reduce_max_sync(0xFFFFFFFFu, hi[k]);
-    }
-    // warps meet in shared memory, then one atomic per block and bound (the
-    // six global words are the only addresses every block updates)
-    __shared__ int32_t sb[6];
-    if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? INT32_MAX : INT32_MIN;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) { atomicMin(&sb[k], lo[k]); atomicMax(&sb[3 + k], hi[k]); }
-    __syncthreads();
-    if (threadIdx.x < 3) atomicMin(&b[threadIdx.x], sb[threadIdx.x]);
-    else if (threadIdx.x < 6) atomicMax(&b[threadIdx.x], sb[threadIdx.x]);
-}
-__global__ void k_smc_bounds_init(int32_t* b) {
-    if (threadIdx.x < 3) b[threadIdx.x] = INT32_MAX;
-    else if (threadIdx.x < 6) b[threadIdx.x] = INT32_MIN;
 }
 
 unsigned grid_for(int64_t n) {
@@ -443,6 +532,87 @@ struct AsyncTemps {
     }
 };
 
+// Several arrays in one allocation: the places first, the pointers once it is made.
+struct Layout {
+    size_t bytes = 0;
+    template <class T>
+    size_t add(size_t count) {
+        const size_t at = bytes;
+        bytes += (count * sizeof(T) + 255) & ~size_t(255);
+        return at;
+    }
+};
+
+// Every corner's mean over the voxels that share it, by a sort of all corners.
+template <class Key>
+int smc_average(int64_t n, const int32_t* coords, const float* corners, KeyPack kp, int cbits, AsyncTemps& tmp,
+                cudaStream_t s, float* avg, std::string& err) {
+    cudaError_t e;
+    auto fail = [&](cudaError_t x, const char* what) { err = std::string(what) + ": " + cudaGetErrorString(x); return 2; };
+    const int64_t m = 8 * n;
+    size_t tb = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, (Key*)nullptr, (Key*)nullptr, (int32_t*)nullptr, (int32_t*)nullptr,
+                                    (int)m, 0, cbits, s);
+    Layout lay;
+    const size_t o_key = lay.add<Key>(m), o_key2 = lay.add<Key>(m), o_idx = lay.add<int32_t>(m),
+                 o_idx2 = lay.add<int32_t>(m), o_sort = lay.add<char>(tb);
+    char* ws = nullptr;
+    if ((e = tmp.get(&ws, lay.bytes)) != cudaSuccess) return fail(e, "pool allocation");
+    Key *key = reinterpret_cast<Key*>(ws + o_key), *key2 = reinterpret_cast<Key*>(ws + o_key2);
+    int32_t *idx = reinterpret_cast<int32_t*>(ws + o_idx), *idx2 = reinterpret_cast<int32_t*>(ws + o_idx2);
+    k_smc_corner_keys<Key><<<grid_for(m), 256, 0, s>>>(n, coords, kp, key, idx); count_launch();
+    if ((e = cub::DeviceRadixSort::SortPairs(ws + o_sort, tb, key, key2, idx, idx2, (int)m, 0, cbits, s)) != cudaSuccess)
+        return fail(e, "corner sort");
+    count_launch();
+    k_smc_corner_mean<Key><<<grid_for(m), 256, 0, s>>>(m, key2, idx2, corners, avg); count_launch();
+    tmp.put(ws);
+    return 0;
+}
+
+// Vertices and triangles of the m cut edges and t triangles counted: emission,
+// merge by edge key (Key: the smallest type that holds key_bits), remapping.
+template <class Key>
+int smc_vertices(int64_t n, const int32_t* coords, const float* use, float iso, bool table, const uint16_t* counts,
+                 const uint2* bpre, KeyPack kp, int key_bits, int64_t m, int64_t t, AsyncTemps& tmp, cudaStream_t s,
+                 SparseMCResult& out, std::string& err) {
+    cudaError_t e;
+    auto fail = [&](cudaError_t x, const char* what) { err = std::string(what) + ": " + cudaGetErrorString(x); return 2; };
+    const unsigned gm = (unsigned)((m + kSmcBlock - 1) / kSmcBlock);
+    size_t tb = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, tb, (Key*)nullptr, (Key*)nullptr, (int32_t*)nullptr, (int32_t*)nullptr,
+                                    (int)m, 0, key_bits, s);
+    Layout lay;
+    const size_t o_pos = lay.add<float>(3 * m), o_key = lay.add<Key>(m), o_key2 = lay.add<Key>(m),
+                 o_ord = lay.add<int32_t>(m), o_ord2 = lay.add<int32_t>(m), o_map = lay.add<int32_t>(m),
+                 o_hsum = lay.add<uint32_t>((size_t)gm + 1), o_sort = lay.add<char>(tb);
+    char* ws = nullptr;
+    if ((e = tmp.get(&ws, lay.bytes)) != cudaSuccess) return fail(e, "sparse marching cubes buffers");
+    float* pos = reinterpret_cast<float*>(ws + o_pos);
+    Key *key = reinterpret_cast<Key*>(ws + o_key), *key2 = reinterpret_cast<Key*>(ws + o_key2);
+    int32_t *ord = reinterpret_cast<int32_t*>(ws + o_ord), *ord2 = reinterpret_cast<int32_t*>(ws + o_ord2),
+            *map = reinterpret_cast<int32_t*>(ws + o_map);
+    uint32_t* hsum = reinterpret_cast<uint32_t*>(ws + o_hsum);
+    const unsigned g = (unsigned)((n + kSmcBlock - 1) / kSmcBlock);
+    k_smc_emit<Key><<<g, kSmcBlock, 0, s>>>(n, coords, use, iso, table, counts, bpre, kp, pos, key, ord, out.tris);
+    count_launch();
+    // the emission index as the value: the stable sort keeps each key's lowest first
+    if ((e = cub::DeviceRadixSort::SortPairs(ws + o_sort, tb, key, key2, ord, ord2, (int)m, 0, key_bits, s)) != cudaSuccess)
+        return fail(e, "edge key sort");
+    count_launch();
+    k_smc_heads<Key><<<gm, kSmcBlock, 0, s>>>(m, key2, hsum); count_launch();
+    scan::k_top<<<1, 1024, 0, s>>>(hsum, (int64_t)gm); count_launch();   // hsum[gm] = merged vertex count
+    uint32_t u = 0;
+    if ((e = cudaMemcpyAsync(&u, hsum + gm, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+        return fail(e, "sparse marching cubes merge");
+    if ((e = pool_get(tmp.pool, s, &out.verts, (size_t)3 * u)) != cudaSuccess) return fail(e, "vertex buffer");
+    k_smc_merge<Key><<<gm, kSmcBlock, 0, s>>>(m, key2, hsum, ord2, pos, map, out.verts); count_launch();
+    if (t > 0) { k_smc_remap<<<grid_for(3 * t), 256, 0, s>>>(3 * t, map, out.tris); count_launch(); }
+    out.n_verts = u;
+    out.n_tris = t;
+    return 0;
+}
+
 }  // namespace
 
 // Temporaries and results come from the library's pool on `stream`; the
@@ -458,100 +628,54 @@ int sparse_mc_run(const int32_t* coords, const float* corners, int64_t n, float 
     cudaMemPool_t pool = nullptr;
     if ((e = library_pool(&pool)) != cudaSuccess) return fail(e, "memory pool");
     AsyncTemps tmp(pool, s);
-    // coordinate bounds -> key packing (host round trip)
-    int32_t* d_b = nullptr;
-    if ((e = tmp.get(&d_b, 6)) != cudaSuccess) return fail(e, "pool allocation");
-    k_smc_bounds_init<<<1, 32, 0, s>>>(d_b); count_launch();
-    k_smc_bounds<<<grid_for(n), 256, 0, s>>>(n, coords, d_b); count_launch();
-    int32_t b[6];
-    if ((e = cudaMemcpyAsync(b, d_b, sizeof(b), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-        return fail(e, "sparse marching cubes bounds");
-    tmp.put(d_b);
-    const uint64_t rx = (uint64_t)((int64_t)b[3] - b[0] + 2), ry = (uint64_t)((int64_t)b[4] - b[1] + 2),
-                   rz = (uint64_t)((int64_t)b[5] - b[2] + 2);
-    const int key_bits = bits_for(rx) + bits_for(ry) + bits_for(rz) + 2;
-    if (key_bits > 64) { err = "voxel coordinate range too large for 64-bit edge keys"; return 1; }
-    const KeyPack kp{b[0], b[1], b[2], ry, rz};
-    const unsigned g = grid_for(n);
+    const unsigned g = (unsigned)((n + kSmcBlock - 1) / kSmcBlock);
+    Layout lay;
+    const size_t o_counts = lay.add<uint16_t>(n), o_bsum = lay.add<uint2>(g), o_bpre = lay.add<uint2>(g),
+                 o_bbox = lay.add<int32_t>(6 * (size_t)g), o_tot = lay.add<SmcTotals>(1);
+    char* ws = nullptr;
+    if ((e = tmp.get(&ws, lay.bytes)) != cudaSuccess) return fail(e, "pool allocation");
+    uint16_t* counts = reinterpret_cast<uint16_t*>(ws + o_counts);
+    uint2 *bsum = reinterpret_cast<uint2*>(ws + o_bsum), *bpre = reinterpret_cast<uint2*>(ws + o_bpre);
+    int32_t* bbox = reinterpret_cast<int32_t*>(ws + o_bbox);
+    SmcTotals* d_tot = reinterpret_cast<SmcTotals*>(ws + o_tot);
+    // counts, their block prefixes and the coordinate bounds (host round trip)
+    SmcTotals tot{};
+    auto count = [&](const float* from) {
+        k_smc_count<<<g, kSmcBlock, 0, s>>>(n, coords, from, iso, !closed, counts, bsum, bbox); count_launch();
+        k_smc_top<<<1, 1024, 0, s>>>(g, bsum, bbox, bpre, d_tot); count_launch();
+        const cudaError_t x = cudaMemcpyAsync(&tot, d_tot, sizeof(tot), cudaMemcpyDeviceToHost, s);
+        return x == cudaSuccess ? cudaStreamSynchronize(s) : x;
+    };
+    if ((e = count(corners)) != cudaSuccess) return fail(e, "sparse marching cubes counts");
+    const uint64_t rx = (uint64_t)((int64_t)tot.hi[0] - tot.lo[0] + 2), ry = (uint64_t)((int64_t)tot.hi[1] - tot.lo[1] + 2),
+                   rz = (uint64_t)((int64_t)tot.hi[2] - tot.lo[2] + 2);
+    if (bits_for(rx) + bits_for(ry) + bits_for(rz) + 2 > 64) {
+        err = "voxel coordinate range too large for 64-bit edge keys";
+        return 1;
+    }
+    // the keys are mixed-radix numbers below this: 24 bits (three sort passes)
+    // where bits per coordinate make 26 (four) for a 167^3 range
+    const int key_bits = bits_for(rx * ry * rz * 3);
+    const KeyPack kp{tot.lo[0], tot.lo[1], tot.lo[2], ry, rz};
 
     const float* use = corners;
     if (ensure_consistency) {
-        const int64_t m8 = 8 * n;
         float* avg = nullptr;
-        uint64_t *ck = nullptr, *ck2 = nullptr;
-        int32_t *ci = nullptr, *ci2 = nullptr;
-        const int cbits = bits_for(rx) + bits_for(ry) + bits_for(rz);
-        if ((e = tmp.get(&avg, m8)) != cudaSuccess || (e = tmp.get(&ck, m8)) != cudaSuccess ||
-            (e = tmp.get(&ck2, m8)) != cudaSuccess || (e = tmp.get(&ci, m8)) != cudaSuccess ||
-            (e = tmp.get(&ci2, m8)) != cudaSuccess)
-            return fail(e, "pool allocation");
-        k_smc_corner_keys<<<grid_for(m8), 256, 0, s>>>(n, coords, kp, ck, ci); count_launch();
-        size_t tb = 0;
-        char* cub_tmp = nullptr;
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, ck, ck2, ci, ci2, (int)m8, 0, cbits, s);
-        if ((e = tmp.get(&cub_tmp, tb)) != cudaSuccess) return fail(e, "pool allocation");
-        if ((e = cub::DeviceRadixSort::SortPairs(cub_tmp, tb, ck, ck2, ci, ci2, (int)m8, 0, cbits, s)) != cudaSuccess)
-            return fail(e, "corner sort");
-        count_launch();
-        tmp.put(cub_tmp);
-        k_smc_corner_mean<<<grid_for(m8), 256, 0, s>>>(m8, ck2, ci2, corners, avg); count_launch();
-        tmp.put(ck); tmp.put(ck2); tmp.put(ci); tmp.put(ci2);
+        if ((e = tmp.get(&avg, 8 * n)) != cudaSuccess) return fail(e, "pool allocation");
+        const int cbits = bits_for(rx * ry * rz);
+        const int rc = cbits <= 32 ? smc_average<uint32_t>(n, coords, corners, kp, cbits, tmp, s, avg, err)
+                                   : smc_average<uint64_t>(n, coords, corners, kp, cbits, tmp, s, avg, err);
+        if (rc != 0) return rc;
         use = avg;  // freed at scope exit, after the kernels that read it
+        if ((e = count(avg)) != cudaSuccess) return fail(e, "sparse marching cubes counts");
     }
-
-    uint32_t *nv = nullptr, *nt = nullptr, *bs = nullptr;
-    const int64_t nb = scan::num_chunks(n) + 1;
-    if ((e = tmp.get(&nv, n + 1)) != cudaSuccess || (e = tmp.get(&nt, n + 1)) != cudaSuccess ||
-        (e = tmp.get(&bs, nb)) != cudaSuccess)
-        return fail(e, "pool allocation");
-    k_smc_count<<<g, 256, 0, s>>>(n, use, iso, !closed, nv, nt); count_launch();
-    scan::exclusive(nv, bs, n, s);   // nv[n] = total
-    scan::exclusive(nt, bs, n, s);
-    uint32_t tot[2];
-    if ((e = cudaMemcpyAsync(&tot[0], nv + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&tot[1], nt + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-        return fail(e, "sparse marching cubes counts");
-    const int64_t m = tot[0], t = tot[1];
-    float* pos = nullptr;
-    uint64_t *key = nullptr, *key2 = nullptr;
-    int32_t *ord = nullptr, *ord2 = nullptr, *map = nullptr;
-    uint32_t *head = nullptr, *ids = nullptr, *bs2 = nullptr;
+    const int64_t m = tot.nv, t = tot.nt;
     if (m > 0) {
-        const int64_t nb2 = scan::num_chunks(m) + 1;
-        if ((e = tmp.get(&pos, 3 * m)) != cudaSuccess || (e = tmp.get(&key, m)) != cudaSuccess ||
-            (e = tmp.get(&key2, m)) != cudaSuccess || (e = tmp.get(&ord, m)) != cudaSuccess ||
-            (e = tmp.get(&ord2, m)) != cudaSuccess || (e = tmp.get(&map, m)) != cudaSuccess ||
-            (e = tmp.get(&head, m + 1)) != cudaSuccess || (e = tmp.get(&ids, m + 1)) != cudaSuccess ||
-            (e = tmp.get(&bs2, nb2)) != cudaSuccess ||
-            (e = pool_get(pool, s, &out.tris, (size_t)(3 * t))) != cudaSuccess)
-            return fail(e, "sparse marching cubes buffers");
-        k_smc_emit<<<g, 256, 0, s>>>(n, coords, use, iso, !closed, nv, nt, kp, pos, key, out.tris); count_launch();
-        // emission index as the value: the stable sort keeps each key's lowest first
-        k_smc_iota<<<grid_for(m), 256, 0, s>>>(m, ord); count_launch();
-        size_t tb = 0;
-        char* cub_tmp = nullptr;
-        cub::DeviceRadixSort::SortPairs(nullptr, tb, key, key2, ord, ord2, (int)m, 0, key_bits, s);
-        if ((e = tmp.get(&cub_tmp, tb)) != cudaSuccess) return fail(e, "pool allocation");
-        if ((e = cub::DeviceRadixSort::SortPairs(cub_tmp, tb, key, key2, ord, ord2, (int)m, 0, key_bits, s)) !=
-            cudaSuccess)
-            return fail(e, "edge key sort");
-        count_launch();
-        k_smc_heads<<<grid_for(m), 256, 0, s>>>(m, key2, head); count_launch();
-        if ((e = cudaMemcpyAsync(ids, head, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-            return fail(e, "cudaMemcpyAsync");
-        scan::exclusive(ids, bs2, m, s);  // ids[m] = merged vertex count
-        uint32_t u = 0;
-        if ((e = cudaMemcpyAsync(&u, ids + m, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(s)) != cudaSuccess)
-            return fail(e, "sparse marching cubes merge");
-        if ((e = pool_get(pool, s, &out.verts, (size_t)3 * u)) != cudaSuccess)
-            return fail(e, "vertex buffer");
-        k_smc_merge<<<grid_for(m), 256, 0, s>>>(m, head, ids, ord2, pos, map, out.verts); count_launch();
-        if (t > 0) { k_smc_remap<<<grid_for(3 * t), 256, 0, s>>>(3 * t, map, out.tris); count_launch(); }
-        out.n_verts = u;
-        out.n_tris = t;
+        if ((e = pool_get(pool, s, &out.tris, (size_t)(3 * t))) != cudaSuccess) return fail(e, "sparse marching cubes buffers");
+        const int rc = key_bits <= 32
+            ? smc_vertices<uint32_t>(n, coords, use, iso, !closed, counts, bpre, kp, key_bits, m, t, tmp, s, out, err)
+            : smc_vertices<uint64_t>(n, coords, use, iso, !closed, counts, bpre, kp, key_bits, m, t, tmp, s, out, err);
+        if (rc != 0) return rc;
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "sparse marching cubes launch");
     return 0;
