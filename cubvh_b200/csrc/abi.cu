@@ -1060,11 +1060,12 @@ int cubvh_distance_backward(cubvh_bvh* h, const float* points, int64_t n, const 
     cudaStream_t s = (cudaStream_t)stream;
     const int64_t nf = (int64_t)h->ids.size();
     void* ws = nullptr;
-    cudaError_t e = pool_alloc(&ws, backward_workspace_bytes(n, nf), s);
+    const size_t bytes = backward_workspace_bytes(n, nf, grad_vertices != nullptr);
+    cudaError_t e = bytes ? pool_alloc(&ws, bytes, s) : cudaSuccess;
     if (e != cudaSuccess) return cuda_fail(e, "backward workspace allocation");
     e = launch_backward(n, points, face_id, grad_distances, distances, vertices, vertices ? d->face_vidx : nullptr,
                         d->face_slot, d->tris, nf, grad_points, grad_vertices, ws, s);
-    const cudaError_t e2 = cudaFreeAsync(ws, s);
+    const cudaError_t e2 = ws ? cudaFreeAsync(ws, s) : cudaSuccess;
     if (e == cudaSuccess) e = e2;
     if (e != cudaSuccess) return cuda_fail(e, "backward launch");
     return CUBVH_OK;

@@ -94,7 +94,7 @@ cudaError_t launch_expand(int64_t n_nodes, int64_t n_tris, const CNode* nodes, c
 // refit / backward (grad.cu)
 cudaError_t launch_refit(int64_t n_tris, CTri* tris, const int32_t* face_vidx, const float* V, CNode* nodes,
                          float* node_box, const int32_t* level_start, int n_levels, cudaStream_t stream);
-size_t backward_workspace_bytes(int64_t n, int64_t nf);
+size_t backward_workspace_bytes(int64_t n, int64_t nf, bool vertices);   // 0: none needed
 cudaError_t launch_arena_backward(int64_t n, const float* pts, const int64_t* fid, const float* gout,
                                   const float* dist, const int64_t* qoff, int M, const int64_t* face_off,
                                   const int32_t* gslot, const CTri* tris, float* gpts, cudaStream_t stream);
