@@ -1207,6 +1207,14 @@ __global__ void __launch_bounds__(kQBlock) k_udf_few(int64_t n, const float* __r
 }
 
 // ------------------------------------------------------------ watertight
+// A triangle whose FP32 upper bound of the squared distance is below this is in
+// the normal sum; only those near the radius are settled in double.  The bound
+// needs the slack (cp rounded to float moves the distance by less) to stay
+// below 1e-6 itself, so no coordinate above 1e3 takes this way.  A closest
+// point on a vertex has six or more members, whose double tests were a quarter
+// of the sign pass (8.4M points on 82k faces: 5.21 -> 4.89 ms a call; with the
+// list's triangles tested on their frames, tri_d2_w, 4.68).
+constexpr float kInSum = 0.999999e-6f;
 // Sum of unit normals of every triangle whose squared distance to cp is
 // below 1e-6 (src/bvh.cu:356-396; the division by the count does not change
 // the sign and is omitted).  cp lies on the triangle in soup slot `own` (the
@@ -1242,7 +1250,7 @@ __device__ d3 normal_sum(const CNode* __restrict__ nodes, const CTri* __restrict
                 if (d2 - err - slack > 1.000001e-6f) continue;
                 double bary[3]; d3 q;
                 const d3 a = to_d3(t.a), b = to_d3(t.b), c = to_d3(t.c);
-                if (s == own || closest_on_tri_d(cp, a, b, c, bary, &q) < 1e-6) {
+                if (s == own || d2 + err + slack < kInSum || closest_on_tri_d(cp, a, b, c, bary, &q) < 1e-6) {
                     const d3 nr = dcross(dsub(b, a), dsub(c, a));
                     const double len = __dsqrt_rn(ddot(nr, nr));
                     if (len > 0.0) sum = dadd(sum, d3{dD(nr.x, len), dD(nr.y, len), dD(nr.z, len)});
@@ -1257,19 +1265,23 @@ __device__ d3 normal_sum(const CNode* __restrict__ nodes, const CTri* __restrict
 // the same tests in the same order, without the walk from the root, and the
 // unit normals read from the table k_near_lists computed them into (the same
 // operations as normal_sum's).
-__device__ d3 normal_sum_list(const CTri* __restrict__ tris, d3 cp, int own, const int32_t* __restrict__ lst,
+__device__ d3 normal_sum_list(const CTri* __restrict__ tris, const WTri* __restrict__ wtris, d3 cp, int own, const int32_t* __restrict__ lst,
                               int count, const double* __restrict__ nrm) {
     const float3 cf = make_float3(__double2float_rn(cp.x), __double2float_rn(cp.y), __double2float_rn(cp.z));
     const float slack = 1e-9f * (1.f + f3inf(cf));
     d3 sum{0.0, 0.0, 0.0};
     for (int k = 0; k < count; ++k) {
         const int s = __ldg(lst + k);
-        const TriV t = load_tri(tris, s);
+        const float4* tw = reinterpret_cast<const float4*>(wtris + s);
         float err;
-        const float d2 = tri_d2_f(cf, t, &err);
+        const float d2 = tri_d2_w(cf, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
         if (d2 - err - slack > 1.000001e-6f) continue;
-        double bary[3]; d3 q;
-        if (s == own || closest_on_tri_d(cp, to_d3(t.a), to_d3(t.b), to_d3(t.c), bary, &q) < 1e-6)
+        bool in = s == own || d2 + err + slack < kInSum;
+        if (!in) {
+            const TriV t = load_tri(tris, s);
+            in = dist2_on_tri_d(cp, to_d3(t.a), to_d3(t.b), to_d3(t.c)) < 1e-6;
+        }
+        if (in)
             // a zero normal (degenerate triangle) leaves the sum unchanged: its
             // components are never -0, so adding +0 is exact
             sum = dadd(sum, d3{__ldg(nrm + 3 * s), __ldg(nrm + 3 * s + 1), __ldg(nrm + 3 * s + 2)});
@@ -1381,12 +1393,12 @@ __global__ void __launch_bounds__(kQBlock) k_near_lists(int64_t nt, const CNode*
 // point of the query's nearest triangle (soup slot `own`).  LIST: the normal
 // sum over own's candidate list; a query whose list overflowed is queued in
 // ovf for k_sign_watertight_ovf (single BVH).  !LIST: the walk (arenas).
-constexpr int kSignBlocks = 5;   // blocks per SM (8.4M points, whole call: 4 5.41 ms, 5 5.23, 6 5.31)
+constexpr int kSignBlocks = 5;   // blocks per SM (8.4M points, whole call: 4 4.81 ms, 5 4.68, 6 4.72)
 template <bool LIST>
 __global__ void __launch_bounds__(kQBlock, LIST ? kSignBlocks : 1)
 k_sign_watertight(Work w, const uint32_t* __restrict__ order, const float* __restrict__ pts, float* __restrict__ dist,
                   const int32_t* __restrict__ slots, const CNode* __restrict__ nodes, const CTri* __restrict__ tris,
-                  const NearLists near, uint32_t* __restrict__ ovf, unsigned long long* __restrict__ ovf_n,
+                  const WTri* __restrict__ wtris, const NearLists near, uint32_t* __restrict__ ovf, unsigned long long* __restrict__ ovf_n,
                   unsigned long long* __restrict__ ctr, int64_t grab, int block_grabs) {
     __shared__ int s_left;
     if (block_grabs > 0) {
@@ -1411,7 +1423,7 @@ k_sign_watertight(Work w, const uint32_t* __restrict__ order, const float* __res
             ovf[atomicAdd(ovf_n, 1ull)] = (uint32_t)idx;
             continue;
         }
-        const d3 ns = LIST ? normal_sum_list(tris, cp, own, near.lst + (int64_t)own * kNear, nc, near.nrm)
+        const d3 ns = LIST ? normal_sum_list(tris, wtris, cp, own, near.lst + (int64_t)own * kNear, nc, near.nrm)
                            : normal_sum(nodes, tris, cp, root, own);
         // copysign(distance, avg_normal . (p - cp))
         const double s = ddot(ns, dsub(pd, cp));
@@ -2723,7 +2735,7 @@ cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts
         if (near.cnt) {
             const unsigned g = persistent_grid(k_sign_watertight<true>, n);
             const LaunchShape y = yield_shape(g, grabs_for(n, g), yield);
-            k_sign_watertight<true><<<y.grid, kQBlock, 0, stream>>>(work, order, pts, dist, slots, nodes, tris, near, ovf,
+            k_sign_watertight<true><<<y.grid, kQBlock, 0, stream>>>(work, order, pts, dist, slots, nodes, tris, tree.wtris, near, ovf,
                                                                     ctr + kCtOvfN, ctr + kCtSign, grab_for(n, g),
                                                                     y.block_grabs); count_launch();
             if (near.ovf) {
@@ -2733,7 +2745,7 @@ cudaError_t launch_distance(int mode, bool want_uvw, int64_t n, const float* pts
         } else {
             const unsigned g = persistent_grid(k_sign_watertight<false>, n);
             const LaunchShape y = yield_shape(g, grabs_for(n, g), yield);
-            k_sign_watertight<false><<<y.grid, kQBlock, 0, stream>>>(work, order, pts, dist, slots, nodes, tris, near,
+            k_sign_watertight<false><<<y.grid, kQBlock, 0, stream>>>(work, order, pts, dist, slots, nodes, tris, tree.wtris, near,
                                                                      nullptr, nullptr, ctr + kCtSign, grab_for(n, g),
                                                                      y.block_grabs); count_launch();
         }
@@ -2842,7 +2854,7 @@ cudaError_t launch_arena_distance(const ArenaLaunch& a, const float* pts, float*
         const Work w{a.wt_packets, a.meshes, a.n_wt_packets, 0};
         const unsigned gw = persistent_grid(k_sign_watertight<false>, 32 * a.n_wt_packets);
         k_sign_watertight<false><<<gw, kQBlock, 0, stream>>>(w, order, pts, dist, a.slots, a.tree.nodes, a.tree.tris,
-                                                             NearLists{}, nullptr, nullptr, a.counters + kCtSign,
+                                                             a.tree.wtris, NearLists{}, nullptr, nullptr, a.counters + kCtSign,
                                                              grab_for(32 * a.n_wt_packets, gw), 0); count_launch();
     }
     if (a.n_rs_packets > 0) {
