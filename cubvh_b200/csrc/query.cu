@@ -1949,9 +1949,9 @@ __device__ __noinline__ void walk_hits(const CNode* __restrict__ nodes, const CT
 constexpr int kRayBlocks = 8;   // blocks of k_ray per SM
 // Closest hit of 32 rays per warp (a packet: the rays of 4 consecutive
 // entries of `order`, units of 8 consecutive rays sorted so that nearby ones
-// are side by side (k_ray_order); packets k_ray_order marked incoherent are
-// skipped, k_ray_lanes traces them, as it does packets holding a ray that is
-// not finite or has no direction, listed here): warp-uniform walk of the
+// are side by side (k_ray_order, which lists the coherent packets for this
+// kernel and the others for k_ray_lanes; packets holding a ray that is not
+// finite or has no direction are added to its list here): warp-uniform walk of the
 // union of the rays' paths.  At an inner node lane 8 g + j tests child j
 // against unit g in interval arithmetic: what its two halves' origins and
 // directions lie within against the box's planes (group_entry).  Eight
@@ -1969,7 +1969,8 @@ __global__ void __launch_bounds__(kQBlock, kRayBlocks) k_ray(int64_t n, const ui
                                                  const float* __restrict__ rd, float* __restrict__ pos,
                                                  int64_t* __restrict__ face_id, float* __restrict__ depth,
                                                  const DeviceTree tree, unsigned long long* __restrict__ ctr,
-                                                 int64_t grab, const uint8_t* __restrict__ skip,
+                                                 int64_t grab, const uint32_t* __restrict__ packets,
+                                                 const unsigned long long* __restrict__ packets_n,
                                                  uint32_t* __restrict__ lanes,
                                                  unsigned long long* __restrict__ lanes_n) {
     const CTri* __restrict__ tris = tree.tris;
@@ -1978,9 +1979,9 @@ __global__ void __launch_bounds__(kQBlock, kRayBlocks) k_ray(int64_t n, const ui
     __shared__ uint2 s_cand[kQBlock / 32][kCand][32];
     uint2* stk = s_stack[threadIdx.x >> 5];
     uint2* cand = &s_cand[threadIdx.x >> 5][0][lane];   // the lane's candidates, 32 entries apart: slot, lower bound
-    PacketQueue pq(ctr, (n + 31) >> 5, grab);
-    for (int64_t pk = pq.take(); pk >= 0; pk = pq.take()) {
-        if (__ldg(skip + pk)) continue;   // incoherent: k_ray_lanes traces it
+    PacketQueue pq(ctr, (int64_t)*packets_n, grab);
+    for (int64_t at = pq.take(); at >= 0; at = pq.take()) {
+        const int64_t pk = __ldg(packets + at);
         const int64_t q = packet_ray(pk, lane, n, order);
         const bool act = q < n;
         const float3 o = act ? load3(ro, q) : make_float3(0.f, 0.f, 0.f);
@@ -2370,12 +2371,15 @@ __device__ __forceinline__ int ray_entry(float3 o, float3 d, const float lo[3], 
 // window (4 consecutive sorted units) is judged: coherent when each unit's
 // first and last rays lie within kCohDir (unit directions, max-norm) and
 // kCohOrigin (origins) of the unit's fourth ray, and each unit's fourth ray
-// within kCohUnits and kCohOrigin of the first unit's.  skip[p] = 1 marks the others for
-// k_ray, and they are listed for k_ray_lanes.
+// within kCohUnits and kCohOrigin of the first unit's.  The coherent ones are
+// listed for k_ray, the others for k_ray_lanes (with a flag per packet instead,
+// k_ray took 359 us to pass over the packets of 16.8M incoherent rays: an
+// atomic each on its queue; 5M such rays 2.31 -> 2.20 ms a call).
 __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const float* __restrict__ ro,
                                                            const float* __restrict__ rd,
                                                            const CNode* __restrict__ nodes,
-                                                           uint32_t* __restrict__ order, uint8_t* __restrict__ skip,
+                                                           uint32_t* __restrict__ order, uint32_t* __restrict__ packets,
+                                                           unsigned long long* __restrict__ packets_n,
                                                            uint32_t* __restrict__ lanes,
                                                            unsigned long long* __restrict__ lanes_n) {
     using Sort = cub::BlockRadixSort<uint32_t, kOrdThreads, kOrdItems, uint16_t>;
@@ -2479,15 +2483,18 @@ __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const floa
             }
             inc |= s_bad[v] || !(dv <= kCohUnits && dov <= spread_max);
         }
-        skip[pk] = inc ? 1 : 0;
     }
-    const unsigned m = __ballot_sync(kFull, valid && inc);
-    if (m) {                          // one atomic per warp
-        unsigned long long base = 0;
-        if ((t & 31) == __ffs(m) - 1) base = atomicAdd(lanes_n, (unsigned long long)__popc(m));
-        base = __shfl_sync(kFull, base, __ffs(m) - 1);
-        if (valid && inc) lanes[base + __popc(m & ((1u << (t & 31)) - 1u))] = (uint32_t)pk;
-    }
+    auto list = [&](bool in, uint32_t* __restrict__ to, unsigned long long* __restrict__ to_n) {
+        const unsigned m = __ballot_sync(kFull, in);
+        if (m) {                      // one atomic per warp
+            unsigned long long base = 0;
+            if ((t & 31) == __ffs(m) - 1) base = atomicAdd(to_n, (unsigned long long)__popc(m));
+            base = __shfl_sync(kFull, base, __ffs(m) - 1);
+            if (in) to[base + __popc(m & ((1u << (t & 31)) - 1u))] = (uint32_t)pk;
+        }
+    };
+    list(valid && !inc, packets, packets_n);
+    list(valid && inc, lanes, lanes_n);
 }
 
 // --------------------------------------------------------------- launchers
@@ -2526,16 +2533,16 @@ int64_t heavy_cap_for(int64_t n) {
 }
 
 namespace {
-// Ray launch workspace: counters (256 bytes), the unit order, a skip flag
-// per packet, the list of incoherent packets; byte offsets and total.
-struct RayWs { size_t order, skip, lanes, end; };
+// Ray launch workspace: counters (256 bytes), the unit order, the lists of
+// coherent and of incoherent packets; byte offsets and total.
+struct RayWs { size_t order, packets, lanes, end; };
 RayWs ray_ws(int64_t n) {
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t units = (size_t)((n + kUnit - 1) / kUnit), packets = (size_t)((n + 31) / 32);
     RayWs r;
     r.order = 256;
-    r.skip = r.order + al(sizeof(uint32_t) * units);
-    r.lanes = r.skip + al(packets);
+    r.packets = r.order + al(sizeof(uint32_t) * units);
+    r.lanes = r.packets + al(sizeof(uint32_t) * packets);
     r.end = r.lanes + al(sizeof(uint32_t) * packets);
     return r;
 }
@@ -2555,7 +2562,7 @@ size_t query_workspace_bytes(int mode, int64_t n) {
     if (mode == 1) b += al(sizeof(uint32_t) * n);                 // watertight overflow queue
     if (mode >= 0) b += al(sizeof(uint4) * heavy_cap_for(n));     // heavy-query list
     if (mode == 2) b += al(sizeof(uint4) * n);                    // raystab candidates (second pass)
-    if (mode == -1) b = ray_ws(n).end;                           // unit order, skip flags, incoherent packets
+    if (mode == -1) b = ray_ws(n).end;                           // unit order, coherent and incoherent packets
     return b;
 }
 
@@ -2572,8 +2579,9 @@ enum : int {
     kCtCandN = 12,      // raystab second-pass candidates
     kCtLinesNext = 13,  // raystab second-pass queue
     kCtParity = 11,     // edge parity of a single BVH (k_edge_parity)
-    kCtRayLanesN = 14,  // incoherent ray packets listed by k_ray
+    kCtRayLanesN = 14,  // incoherent ray packets
     kCtRayLanesNext = 15,  // k_ray_lanes queue
+    kCtRayPacketsN = 16,   // coherent ray packets
 };
 // packets per atomic grab: about 64 grabs per warp
 int64_t grab_for(int64_t n, unsigned grid) {
@@ -2778,14 +2786,14 @@ cudaError_t launch_ray(int64_t n, const float* ro, const float* rd, float* pos, 
     const RayWs r = ray_ws(n);
     char* w = static_cast<char*>(ws);
     uint32_t* order = reinterpret_cast<uint32_t*>(w + r.order);
-    uint8_t* skip = reinterpret_cast<uint8_t*>(w + r.skip);
+    uint32_t* packets = reinterpret_cast<uint32_t*>(w + r.packets);
     uint32_t* lanes = reinterpret_cast<uint32_t*>(w + r.lanes);
     const int64_t units = (n + kUnit - 1) / kUnit;
     k_ray_order<<<(unsigned)((units + kOrdUnits - 1) / kOrdUnits), kOrdThreads, 0, stream>>>(
-        n, ro, rd, nodes, order, skip, lanes, ctr + kCtRayLanesN); count_launch();
+        n, ro, rd, nodes, order, packets, ctr + kCtRayPacketsN, lanes, ctr + kCtRayLanesN); count_launch();
     const unsigned g = persistent_grid(k_ray, n);
-    k_ray<<<g, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, tree, ctr + kCtUdf, grab_for(n, g), skip, lanes,
-                                     ctr + kCtRayLanesN); count_launch();
+    k_ray<<<g, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, tree, ctr + kCtUdf, grab_for(n, g), packets,
+                                     ctr + kCtRayPacketsN, lanes, ctr + kCtRayLanesN); count_launch();
     const unsigned gl = persistent_grid(k_ray_lanes, n);
     k_ray_lanes<<<gl, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, nodes, tris, lanes,
                                             ctr + kCtRayLanesN, ctr + kCtRayLanesNext); count_launch();
