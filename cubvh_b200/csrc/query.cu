@@ -585,9 +585,9 @@ __device__ __noinline__ void walk_ties(const DeviceTree& tree, int root, float3 
 //
 // Bound by instruction issue and the latency of node and triangle loads.
 // Measured against the walk with a lane per point and the records of
-// layout.h's first half (call times): 1M points on 5,120 faces 1.98 -> 0.99
-// ms, 384^3 grid on 177k faces 107.5 -> 48.0 ms, 8.4M watertight points on
-// 82k faces 9.70 -> 5.52 ms, 1,000 points 1.16 -> 0.22 ms.
+// layout.h's first half (whole calls, today's other passes included): 1M
+// points on 5,120 faces 1.98 -> 0.92 ms, 384^3 grid on 177k faces 107.5 ->
+// 46.2 ms, 8.4M watertight points on 82k faces 9.70 -> 4.88 ms.
 //
 // Heavy queries, served afterwards with a warp each (k_udf_heavy, from the
 // bound found so far): a point whose candidate list overflows (many
@@ -1472,7 +1472,8 @@ __global__ void __launch_bounds__(kQBlock) k_sign_watertight_ovf(const uint32_t*
 // rounding of the double test lets slip between two triangles at their common
 // edge, about 1e-14 of all rays, is not seen this way.)  Inside points took
 // 64 rays, bound by divergence (12.5 of 32 lanes): 2.1M points in the box of a
-// closed 82k-face mesh, 18.9 -> 4.2 ms with the faster distance search.
+// closed 82k-face mesh, 18.9 -> 4.2 ms with the faster distance search (3.1 with
+// today's first pass).
 
 // Hash of an undirected edge by its end points' coordinates (0 for an edge
 // of no length): mesh edges cancel in pairs under XOR.
@@ -2327,9 +2328,9 @@ __global__ void __launch_bounds__(kQBlock, kLaneBlocks) k_ray_lanes(int64_t n, c
 // past the last unit.  A packet is four consecutive units of the sorted
 // order.  Camera rays stored row by row then make packets of 8 pixels from
 // each of 4 neighbouring rows instead of 32 x 1 strips, and the union of the
-// 32 rays' walks visits far fewer nodes (C1 camera rays: k_ray 6.4 -> 5.1
-// ms, for a sort of 1,024 keys per 8,192 rays).  The order changes no
-// result: each ray's hit is its own.
+// 32 rays' walks visits far fewer nodes (33.5M camera rays: k_ray 6.4 -> 5.1
+// ms when it tested every ray, for a sort of 1,024 keys per 8,192 rays, 0.22
+// ms).  The order changes no result: each ray's hit is its own.
 constexpr int kOrdThreads = 256, kOrdItems = 4;
 constexpr int kOrdUnits = kOrdThreads * kOrdItems;    // 1024 units = 8192 rays per window
 // Entry point of ray (o, d) into the box [lo, lo + 255 * 2^ex] (the origin when
