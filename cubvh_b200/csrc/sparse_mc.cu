@@ -320,9 +320,9 @@ __global__ void __launch_bounds__(kSmcBlock, 4) k_smc_emit(int64_t n, const int3
             }
             const int ax = x + c_corner_off[a][0], ay = y + c_corner_off[a][1], az = z + c_corner_off[a][2];
             const int bx = x + c_corner_off[b][0], by = y + c_corner_off[b][1], bz = z + c_corner_off[b][2];
-            pos[3 * k] = __fmaf_rn(t, __fsub_rn((float)bx, (float)ax), (float)ax);
-            pos[3 * k + 1] = __fmaf_rn(t, __fsub_rn((float)by, (float)ay), (float)ay);
-            pos[3 * k + 2] = __fmaf_rn(t, __fsub_rn((float)bz, (float)az), (float)az);
+            pos[3 * (int64_t)k] = __fmaf_rn(t, __fsub_rn((float)bx, (float)ax), (float)ax);
+            pos[3 * (int64_t)k + 1] = __fmaf_rn(t, __fsub_rn((float)by, (float)ay), (float)ay);
+            pos[3 * (int64_t)k + 2] = __fmaf_rn(t, __fsub_rn((float)bz, (float)az), (float)az);
             const int axis = ax != bx ? 0 : (ay != by ? 1 : 2);
             key[k] = (Key)(pack_point(min(ax, bx), min(ay, by), min(az, bz), kp) * 3u + (uint64_t)axis);
             ord[k] = (int32_t)k;
@@ -336,9 +336,9 @@ __global__ void __launch_bounds__(kSmcBlock, 4) k_smc_emit(int64_t n, const int3
             for (int t = 0; t < 5 && t_out < t_end; ++t) {
                 const int e0 = c_mc_tri[c.inside][3 * t];
                 if (e0 < 0) break;
-                tri[3 * t_out] = vid(e0);
-                tri[3 * t_out + 1] = vid(c_mc_tri[c.inside][3 * t + 2]);
-                tri[3 * t_out + 2] = vid(c_mc_tri[c.inside][3 * t + 1]);
+                tri[3 * (int64_t)t_out] = vid(e0);
+                tri[3 * (int64_t)t_out + 1] = vid(c_mc_tri[c.inside][3 * t + 2]);
+                tri[3 * (int64_t)t_out + 2] = vid(c_mc_tri[c.inside][3 * t + 1]);
                 ++t_out;
             }
             return;
@@ -395,9 +395,9 @@ __global__ void __launch_bounds__(kSmcBlock, 4) k_smc_emit(int64_t n, const int3
             }
             if (apex >= 0) {
                 for (int m = 1; m + 1 < L && t_out < t_end; ++m) {
-                    tri[3 * t_out] = vid(q[apex]);
-                    tri[3 * t_out + 1] = vid(q[(apex + m) % L]);
-                    tri[3 * t_out + 2] = vid(q[(apex + m + 1) % L]);
+                    tri[3 * (int64_t)t_out] = vid(q[apex]);
+                    tri[3 * (int64_t)t_out + 1] = vid(q[(apex + m) % L]);
+                    tri[3 * (int64_t)t_out + 2] = vid(q[(apex + m + 1) % L]);
                     ++t_out;
                 }
             } else {
@@ -412,9 +412,9 @@ __global__ void __launch_bounds__(kSmcBlock, 4) k_smc_emit(int64_t n, const int3
                         const int a0 = ring[(m + r - 1) % r], a2 = ring[(m + 1) % r];
                         if (r == 3 || !(mark[a0] & mark[a2])) { ear = m; break; }
                     }
-                    tri[3 * t_out] = vid(ring[(ear + r - 1) % r]);
-                    tri[3 * t_out + 1] = vid(ring[ear]);
-                    tri[3 * t_out + 2] = vid(ring[(ear + 1) % r]);
+                    tri[3 * (int64_t)t_out] = vid(ring[(ear + r - 1) % r]);
+                    tri[3 * (int64_t)t_out + 1] = vid(ring[ear]);
+                    tri[3 * (int64_t)t_out + 2] = vid(ring[(ear + 1) % r]);
                     ++t_out;
                     for (int m = ear; m + 1 < r; ++m) ring[m] = ring[m + 1];
                     --r;
@@ -448,9 +448,10 @@ __global__ void __launch_bounds__(kSmcBlock) k_smc_merge(int64_t m, const Key* _
     const int32_t src = order[i];
     map[src] = id;
     if (head) {
-        out[3 * id] = pos[3 * src];
-        out[3 * id + 1] = pos[3 * src + 1];
-        out[3 * id + 2] = pos[3 * src + 2];
+        const int64_t to = 3 * (int64_t)id, from = 3 * (int64_t)src;
+        out[to] = pos[from];
+        out[to + 1] = pos[from + 1];
+        out[to + 2] = pos[from + 2];
     }
 }
 __global__ void k_smc_remap(int64_t n3, const int32_t* __restrict__ map, int32_t* __restrict__ tri) {
