@@ -1918,33 +1918,55 @@ __device__ __forceinline__ uint32_t group_entry(const RayAxis& X, const RayAxis&
     return key;
 }
 
-// A ray's closest hit by a walk of its own in double, given a bound U of it:
-// for a ray with more triangles at almost the same hit than its list holds.
-__device__ __noinline__ void walk_hits(const CNode* __restrict__ nodes, const CTri* __restrict__ tris, float3 o,
-                                       float3 d, float U, double* bt, int* sx, int* ix) {
-    const float3 inv = ray_inv(d);
-    const bool degen = ray_degenerate(inv);
-    const float cull = U * 1.000002f;
-    int st[kStack];
-    int sp = 0;
-    st[sp++] = 0;
-    while (sp > 0) {
-        const int ref = st[--sp];
-        if (ref >= 0) {
-            const NodeView nd = load_node(nodes, ref);
-            if (degen) push_ray_children<true>(nd, o, inv, cull, st, sp);
-            else push_ray_children<false>(nd, o, inv, cull, st, sp);
-        } else {
-            int s0, s1;
-            leaf_range(ref, s0, s1);
-            for (int s = s0; s < s1; ++s) {
-                const TriV t = load_tri(tris, s);
-                double t64;
-                if (!ray_tri_d(to_d3(o), to_d3(d), to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
-                if (t64 < *bt || (t64 == *bt && (*sx < 0 || t.id < *ix))) { *bt = t64; *sx = s; *ix = t.id; }
-            }
-        }
+// The closest hit in double (ties -> lowest face index) among a ray's first n
+// candidates (32 entries apart) whose lower bound is within U; slot -1: none.
+struct Hit { double t; int slot, id; };
+__device__ __forceinline__ Hit closest_hit(const uint2* cand, int n, float U, const CTri* __restrict__ tris, float3 o,
+                                           float3 d) {
+    Hit h{1000.0, -1, -1};
+    const d3 od = to_d3(o), dd = to_d3(d);
+    for (int i = 0; i < n; ++i) {
+        const uint2 e = cand[32 * i];
+        if (__uint_as_float(e.y) > U) continue;
+        const TriV t = load_tri(tris, (int)e.x);
+        double t64;
+        if (!ray_tri_d(od, dd, to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
+        if (t64 < h.t || (t64 == h.t && (h.slot < 0 || t.id < h.id))) h = Hit{t64, (int)e.x, t.id};
     }
+    return h;
+}
+// A list that the walk has filled holds only its closest hit afterwards, whose
+// distance bounds U.  Lists fill where more triangles than they hold may be
+// the closest hit: faces that are there several times, or edge-on ones at a
+// silhouette.  Settled where the walk meets them they cost their own double
+// tests; a second walk of each such ray, by one lane, held whole launches (1M
+// parallel rays along a height field of 80k faces, 294 of them with a full
+// list: 773 against 430 us a call; 12 copies of 5,120 faces, 65k rays 390
+// against 260).
+__device__ __forceinline__ void keep_hit(const Hit& h, uint2* cand, int& nc, float& U) {
+    nc = 0;
+    if (h.slot < 0) return;
+    cand[0] = make_uint2((uint32_t)h.slot, __float_as_uint(__double2float_rd(h.t)));
+    U = fminf(U, __double2float_ru(h.t));
+    nc = 1;
+}
+// A ray's result.
+__device__ __forceinline__ void write_hit(const Hit& h, int64_t q, float3 o, float3 d, float* __restrict__ pos,
+                                          int64_t* __restrict__ face_id, float* __restrict__ depth) {
+    depth[q] = __double2float_rn(h.t);
+    pos[3 * q] = __double2float_rn(dA((double)o.x, dM(h.t, (double)d.x)));
+    pos[3 * q + 1] = __double2float_rn(dA((double)o.y, dM(h.t, (double)d.y)));
+    pos[3 * q + 2] = __double2float_rn(dA((double)o.z, dM(h.t, (double)d.z)));
+    face_id[q] = h.slot >= 0 ? (int64_t)h.id : (int64_t)-1;
+}
+
+// closest_hit and keep_hit out of line, so that the walks keep their registers
+// (inline in k_ray's loop: 33.5M camera rays 3.41 against 3.08 ms).
+struct Settled { int n; float U; };
+__device__ __noinline__ Settled settle_full(uint2* cand, int n, const CTri* __restrict__ tris, float3 o, float3 d, float U) {
+    Settled e{0, U};
+    keep_hit(closest_hit(cand, n, U, tris, o, d), cand, e.n, e.U);
+    return e;
 }
 
 constexpr int kRayBlocks = 8;   // blocks of k_ray per SM
@@ -1977,7 +1999,7 @@ __global__ void __launch_bounds__(kQBlock, kRayBlocks) k_ray(int64_t n, const ui
     const CTri* __restrict__ tris = tree.tris;
     const int lane = threadIdx.x & 31;
     __shared__ uint2 s_stack[kQBlock / 32][kStack];
-    __shared__ uint2 s_cand[kQBlock / 32][kCand][32];
+    __shared__ uint2 s_cand[kQBlock / 32][kCand + 4][32];
     uint2* stk = s_stack[threadIdx.x >> 5];
     uint2* cand = &s_cand[threadIdx.x >> 5][0][lane];   // the lane's candidates, 32 entries apart: slot, lower bound
     PacketQueue pq(ctr, (int64_t)*packets_n, grab);
@@ -1993,94 +2015,74 @@ __global__ void __launch_bounds__(kQBlock, kRayBlocks) k_ray(int64_t n, const ui
             if (lane == 0) lanes[atomicAdd(lanes_n, 1ull)] = (uint32_t)pk;
             continue;
         }
-        const RayAxis X = ray_axis(o.x, d.x, act), Y = ray_axis(o.y, d.y, act), Z = ray_axis(o.z, d.z, act);
-        const bool mixed = __any_sync(kFull, X.kind == 2 || Y.kind == 2 || Z.kind == 2);
         float U = act ? 1000.0f : -1.f;             // MAX_DIST
-        float c[2];                                 // bounds of the lane's quad and of the other one
-        uint32_t cullmax;
-        auto share_bounds = [&]() {
-            float m = act ? U * 1.000002f : -1.f;
-            cullmax = __reduce_max_sync(kFull, __float_as_uint(fmaxf(m, 0.f)));
-            m = fmaxf(m, __shfl_xor_sync(kFull, m, 1));
-            c[0] = fmaxf(m, __shfl_xor_sync(kFull, m, 2));
-            c[1] = __shfl_xor_sync(kFull, c[0], 4);
-        };
-        share_bounds();
         int nc = 0, sp = 0, cur = 0;
         bool live = true;
-        while (live) {
-            if (cur >= 0) {
-                const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + cur);
-                const int j = lane & 7;
-                const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
-                uint32_t key = mixed ? group_entry<true>(X, Y, Z, lo, hi, c) : group_entry<false>(X, Y, Z, lo, hi, c);
-                key = min(key, __shfl_xor_sync(kFull, key, 8));
-                key = min(key, __shfl_xor_sync(kFull, key, 16));
-                if (key != kFull) key = (key & ~7u) | (uint32_t)j;
-                // its place on the stack: the number of needed children farther than it, two of
-                // the eight compared by each of the four lanes with this child
-                const uint32_t ka = __shfl_sync(kFull, key, 2 * (lane >> 3)), kb = __shfl_sync(kFull, key, 2 * (lane >> 3) + 1);
-                int place = (ka > key && ka != kFull ? 1 : 0) + (kb > key && kb != kFull ? 1 : 0);
-                place += __shfl_xor_sync(kFull, place, 8);
-                place += __shfl_xor_sync(kFull, place, 16);
-                const int kept = __popc(__ballot_sync(kFull, key != kFull) & 0xFFu);
-                __syncwarp();   // the popped entry has been read
-                if (lane < 8 && key != kFull) stk[sp + place] = make_uint2((uint32_t)__float_as_int(lo.w), key & ~7u);
-                sp += kept;
-                __syncwarp();
-            } else {
-                int s0, s1;
-                leaf_range(cur, s0, s1);
-                const float U0 = U;
-                for (int s = s0; s < s1; ++s) {
-                    const TriV t = load_tri(tris, s);
-                    float tt, terr;
-                    const int r = ray_tri_f(o, d, dinf, t, 1000.0f, &tt, &terr);
-                    const float lb = tt - terr;
-                    if (act && r != 0 && lb <= U) {
-                        if (r == 1) U = fminf(U, tt + terr);
-                        if (nc == kCand) {   // keep only live candidates
-                            int m = 0;
-                            for (int i = 0; i < kCand; ++i)
-                                if (__uint_as_float(cand[32 * i].y) <= U) { cand[32 * m] = cand[32 * i]; ++m; }
-                            nc = m < kCand ? m : kCand + 1;
-                        }
-                        if (nc < kCand) {
+        while (true) {   // the walk, anew after the lists have been settled because one was full
+            const RayAxis X = ray_axis(o.x, d.x, act), Y = ray_axis(o.y, d.y, act), Z = ray_axis(o.z, d.z, act);
+            const bool mixed = __any_sync(kFull, X.kind == 2 || Y.kind == 2 || Z.kind == 2);
+            float c[2];                                 // bounds of the lane's quad and of the other one
+            uint32_t cullmax;
+            auto share_bounds = [&]() {
+                float m = act ? U * 1.000002f : -1.f;
+                cullmax = __reduce_max_sync(kFull, __float_as_uint(fmaxf(m, 0.f)));
+                m = fmaxf(m, __shfl_xor_sync(kFull, m, 1));
+                c[0] = fmaxf(m, __shfl_xor_sync(kFull, m, 2));
+                c[1] = __shfl_xor_sync(kFull, c[0], 4);
+            };
+            share_bounds();
+            bool full = false;
+            while (live && !full) {
+                if (cur >= 0) {
+                    const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + cur);
+                    const int j = lane & 7;
+                    const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
+                    uint32_t key = mixed ? group_entry<true>(X, Y, Z, lo, hi, c) : group_entry<false>(X, Y, Z, lo, hi, c);
+                    key = min(key, __shfl_xor_sync(kFull, key, 8));
+                    key = min(key, __shfl_xor_sync(kFull, key, 16));
+                    if (key != kFull) key = (key & ~7u) | (uint32_t)j;
+                    // its place on the stack: the number of needed children farther than it, two of
+                    // the eight compared by each of the four lanes with this child
+                    const uint32_t ka = __shfl_sync(kFull, key, 2 * (lane >> 3)), kb = __shfl_sync(kFull, key, 2 * (lane >> 3) + 1);
+                    int place = (ka > key && ka != kFull ? 1 : 0) + (kb > key && kb != kFull ? 1 : 0);
+                    place += __shfl_xor_sync(kFull, place, 8);
+                    place += __shfl_xor_sync(kFull, place, 16);
+                    const int kept = __popc(__ballot_sync(kFull, key != kFull) & 0xFFu);
+                    __syncwarp();   // the popped entry has been read
+                    if (lane < 8 && key != kFull) stk[sp + place] = make_uint2((uint32_t)__float_as_int(lo.w), key & ~7u);
+                    sp += kept;
+                    __syncwarp();
+                } else {
+                    int s0, s1;
+                    leaf_range(cur, s0, s1);
+                    const float U0 = U;
+                    for (int s = s0; s < s1; ++s) {
+                        const TriV t = load_tri(tris, s);
+                        float tt, terr;
+                        const int r = ray_tri_f(o, d, dinf, t, 1000.0f, &tt, &terr);
+                        const float lb = tt - terr;
+                        if (act && r != 0 && lb <= U) {
+                            if (r == 1) U = fminf(U, tt + terr);
                             cand[32 * nc] = make_uint2((uint32_t)s, __float_as_uint(lb));
                             ++nc;
-                        }   // else the list has overflowed (nc = kCand + 1)
+                        }
                     }
+                    full = __any_sync(kFull, nc > kCand);
+                    if (__any_sync(kFull, U < U0)) share_bounds();
                 }
-                if (__any_sync(kFull, U < U0)) share_bounds();
+                // the next entry that some ray still needs
+                live = false;
+                while (sp > 0) {
+                    const uint2 e = stk[--sp];
+                    if (e.y <= cullmax) { cur = (int)e.x; live = true; break; }
+                }
             }
-            // the next entry that some ray still needs
-            live = false;
-            while (sp > 0) {
-                const uint2 e = stk[--sp];
-                if (e.y <= cullmax) { cur = (int)e.x; live = true; break; }
-            }
+            if (!live) break;
+            const Settled e = settle_full(cand, nc, tris, o, d, U);
+            nc = e.n;
+            U = e.U;
         }
-        if (!act) continue;
-        double bt = 1000.0;
-        int sx = -1, ix = -1;
-        if (nc > kCand) {
-            walk_hits(tree.nodes, tris, o, d, U, &bt, &sx, &ix);
-            nc = 0;
-        }
-        const d3 od = to_d3(o), dd = to_d3(d);
-        for (int i = 0; i < nc; ++i) {
-            const uint2 e = cand[32 * i];
-            if (__uint_as_float(e.y) > U) continue;
-            const TriV t = load_tri(tris, (int)e.x);
-            double t64;
-            if (!ray_tri_d(od, dd, to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
-            if (t64 < bt || (t64 == bt && (sx < 0 || t.id < ix))) { bt = t64; sx = (int)e.x; ix = t.id; }
-        }
-        depth[q] = __double2float_rn(bt);
-        pos[3 * q] = __double2float_rn(dA((double)o.x, dM(bt, (double)d.x)));
-        pos[3 * q + 1] = __double2float_rn(dA((double)o.y, dM(bt, (double)d.y)));
-        pos[3 * q + 2] = __double2float_rn(dA((double)o.z, dM(bt, (double)d.z)));
-        face_id[q] = sx >= 0 ? (int64_t)ix : (int64_t)-1;
+        if (act) write_hit(closest_hit(cand, nc, U, tris, o, d), q, o, d, pos, face_id, depth);
     }
 }
 
@@ -2206,26 +2208,7 @@ __global__ void __launch_bounds__(kQBlock, kLaneBlocks) k_ray_lanes(int64_t n, c
         const unsigned idle = __ballot_sync(kFull, !live);
         if (idle == kFull || (more && __popc(idle) >= kLaneRefill)) {
             if (!live && q >= 0) {           // settle and write
-                double bt = 1000.0;
-                int sx = -1, ix = -1;
-                if (nc > kCand) {
-                    walk_hits(nodes, tris, o, d, U, &bt, &sx, &ix);
-                    nc = 0;
-                }
-                const d3 od = to_d3(o), dd = to_d3(d);
-                for (int i = 0; i < nc; ++i) {
-                    const uint2 e = cand[32 * i];
-                    if (__uint_as_float(e.y) > U) continue;
-                    const TriV t = load_tri(tris, (int)e.x);
-                    double t64;
-                    if (!ray_tri_d(od, dd, to_d3(t.a), to_d3(t.b), to_d3(t.c), 1000.0, &t64)) continue;
-                    if (t64 < bt || (t64 == bt && (sx < 0 || t.id < ix))) { bt = t64; sx = (int)e.x; ix = t.id; }
-                }
-                depth[q] = __double2float_rn(bt);
-                pos[3 * q] = __double2float_rn(dA((double)o.x, dM(bt, (double)d.x)));
-                pos[3 * q + 1] = __double2float_rn(dA((double)o.y, dM(bt, (double)d.y)));
-                pos[3 * q + 2] = __double2float_rn(dA((double)o.z, dM(bt, (double)d.z)));
-                face_id[q] = sx >= 0 ? (int64_t)ix : (int64_t)-1;
+                write_hit(closest_hit(cand, nc, U, tris, o, d), q, o, d, pos, face_id, depth);
                 q = -1;
             }
             __syncwarp();
@@ -2295,15 +2278,17 @@ __global__ void __launch_bounds__(kQBlock, kLaneBlocks) k_ray_lanes(int64_t n, c
                 if (r != 0 && lb <= U) {
                     if (r == 1) U = fminf(U, tt + terr);
                     if (nc == kCand) {   // keep only live candidates
-                        int m = 0;
+                        nc = 0;
                         for (int i = 0; i < kCand; ++i)
-                            if (__uint_as_float(cand[32 * i].y) <= U) { cand[32 * m] = cand[32 * i]; ++m; }
-                        nc = m < kCand ? m : kCand + 1;
+                            if (__uint_as_float(cand[32 * i].y) <= U) { cand[32 * nc] = cand[32 * i]; ++nc; }
+                        if (nc == kCand) {
+                            const Settled e = settle_full(cand, kCand, tris, o, d, U);
+                            nc = e.n;
+                            U = e.U;
+                        }
                     }
-                    if (nc < kCand) {
-                        cand[32 * nc] = make_uint2((uint32_t)s, __float_as_uint(lb));
-                        ++nc;
-                    }   // else the list has overflowed (nc = kCand + 1)
+                    cand[32 * nc] = make_uint2((uint32_t)s, __float_as_uint(lb));
+                    ++nc;
                 }
             }
             const float cull = U * 1.000002f;
