@@ -1833,20 +1833,23 @@ __device__ __forceinline__ int64_t packet_ray(int64_t pk, int lane, int64_t n, c
 constexpr float kCohDir = 0.008f;
 constexpr float kCohUnits = 0.03f;
 constexpr float kCohOrigin = 0.01f;
-// The reciprocal of a direction component for the node tests: a component
-// that is zero, or too small for its reciprocal to be a number, counts as one
-// that moves by 1e-30 a unit.
-__device__ __forceinline__ float slab_inv(float d, float sign) {
-    return fabsf(d) > 1e-30f ? 1.0f / d : copysignf(1e30f, sign);
-}
+// A direction component up to this counts as parallel to the planes of its
+// axis (kind 2 below), whatever its sign: as a fraction of the ray's largest
+// component, and at the least.  A ray whose origin lies in a box's plane does
+// not leave the box there when the component is zero, nor, as far as the double
+// test can tell (its own rounding is about 1e-16 of the origin's distance), when
+// it is that small; below 1e-30 its reciprocal would not stay a number.
+constexpr float kParallel = 1e-12f, kSmallest = 1e-30f;
 // One axis of the node tests of a lane's eight rays, in two halves of four
 // (a pair of values each): what the halves' origins lie within and their
-// directions' reciprocals.  kind: 0 all directions positive (or all zero), 1
-// all negative, 2 otherwise.
+// directions' reciprocals.  kind: 0 all directions positive, 1 all negative, 2
+// otherwise: signs that differ, or a ray parallel to the axis' planes, which
+// is between them for every parameter or for none.
 struct RayAxis { f2 on, of, i0, i1; int kind; };
 // The axis of the lane's quad of rays and the other quad of its group of
-// eight, from o, d of the lane's ray (ok: the lane has one).
-__device__ __forceinline__ RayAxis ray_axis(float o, float d, bool ok) {
+// eight, from o, d of the lane's ray (ok: the lane has one); dinf: the ray's
+// largest component.
+__device__ __forceinline__ RayAxis ray_axis(float o, float d, float dinf, bool ok) {
     float o0 = ok ? o : CUDART_INF_F, o1 = ok ? o : -CUDART_INF_F;
     float d0 = ok ? d : CUDART_INF_F, d1 = ok ? d : -CUDART_INF_F;
 #pragma unroll
@@ -1856,20 +1859,22 @@ __device__ __forceinline__ RayAxis ray_axis(float o, float d, bool ok) {
         d0 = fminf(d0, __shfl_xor_sync(kFull, d0, s));
         d1 = fmaxf(d1, __shfl_xor_sync(kFull, d1, s));
     }
-    const int own = d0 > 0.f || (d0 == 0.f && d1 == 0.f) ? 0 : (d1 < 0.f ? 1 : 2);
+    const float along = fmaxf(kParallel * dinf, kSmallest);
+    const unsigned group = 0xFFu << (threadIdx.x & 24);
+    const bool up = (~__ballot_sync(kFull, !ok || d > along) & group) == 0u;
+    const bool down = (~__ballot_sync(kFull, !ok || d < -along) & group) == 0u;
     RayAxis r;
-    r.kind = own == __shfl_xor_sync(kFull, own, 4) ? own : 2;
+    r.kind = up ? 0 : (down ? 1 : 2);
     float on, of, i0, i1;
     if (r.kind == 2) {   // reached upwards from o1 by the largest direction, downwards from o0 by the smallest
         on = o1; of = o0;
-        i0 = d1 > 0.f ? slab_inv(d1, 1.f) : 1e30f;
-        i1 = d0 < 0.f ? slab_inv(d0, -1.f) : -1e30f;
+        i0 = d1 > kSmallest ? 1.0f / d1 : 1.0f / kSmallest;
+        i1 = d0 < -kSmallest ? 1.0f / d0 : -1.0f / kSmallest;
     } else {
         on = r.kind == 0 ? o1 : o0;
         of = r.kind == 0 ? o0 : o1;
-        const float sg = r.kind == 0 ? 1.f : -1.f;
-        i0 = slab_inv(d0, sg);
-        i1 = slab_inv(d1, sg);
+        i0 = 1.0f / d0;
+        i1 = 1.0f / d1;
     }
     r.on = f2pack(-on, -__shfl_xor_sync(kFull, on, 4));   // negated
     r.of = f2pack(-of, -__shfl_xor_sync(kFull, of, 4));
@@ -2019,7 +2024,7 @@ __global__ void __launch_bounds__(kQBlock, kRayBlocks) k_ray(int64_t n, const ui
         int nc = 0, sp = 0, cur = 0;
         bool live = true;
         while (true) {   // the walk, anew after the lists have been settled because one was full
-            const RayAxis X = ray_axis(o.x, d.x, act), Y = ray_axis(o.y, d.y, act), Z = ray_axis(o.z, d.z, act);
+            const RayAxis X = ray_axis(o.x, d.x, dinf, act), Y = ray_axis(o.y, d.y, dinf, act), Z = ray_axis(o.z, d.z, dinf, act);
             const bool mixed = __any_sync(kFull, X.kind == 2 || Y.kind == 2 || Z.kind == 2);
             float c[2];                                 // bounds of the lane's quad and of the other one
             uint32_t cullmax;
