@@ -145,36 +145,44 @@ __device__ __forceinline__ float box_d2(float3 p, float3 lo, float3 hi) {
     const float dz = fmaxf(fmaxf(lo.z - p.z, p.z - hi.z), 0.f);
     return dx * dx + dy * dy + dz * dz;
 }
-// Conservative slab interval: computed bounds widened by 1e-6 relative
-// (each bound carries at most three roundings).
-// SAFE: for rays with a zero direction component (inv = +-inf).  A ray with
-// d.x == 0 stays in the x slab of a box for every t if lo.x <= o.x <= hi.x
-// and never otherwise; (lo.x - o.x) * inv.x is +-inf except when the origin
-// lies on the plane (0 * inf = NaN), which then counts as inside the slab.
-template <bool SAFE = false>
+// Conservative slab interval of a ray with a zero direction component (inv =
+// +-inf): computed bounds widened by 1e-6 relative (each bound carries at most
+// three roundings).  A ray with d.x == 0 stays in the x slab of a box for every
+// t if lo.x <= o.x <= hi.x and never otherwise; (lo.x - o.x) * inv.x is +-inf
+// except when the origin lies on the plane (0 * inf = NaN), which then counts as
+// inside the slab.  The other components may be all but zero, and then the
+// double test cannot tell whether a ray from a plane leaves the box there:
+// below 1e-12 of the largest component (kParallel), a slab that is not behind
+// the ray has no exit.
+constexpr float kParallel = 1e-12f;
 __device__ __forceinline__ void box_ray(float3 o, float3 inv, float3 lo, float3 hi, float& tn, float& tf) {
     float t0x = (lo.x - o.x) * inv.x, t1x = (hi.x - o.x) * inv.x;
     float t0y = (lo.y - o.y) * inv.y, t1y = (hi.y - o.y) * inv.y;
     float t0z = (lo.z - o.z) * inv.z, t1z = (hi.z - o.z) * inv.z;
-    if (SAFE) {
-        if (t0x != t0x) t0x = -inv.x;
-        if (t1x != t1x) t1x = inv.x;
-        if (t0y != t0y) t0y = -inv.y;
-        if (t1y != t1y) t1y = inv.y;
-        if (t0z != t0z) t0z = -inv.z;
-        if (t1z != t1z) t1z = inv.z;
-    }
+    if (t0x != t0x) t0x = -inv.x;
+    if (t1x != t1x) t1x = inv.x;
+    if (t0y != t0y) t0y = -inv.y;
+    if (t1y != t1y) t1y = inv.y;
+    if (t0z != t0z) t0z = -inv.z;
+    if (t1z != t1z) t1z = inv.z;
+    const float ix = fabsf(inv.x), iy = fabsf(inv.y), iz = fabsf(inv.z);
+    const float along = fminf(fminf(ix, iy), iz) * (1.f / kParallel);
+    float fx = fmaxf(t0x, t1x), fy = fmaxf(t0y, t1y), fz = fmaxf(t0z, t1z);
+    if (ix >= along && fx >= 0.f) fx = CUDART_INF_F;
+    if (iy >= along && fy >= 0.f) fy = CUDART_INF_F;
+    if (iz >= along && fz >= 0.f) fz = CUDART_INF_F;
     tn = fmaxf(fmaxf(fminf(t0x, t1x), fminf(t0y, t1y)), fminf(t0z, t1z));
-    tf = fminf(fminf(fmaxf(t0x, t1x), fmaxf(t0y, t1y)), fmaxf(t0z, t1z));
+    tf = fminf(fminf(fx, fy), fz);
     tn -= 1e-6f * fabsf(tn);
     tf += 1e-6f * fabsf(tf);
 }
-// 1/d per axis for box_ray; a ray with an infinite reciprocal (a zero or
-// subnormal direction component) must use box_ray<true>.
+// 1/d per axis; a ray with an infinite reciprocal (a zero or
+// subnormal direction component) is tested with box_ray, the others as in
+// affine_node.
 __device__ __forceinline__ float3 ray_inv(float3 d) { return make_float3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z); }
 __device__ __forceinline__ bool ray_degenerate(float3 inv) { return isinf(inv.x) || isinf(inv.y) || isinf(inv.z); }
-// 1/d with the hardware approximation (at most 1 ulp off: box_ray's 1e-6
-// widening covers it) for unit directions; zero and subnormal components
+// 1/d with the hardware approximation (at most 1 ulp off: the 1e-6 margins
+// cover it) for unit directions; zero and subnormal components
 // give +-inf, as ray_inv.
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
@@ -187,7 +195,6 @@ __device__ __forceinline__ float3 ray_inv_approx(float3 d) {
 
 // Any-hit traversal step: push the children of node nd that the ray (o, inv)
 // enters within [0, cull].
-template <bool SAFE>
 __device__ __forceinline__ void push_ray_children(const NodeView& nd, float3 o, float3 inv, float cull, int* st,
                                                   int& sp) {
 #pragma unroll
@@ -196,7 +203,7 @@ __device__ __forceinline__ void push_ray_children(const NodeView& nd, float3 o, 
         float3 lo, hi;
         child_box(nd, j, lo, hi);
         float tn, tf;
-        box_ray<SAFE>(o, inv, lo, hi, tn, tf);
+        box_ray(o, inv, lo, hi, tn, tf);
         if (m != kEmpty && tn <= tf && tf >= 0.f && tn <= cull) st[sp++] = child_ref(nd, m);
     }
 }
@@ -267,7 +274,7 @@ __device__ __forceinline__ void push_ray_children_affine(const NodeView& nd, flo
 // Closest-hit step of one lane's own walk: entry distance (ordered bits of
 // max(tn, 0), child index in the low 3 bits) of the ray into each child of
 // nd that it enters within [0, cull], kFull for the others.  degen (a zero
-// or subnormal direction component): box_ray<true> on the decoded boxes;
+// or subnormal direction component): box_ray on the decoded boxes;
 // else the affine fold of push_ray_children_affine (same error margins).
 __device__ __forceinline__ void lane_child_keys(const NodeView& nd, float3 o, float3 inv, bool degen, float cull,
                                                 uint32_t k[8]) {
@@ -277,7 +284,7 @@ __device__ __forceinline__ void lane_child_keys(const NodeView& nd, float3 o, fl
             float3 lo, hi;
             child_box(nd, j, lo, hi);
             float tn, tf;
-            box_ray<true>(o, inv, lo, hi, tn, tf);
+            box_ray(o, inv, lo, hi, tn, tf);
             const float key = fmaxf(tn, 0.f);
             const bool need = meta_of(nd, j) != kEmpty && tn <= tf && tf >= 0.f && key <= cull;
             k[j] = need ? ((__float_as_uint(key) & ~7u) | (uint32_t)j) : kFull;
@@ -1657,7 +1664,7 @@ __global__ void __launch_bounds__(kQBlock, kStabBlocks) k_sign_raystab(Work w, c
             if (!in || (__popc(in) < kStabInner && __any_sync(kFull, live && !ended && cur < 0))) break;
             if (inner) {
                 const NodeView nd = load_node(nodes, cur);
-                if (degen) push_ray_children<true>(nd, p, inv, cull, st, sp);
+                if (degen) push_ray_children(nd, p, inv, cull, st, sp);
                 else push_ray_children_affine(nd, p, inv, cull, st, sp);
                 if (sp > 0) cur = st[--sp];
                 else ended = true;
@@ -1782,7 +1789,7 @@ __global__ void __launch_bounds__(kQBlock, 10) k_sign_raystab_lines(const float*
                         const int ref = st[--sp];
                         if (ref >= 0) {
                             const NodeView nd = load_node(nodes, ref);
-                            if (degen) push_ray_children<true>(nd, p, inv, cull, st, sp);
+                            if (degen) push_ray_children(nd, p, inv, cull, st, sp);
                             else push_ray_children_affine(nd, p, inv, cull, st, sp);
                         } else {
                             leaf_range(ref, ls, le);
@@ -1833,13 +1840,13 @@ __device__ __forceinline__ int64_t packet_ray(int64_t pk, int lane, int64_t n, c
 constexpr float kCohDir = 0.008f;
 constexpr float kCohUnits = 0.03f;
 constexpr float kCohOrigin = 0.01f;
-// A direction component up to this counts as parallel to the planes of its
-// axis (kind 2 below), whatever its sign: as a fraction of the ray's largest
-// component, and at the least.  A ray whose origin lies in a box's plane does
+// A direction component up to kParallel of the ray's largest, or up to this,
+// counts as parallel to the planes of its axis (kind 2 below), whatever its
+// sign.  A ray whose origin lies in a box's plane does
 // not leave the box there when the component is zero, nor, as far as the double
 // test can tell (its own rounding is about 1e-16 of the origin's distance), when
 // it is that small; below 1e-30 its reciprocal would not stay a number.
-constexpr float kParallel = 1e-12f, kSmallest = 1e-30f;
+constexpr float kSmallest = 1e-30f;
 // One axis of the node tests of a lane's eight rays, in two halves of four
 // (a pair of values each): what the halves' origins lie within and their
 // directions' reciprocals.  kind: 0 all directions positive, 1 all negative, 2

@@ -27,7 +27,8 @@ def _check(oracle, v, f, o, d, got):
 
 @pytest.mark.parametrize("copies", [1, 2, 4, 5, 9, 20])
 @pytest.mark.parametrize("tiny", [1e-14, 1e-20, 1e-31])
-def test_rays_alone_in_a_plane(oracle, dev, copies, tiny):
+@pytest.mark.parametrize("third", [0.03125, 0.0])
+def test_rays_alone_in_a_plane(oracle, dev, copies, tiny, third):
     """Along the sides of a cube, with a component away from them or towards them that the double test hardly sees."""
     v, f = _cube(copies)
     rng = np.random.default_rng(copies)
@@ -39,7 +40,7 @@ def test_rays_alone_in_a_plane(oracle, dev, copies, tiny):
                 for x in (-0.9, -0.3, 0.2, 0.7):
                     p, q = np.zeros(3), np.zeros(3)
                     p[axis], p[u], p[w] = 3.0, side, x
-                    q[axis], q[u], q[w] = -1.0, out * tiny, 0.03125
+                    q[axis], q[u], q[w] = -1.0, out * tiny, third
                     o.append(p)
                     d.append(q)
     o, d = np.array(o, np.float32), np.array(d, np.float32)
