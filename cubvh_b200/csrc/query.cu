@@ -530,39 +530,52 @@ __device__ __forceinline__ float tri_lower_bound(const WTri* __restrict__ wtris,
     return d2 - err;
 }
 
-// A point's exact nearest triangle by a walk of its own, given an upper
-// bound U of its squared distance: every triangle whose lower bound is
-// within U is evaluated in double.  The bound k_udf ends with is all but
-// exact, so the walk meets little more than the triangles that tie.
-__device__ __noinline__ void walk_ties(const DeviceTree& tree, int root, float3 p, float U, double* bx, int* sx,
-                                       int* ix) {
-    int st[kStack];
-    int sp = 0;
-    st[sp++] = root;
-    double best = *bx;
-    int s_best = *sx, id_best = *ix;
-    const float cull = U * 1.000002f;
-    while (sp > 0) {
-        const int ref = st[--sp];
-        if (ref >= 0) {
-            const float4* nb = reinterpret_cast<const float4*>(tree.wnodes + ref);
+// Exact nearest triangles of the points of a packet's lanes `on`, given upper
+// bounds U of their squared distances, as the only entries of their lists (32
+// entries apart): the warp walks the union of their paths once more, and each
+// lane evaluates in double every triangle whose lower bound is within its U.
+// The bounds that k_udf's walk ends with are all but exact, so this meets
+// little more than the triangles that tie.  Returns the list's length.
+__device__ __noinline__ int walk_ties(const WNode* __restrict__ wnodes, const WTri* __restrict__ wtris,
+                                      const CTri* __restrict__ tris, uint2* stk, uint2* cand, int root, float3 p, float U,
+                                      bool on) {
+    double best = 1e6;
+    int slot = -1, id = 0;
+    int sp = 0, cur = root;
+    while (true) {
+        if (cur >= 0) {
+            const float4* nb = reinterpret_cast<const float4*>(wnodes + cur);
+            const float cull = on ? U * 1.000002f : -1.f;
+            __syncwarp();   // the popped entry has been read
             for (int j = 0; j < 8; ++j) {
                 const float4 lo = __ldg(nb + j), hi = __ldg(nb + 8 + j);
-                if (box_d2(p, make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z)) <= cull)
-                    st[sp++] = __float_as_int(lo.w);
+                if (__any_sync(kFull, box_d2(p, make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z)) <= cull)) {
+                    if ((threadIdx.x & 31) == 0) stk[sp].x = (uint32_t)__float_as_int(lo.w);
+                    ++sp;
+                }
             }
+            __syncwarp();
         } else {
             int s0, s1;
-            leaf_range(ref, s0, s1);
+            leaf_range(cur, s0, s1);
             for (int s = s0; s < s1; ++s) {
-                if (tri_lower_bound(tree.wtris, s, p) > U) continue;
-                const TriV t = load_tri(tree.tris, s);
+                const float4* tw = reinterpret_cast<const float4*>(wtris + s);
+                float err;
+                const float d2 = tri_d2_w(p, make_triw(__ldg(tw), __ldg(tw + 1), __ldg(tw + 2), __ldg(tw + 3)), &err);
+                if (!on || d2 - err > U) continue;   // no number: undecided
+                const TriV t = load_tri(tris, s);
                 const double e = dist2_on_tri_d(to_d3(p), to_d3(t.a), to_d3(t.b), to_d3(t.c));
-                if (e < best || (e == best && (s_best < 0 || t.id < id_best))) { best = e; s_best = s; id_best = t.id; }
+                if (e < best || (e == best && (slot < 0 || t.id < id))) { best = e; slot = s; id = t.id; }
             }
+            if (slot >= 0) U = fminf(U, __double2float_ru(best));
+            __syncwarp();
         }
+        if (sp == 0) break;
+        cur = (int)stk[--sp].x;
     }
-    *bx = best; *sx = s_best; *ix = id_best;
+    if (slot < 0) return 0;
+    cand[0] = make_uint2((uint32_t)slot, __float_as_uint(0.f));
+    return 1;
 }
 
 // Exact nearest triangle of 32 Morton-adjacent points per warp (a packet):
@@ -598,12 +611,20 @@ __device__ __noinline__ void walk_ties(const DeviceTree& tree, int root, float3 
 //
 // Heavy queries, served afterwards with a warp each (k_udf_heavy, from the
 // bound found so far): a point whose candidate list overflows (many
-// triangles at almost the same distance), and the points of a packet that
+// triangles at almost the same distance) in a packet with fewer than
+// kTiesHere of them, and the points of a packet that
 // is still walking after kHandOff visits when the queue is empty: deep
 // inside a closed mesh or near its medial axis points are about equally far
 // from very many triangles, and such a packet would hold the launch's end
-// alone.  When the heavy list is full both finish here instead.
+// alone.  When the heavy list is full both finish here instead, as do the
+// points of a packet most of which tie (faces that are there several times):
+// walked together once more they cost a fraction of a warp each (300k points
+// on 12 copies of 5,120 faces 36 against 5.1 ms, 1M at the middle of 3 copies
+// of 82k faces 7.7 against 5.5).  The grid of 384^3 points has packets of both
+// kinds and pays 2 % (48.9 against 50.0 ms); lines of 4 to 28 points measure
+// the same, so the line is a quarter of the packet.
 constexpr int kHandOff = 192;
+constexpr int kTiesHere = 8;
 template <bool UVW, bool SLOT>
 __global__ void __launch_bounds__(kQBlock, kUdfBlocks) k_udf(Work w, const uint32_t* __restrict__ order,
                                                  const float* __restrict__ pts, float* __restrict__ dist,
@@ -766,18 +787,24 @@ __global__ void __launch_bounds__(kQBlock, kUdfBlocks) k_udf(Work w, const uint3
         }
         if (handed_off) continue;
         bool mine = act;
-        double bx = 1e6;
-        int sx = -1, ix = 0;
+        const bool many = __popc(__ballot_sync(kFull, nc > kCand)) >= kTiesHere;
+        bool again = false;
         if (nc > kCand) {
-            const unsigned long long b = atomicAdd(n_heavy, 1ull);
+            const unsigned long long b = many ? (unsigned long long)heavy_cap : atomicAdd(n_heavy, 1ull);
             if ((int64_t)b < heavy_cap) {
                 heavy[b] = make_uint4((uint32_t)idx, w.table ? (uint32_t)w.table[pk].mesh : 0u, __float_as_uint(U), 0u);
                 mine = false;
             } else {
-                walk_ties(tree, root, p, U, &bx, &sx, &ix);
+                again = true;
             }
             nc = 0;
         }
+        if (__any_sync(kFull, again)) {
+            const int left = walk_ties(tree.wnodes, tree.wtris, tris, stk, cand, root, p, U, again);
+            if (again) nc = left;
+        }
+        double bx = 1e6;
+        int sx = -1, ix = 0;
         // the k-th live candidates of all lanes together
         for (int i = 0;; ++i) {
             while (i < nc && __uint_as_float(cand[32 * i].y) > U) ++i;
