@@ -10,7 +10,7 @@
 // a C-order [D][H][W] array; this implementation uses the same neighbourhood
 // (identical to [H][W][D] when H = W = D).
 //
-// Algorithm (three kernels, no host round trip).  A row is W consecutive
+// Algorithm (four kernels, no host round trip).  A row is W consecutive
 // voxels of memory; a run is a maximal stretch of free voxels in a row.
 //   1. tile     one block per tile of T consecutive rows of one z-slice,
 //               four bitmask words per thread: packs the tile's free-voxel
@@ -28,7 +28,9 @@
 //               above; lock-free union-find on the global roots that always
 //               links the larger root under the smaller, so every root is
 //               its component's smallest run id, i.e. smallest voxel index
-//   3. label    one block per tile: the tile's run labels (each run's
+//   3. resolve  for tiles whose runs do not fit in shared memory: every run's
+//               label, its root's first voxel, in place
+//   4. label    one block per tile: the tile's run labels (each run's
 //               root's first voxel), start marks and run bases staged in
 //               shared memory, then the int32 labels (or the signed
 //               distances of udf_to_sdf) written: 16-byte streaming stores,
@@ -406,10 +408,13 @@ k_ff_tile(Src src, int W, int wpr, uint32_t magic, int T, int64_t tiles_per_slic
     // covering that voxel (uniting rows in binary-tree rounds instead, which
     // bounds the forest's depth, measured 40 % slower: the rounds' barriers
     // cost more than the longer paths)
+    // Lanes take neighbouring words, one at a time: a lane on four words of its
+    // own, unrolled, left the warp's lanes in different copies of the loop (128^3
+    // noise, 70 % free: 305 us, a word at a time 211, neighbouring words 112).
     if (one && nrow > 1) {
-#pragma unroll
+#pragma unroll 1
         for (int j = 0; j < 4; ++j) {
-            const int w = t4 + j;
+            const int w = (int)threadIdx.x + j * kTileThreads;
             if (w < wpr || w >= nwords) continue;
             const int q = w - wpr;
             int row, wi;
@@ -519,7 +524,41 @@ __global__ void k_ff_merge(const uint32_t* __restrict__ bits, const uint32_t* __
     }
 }
 
-// 3. One block per tile: the tile's run labels (up to kSmemRuns) and its
+// 3. Labels of the runs of tiles with more than kSmemRuns runs, in place (a
+// root's own entry is its label already and stays as it is, so other blocks
+// reading roots see final values).  In a kernel of its own, whose walks have
+// the L2 to themselves: in the label writer they ran beside its streamed
+// stores (512^3 noise, 30 % free: the writer took 591 us, without it 143
+// and this kernel 154).  Grids without such tiles pay the
+// launch, 3 us.
+__global__ void __launch_bounds__(kTileThreads)
+k_ff_resolve(const uint32_t* __restrict__ tcount, int64_t ntiles, int64_t cap, const int32_t* __restrict__ parent,
+             int32_t* __restrict__ start, int* __restrict__ status) {
+    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const uint32_t n = tcount[tile];
+        if (n <= (uint32_t)kSmemRuns) continue;
+        const int32_t base = (int32_t)(tile * cap);
+        for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 4 * kTileThreads) {
+            int32_t root[4], l[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t i = i0 + j * kTileThreads;
+                root[j] = i < n ? base + (int32_t)i : -1;
+            }
+            uf_root4(parent, root, status);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int32_t r = base + (int32_t)(i0 + j * kTileThreads);
+                l[j] = root[j] >= 0 && root[j] != r ? start[root[j]] : -1;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (l[j] >= 0) start[base + (int32_t)(i0 + j * kTileThreads)] = l[j];
+        }
+    }
+}
+
+// 4. One block per tile: the tile's run labels (up to kSmemRuns) and its
 // words' free bits are staged in shared memory with coalesced loads, the
 // words' run starts and run bases (tile-relative) recomputed from the bits
 // with one block-wide scan, then (VEC: W % 32 == 0, 16-byte aligned output)
@@ -534,7 +573,7 @@ __global__ void k_ff_merge(const uint32_t* __restrict__ bits, const uint32_t* __
 template <bool SDF, bool VEC>
 __global__ void __launch_bounds__(kTileThreads)
 k_write_tile(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ rowid,
-             const uint32_t* __restrict__ tcount, int32_t* __restrict__ runlab,
+             const uint32_t* __restrict__ tcount, const int32_t* __restrict__ runlab,
              const int32_t* __restrict__ parent, int* __restrict__ status, int W, int wpr, uint32_t magic, int T,
              int64_t tiles_per_slice, int H, int64_t cap, int32_t* __restrict__ labels, float* __restrict__ sdf,
              int64_t rows_per_volume) {
@@ -556,11 +595,10 @@ k_write_tile(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ row
         const int64_t rv = (r0 / rows_per_volume) * rows_per_volume;
         if (bits[rv * wpr] & 1u) empty = runlab[uf_root(parent, (int32_t)rowid[rv], status)];
     }
-    // each run's label is its root's first voxel: staged, or for a tile with
-    // more runs than fit resolved in place.  A root's own entry is its label
-    // already and stays as it is, so other blocks reading roots see final values.
+    // staged tiles: each run's label is its root's first voxel; the others'
+    // labels have been resolved in place
     bool other = !inl;   // SDF: the tile may hold a run whose label differs from empty
-    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 4 * kTileThreads) {
+    for (uint32_t i0 = threadIdx.x; inl && i0 < n; i0 += 4 * kTileThreads) {
         int32_t root[4], l[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -574,15 +612,10 @@ k_write_tile(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ row
         for (int j = 0; j < 4; ++j) {
             const uint32_t i = i0 + j * kTileThreads;
             if (i >= n) continue;
-            if (inl) {
-                slab[i] = l[j];
-                other |= l[j] != empty;
-            } else if (root[j] != (int32_t)(tbase + i)) {
-                runlab[tbase + i] = l[j];
-            }
+            slab[i] = l[j];
+            other |= l[j] != empty;
         }
     }
-    if (!inl) __syncthreads();
     // SDF: sdf already holds udf - eps, and only free voxels of runs labelled
     // differently from the volume's first voxel can flip; a tile with none
     // is done
@@ -701,7 +734,7 @@ FFBufs carve(const FFPlan& p, void* ws) {
                   reinterpret_cast<int*>(base + p.off_status)};
 }
 
-// 1-2: tiles, cross-tile unions
+// 1-3: tiles, cross-tile unions, the labels that the writer does not stage
 template <class Src>
 void label_runs(const FFPlan& p, int D, const Src& src, const FFBufs& b, cudaStream_t stream) {
     k_zero<<<1, 1, 0, stream>>>(b.status); count_launch();
@@ -711,8 +744,13 @@ void label_runs(const FFPlan& p, int D, const Src& src, const FFBufs& b, cudaStr
     const unsigned mgrid = (unsigned)((2 * p.rows + 255) / 256);
     k_ff_merge<<<mgrid, 256, 0, stream>>>(b.bits, b.rowid, b.parent, b.status, p.rows, p.wpr, p.H, D,
                                           p.tile_rows); count_launch();
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    k_ff_resolve<<<(unsigned)std::min<int64_t>(p.ntiles, 8 * (int64_t)nsm), kTileThreads, 0, stream>>>(
+        b.tcount, p.ntiles, p.cap, b.parent, b.start, b.status); count_launch();
 }
-// 3
+// 4
 template <bool SDF>
 void write_tiles(const FFPlan& p, const FFBufs& b, bool vec, int32_t* labels, float* sdf, int64_t rows_per_volume,
                  cudaStream_t stream) {
