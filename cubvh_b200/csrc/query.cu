@@ -1855,18 +1855,35 @@ __device__ __forceinline__ int64_t packet_ray(int64_t pk, int lane, int64_t n, c
     const int64_t slot = pk * (32 / kUnit) + lane / kUnit;
     return slot < units ? (int64_t)__ldg(order + slot) * kUnit + lane % kUnit : n;
 }
-// A packet is traced as a packet only when the rays of each unit are all but
-// parallel (unit directions within kCohDir, max-norm: half a degree), its
-// units' nearly so (kCohUnits) and they start close together (origins within
-// kCohOrigin of the root box's extent), as k_ray_order judges it; the others
-// go to k_ray_lanes, where each ray walks alone.  k_ray bounds a unit's rays
-// by intervals, which keep ever more nodes that no ray needs as the unit
-// spreads: 4 cameras x 1024^2 with directions jittered by 0.5 / 1 / 2 degrees
-// take 2.0 / 1.6 / 1.8 ms with the limit at 0.01 and 3.5 / 10 / 25 ms at
-// 0.1; exact cameras of 2048^2 pixels 3.11 against 3.10 ms, and 3.2 at 0.005.
+// Whether a window's packets (k_ray_order) are traced as packets (k_ray) or ray
+// by ray (k_ray_lanes).  k_ray bounds a unit's rays by intervals, which keep
+// ever more nodes that no ray needs as the unit spreads against the faces it
+// meets, so a packet is within limits when
+//  - each unit's rays are all but parallel (unit directions within kCohDir,
+//    max-norm: half a degree; and, at the distance of the mesh, within kCohFaces
+//    faces, the extent of the root box over the square root of their number),
+//  - its units are nearly so (kCohUnits),
+//  - and they start close together (origins within kCohOrigin of the extent).
+// The packets of a window go one way, packets if half of them are within
+// limits, so that one kernel's longest walks do not follow the other's; only
+// packets beyond twice the limits are always traced ray by ray.  A call of few
+// rays, which fills the chip with neither, is bound by its longest walk, the
+// longer one in a packet: a quarter of the limits (kCohFew).
+//
+// 1M camera rays with directions jittered by 0, 0.001, 0.002, 0.004 radians
+// against no density limit and a decision per packet: 1.3M faces 0.68, 0.82,
+// 0.84, 0.84 against 0.67, 1.23, 1.97, 3.35 ms, 82k faces 0.20, 0.26, 0.34, 0.36
+// against 0.20, 0.30, 0.40, 0.59; 0.26M camera rays on 1.3M faces 0.41 against
+// 0.70.  kCohFaces 2 / 2.5 / 5: 0.82 / 0.68 / 0.68, 0.82 / 0.82 / 1.08 ms at 0 and
+// 0.001.  33.5M exact camera rays 3.14 against 3.14, at kCohDir 0.005 3.2.
+// 65k of them, 0.0009 radians apart, on 1.3M faces 0.18 against 0.34 ms without
+// kCohFew, 0.0002 apart 0.12 as packets and 0.14 ray by ray.
 constexpr float kCohDir = 0.008f;
+constexpr float kCohFaces = 3.f;
 constexpr float kCohUnits = 0.03f;
 constexpr float kCohOrigin = 0.01f;
+constexpr int64_t kFewRays = 1 << 17;
+constexpr float kCohFew = 0.25f;
 // A direction component up to kParallel of the ray's largest, or up to this,
 // counts as parallel to the planes of its axis (kind 2 below), whatever its
 // sign.  A ray whose origin lies in a box's plane does
@@ -2206,6 +2223,10 @@ __global__ void k_cell_scatter(int64_t n, const float* __restrict__ pts, const u
 constexpr int kLaneBlocks = 6;    // blocks of k_ray_lanes per SM
 constexpr int kLaneRefill = 16;   // idle lanes that make a warp finish them and take new rays
 constexpr int kLaneInner = 12;    // fewer lanes at inner nodes than this wait for those at leaves
+// the same for few rays, bound by the latency of a walk: registers without
+// spills, and lanes at leaves wait less (1,000 rays on 1.3M faces 233 against
+// 264 us; 5M rays 2.31 against 2.08 ms)
+constexpr int kFewLaneBlocks = 4, kFewLaneInner = 4;
 // Closest hit of the rays of the incoherent packets (k_ray_order and k_ray
 // list them): each lane walks its own ray alone (own stack in local memory,
 // children nearest first, a child popped only while its entry distance is
@@ -2220,7 +2241,8 @@ constexpr int kLaneInner = 12;    // fewer lanes at inner nodes than this wait f
 // load latency and divergence).  Filters,
 // candidate list and the FP64 settlement are k_ray's, so every result is the
 // one k_ray would give.
-__global__ void __launch_bounds__(kQBlock, kLaneBlocks) k_ray_lanes(int64_t n, const uint32_t* __restrict__ order,
+template <bool FEW>
+__global__ void __launch_bounds__(kQBlock, FEW ? kFewLaneBlocks : kLaneBlocks) k_ray_lanes(int64_t n, const uint32_t* __restrict__ order,
                                                        const float* __restrict__ ro, const float* __restrict__ rd,
                                                        float* __restrict__ pos, int64_t* __restrict__ face_id,
                                                        float* __restrict__ depth, const CNode* __restrict__ nodes,
@@ -2283,7 +2305,7 @@ __global__ void __launch_bounds__(kQBlock, kLaneBlocks) k_ray_lanes(int64_t n, c
         // inner nodes
         while (true) {
             const unsigned in = __ballot_sync(kFull, live && cur >= 0);
-            if (!in || (__popc(in) < kLaneInner && __any_sync(kFull, live && cur < 0))) break;
+            if (!in || (__popc(in) < (FEW ? kFewLaneInner : kLaneInner) && __any_sync(kFull, live && cur < 0))) break;
             if (live && cur >= 0) {
                 const float cull = U * 1.000002f;
                 const NodeView nd = load_node(nodes, cur);
@@ -2393,16 +2415,15 @@ __device__ __forceinline__ int ray_entry(float3 o, float3 d, const float lo[3], 
 // One block per window: entry points of the units' rays, the box of those
 // that enter, Morton keys, a block radix sort of (key, unit in the window),
 // and the sorted unit indices written to order[].  Then each packet of the
-// window (4 consecutive sorted units) is judged: coherent when each unit's
-// first and last rays lie within kCohDir (unit directions, max-norm) and
-// kCohOrigin (origins) of the unit's fourth ray, and each unit's fourth ray
-// within kCohUnits and kCohOrigin of the first unit's.  The coherent ones are
+// window (4 consecutive sorted units) is judged by the first and last rays of
+// its units against their fourth, and by the fourths (above); face: the
+// density of the mesh, 1 / sqrt(faces).  The packets to trace as such are
 // listed for k_ray, the others for k_ray_lanes (with a flag per packet instead,
 // k_ray took 359 us to pass over the packets of 16.8M incoherent rays: an
 // atomic each on its queue; 5M such rays 2.31 -> 2.20 ms a call).
 __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const float* __restrict__ ro,
                                                            const float* __restrict__ rd,
-                                                           const CNode* __restrict__ nodes,
+                                                           const CNode* __restrict__ nodes, float face,
                                                            uint32_t* __restrict__ order, uint32_t* __restrict__ packets,
                                                            unsigned long long* __restrict__ packets_n,
                                                            uint32_t* __restrict__ lanes,
@@ -2411,7 +2432,7 @@ __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const floa
     __shared__ typename Sort::TempStorage s_sort;
     __shared__ uint32_t s_box[6];
     __shared__ float s_ray[kOrdUnits][6];     // each unit's fourth ray: unit direction, origin
-    __shared__ uint8_t s_bad[kOrdUnits];       // the unit's first or last ray strays from its fourth
+    __shared__ uint8_t s_bad[kOrdUnits];       // the unit's first or last ray strays from its fourth: beyond the limits 1, twice 2
     __shared__ uint16_t s_sorted[kOrdUnits];
     const int64_t units = (n + kUnit - 1) / kUnit;
     const int64_t u0 = (int64_t)blockIdx.x * kOrdUnits;
@@ -2421,7 +2442,9 @@ __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const floa
     const NodeView root = load_node(nodes, 0);
     const float blo[3] = {root.ox, root.oy, root.oz};
     const int bex[3] = {nodes[0].ex, nodes[0].ey, nodes[0].ez};
-    const float spread_max = kCohOrigin * 255.f * fmaxf(fmaxf(root.sx, root.sy), root.sz);
+    const float strict = n < kFewRays ? kCohFew : 1.f;
+    const float extent = 255.f * fmaxf(fmaxf(root.sx, root.sy), root.sz);
+    const float spread_max = strict * kCohOrigin * extent;
     float ep[kOrdItems][3];
     int kind[kOrdItems];              // 0 enters the box, 1 misses it, 2 past the last unit
     uint32_t lo[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, hi[3] = {0u, 0u, 0u};
@@ -2441,18 +2464,22 @@ __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const floa
         }
         const float il = rsqrtf(f3dot(d, d));
         const float3 v = make_float3(d.x * il, d.y * il, d.z * il);
-        bool bad = false;
+        const float3 far = f3sub(make_float3(ep[i][0], ep[i][1], ep[i][2]), o);
+        const float dir_max = strict * fminf(kCohDir, kCohFaces * face * extent * rsqrtf(f3dot(far, far)));
+        // a finite fourth direction, not zero (NaN: bad); within the limits, within twice the limits
+        bool in = f3inf(v) <= 2.f, near = in;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int64_t qe = e == 0 ? u * kUnit : min(u * kUnit + kUnit - 1, n - 1);
             const float3 oe = load3(ro, qe), de = load3(rd, qe);
             const float ie = rsqrtf(f3dot(de, de));
-            const float3 ve = make_float3(de.x * ie, de.y * ie, de.z * ie);
-            bad |= !(f3inf(f3sub(ve, v)) <= kCohDir && f3inf(f3sub(oe, o)) <= spread_max);   // NaN: bad
+            const float dv = f3inf(f3sub(make_float3(de.x * ie, de.y * ie, de.z * ie), v)), dov = f3inf(f3sub(oe, o));
+            in &= dv <= dir_max && dov <= spread_max;
+            near &= dv <= 2.f * dir_max && dov <= 2.f * spread_max;
         }
         s_ray[li][0] = v.x; s_ray[li][1] = v.y; s_ray[li][2] = v.z;
         s_ray[li][3] = o.x; s_ray[li][4] = o.y; s_ray[li][5] = o.z;
-        s_bad[li] = bad || !(f3inf(v) <= 2.f);   // a non-finite (or zero) fourth direction: bad
+        s_bad[li] = in ? 0 : (near ? 1 : 2);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -2494,10 +2521,10 @@ __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const floa
     // packet t of the window: sorted units 4t .. 4t + 3
     const int64_t pk = (int64_t)blockIdx.x * (kOrdUnits / 4) + t;
     const bool valid = u0 + 4 * t < units;
-    bool inc = false;
+    int bad = 0;
     if (valid) {
         const int f = s_sorted[4 * t];
-        inc = s_bad[f];
+        bad = s_bad[f];
         for (int j = 1; j < 4 && u0 + 4 * t + j < units; ++j) {
             const int v = s_sorted[4 * t + j];
             float dv = 0.f, dov = 0.f;
@@ -2506,9 +2533,13 @@ __global__ void __launch_bounds__(kOrdThreads) k_ray_order(int64_t n, const floa
                 dv = fmaxf(dv, fabsf(s_ray[v][k] - s_ray[f][k]));
                 dov = fmaxf(dov, fabsf(s_ray[v][3 + k] - s_ray[f][3 + k]));
             }
-            inc |= s_bad[v] || !(dv <= kCohUnits && dov <= spread_max);
+            const bool in = dv <= kCohUnits && dov <= spread_max, near = dv <= 2.f * kCohUnits && dov <= 2.f * spread_max;
+            bad = max(bad, max((int)s_bad[v], in ? 0 : (near ? 1 : 2)));
         }
     }
+    // the window's packets go one way, but for those beyond twice the limits
+    const int total = __syncthreads_count(valid), in_limits = __syncthreads_count(valid && bad == 0);
+    const bool inc = 2 * in_limits < total || bad == 2;
     auto list = [&](bool in, uint32_t* __restrict__ to, unsigned long long* __restrict__ to_n) {
         const unsigned m = __ballot_sync(kFull, in);
         if (m) {                      // one atomic per warp
@@ -2815,13 +2846,20 @@ cudaError_t launch_ray(int64_t n, const float* ro, const float* rd, float* pos, 
     uint32_t* lanes = reinterpret_cast<uint32_t*>(w + r.lanes);
     const int64_t units = (n + kUnit - 1) / kUnit;
     k_ray_order<<<(unsigned)((units + kOrdUnits - 1) / kOrdUnits), kOrdThreads, 0, stream>>>(
-        n, ro, rd, nodes, order, packets, ctr + kCtRayPacketsN, lanes, ctr + kCtRayLanesN); count_launch();
+        n, ro, rd, nodes, 1.f / sqrtf((float)tree.n_tris), order, packets, ctr + kCtRayPacketsN, lanes, ctr + kCtRayLanesN);
+    count_launch();
     const unsigned g = persistent_grid(k_ray, n);
     k_ray<<<g, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, tree, ctr + kCtUdf, grab_for(n, g), packets,
                                      ctr + kCtRayPacketsN, lanes, ctr + kCtRayLanesN); count_launch();
-    const unsigned gl = persistent_grid(k_ray_lanes, n);
-    k_ray_lanes<<<gl, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, nodes, tris, lanes,
-                                            ctr + kCtRayLanesN, ctr + kCtRayLanesNext); count_launch();
+    if (n < kFewRays) {
+        const unsigned gl = persistent_grid(k_ray_lanes<true>, n);
+        k_ray_lanes<true><<<gl, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, nodes, tris, lanes,
+                                                      ctr + kCtRayLanesN, ctr + kCtRayLanesNext); count_launch();
+    } else {
+        const unsigned gl = persistent_grid(k_ray_lanes<false>, n);
+        k_ray_lanes<false><<<gl, kQBlock, 0, stream>>>(n, order, ro, rd, pos, fid, depth, nodes, tris, lanes,
+                                                       ctr + kCtRayLanesN, ctr + kCtRayLanesNext); count_launch();
+    }
     return cudaGetLastError();
 }
 
