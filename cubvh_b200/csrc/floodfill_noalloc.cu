@@ -58,10 +58,7 @@ int floodfill_noalloc_scratch(void** ws, std::string& err) {
 }
 
 int floodfill_noalloc_fits(int B, int H, int W, int D, std::string& err) {
-    // the limit that callers know: the workspace as it was with two more words
-    // per 32 voxels
-    const size_t words = (size_t)B * D * H * (((size_t)W + 31) / 32);
-    const size_t need = floodfill_workspace_bytes(B, H, W, D) + 2 * ((4 * words + 255) & ~(size_t)255);
+    const size_t need = floodfill_workspace_bytes(B, H, W, D);
     if (need > kNoAllocScratchBytes) {
         err = "grid needs " + std::to_string(need) + " bytes of scratch but the no-allocation floodfill holds " +
               std::to_string(kNoAllocScratchBytes) + " (about 192^3 voxels); use cubvh_floodfill";
