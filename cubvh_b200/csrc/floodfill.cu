@@ -408,13 +408,16 @@ k_ff_tile(Src src, int W, int wpr, uint32_t magic, int T, int64_t tiles_per_slic
     // covering that voxel (uniting rows in binary-tree rounds instead, which
     // bounds the forest's depth, measured 40 % slower: the rounds' barriers
     // cost more than the longer paths)
-    // Lanes take neighbouring words, one at a time: a lane on four words of its
-    // own, unrolled, left the warp's lanes in different copies of the loop (128^3
-    // noise, 70 % free: 305 us, a word at a time 211, neighbouring words 112).
+    // A word at a time: unrolled over a lane's four, lanes that diverged stayed in
+    // different copies of the loop (128^3 noise, 70 % free: 305 us, not unrolled
+    // 211).  In rows of fewer than eight words lanes take neighbouring words
+    // rather than their own four (128^3 noise 211 -> 112 us, ragged 2 x 181 x 203 x
+    // 197 grids 65 -> 58); in longer rows there is no gain, and 512^3 tori lose 3 us.
+    const bool own = wpr >= 8;
     if (one && nrow > 1) {
 #pragma unroll 1
         for (int j = 0; j < 4; ++j) {
-            const int w = (int)threadIdx.x + j * kTileThreads;
+            const int w = own ? t4 + j : (int)threadIdx.x + j * kTileThreads;
             if (w < wpr || w >= nwords) continue;
             const int q = w - wpr;
             int row, wi;
