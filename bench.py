@@ -693,7 +693,7 @@ def run_ours(args):
             def fn(res=res, grid=grid, lab=lab, ws=ws, nb=nb.value):
                 check(L.cubvh_floodfill(P(grid), 1, res, res, res, P(lab), P(ws), nb, sp), "floodfill")
             dev_ops.append(("occupancy", 0, occ, "occupancy: udf < 2/res (torch.lt)"))
-            dev_ops.append((op, 0, fn, "floodfill: tile, merge and label kernels"))
+            dev_ops.append((op, 0, fn, "floodfill: tile, merge, resolve and label kernels"))
 
     q_per_step = sum(n for _, n, _, _ in dev_ops)
 

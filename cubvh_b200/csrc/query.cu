@@ -241,7 +241,8 @@ __device__ __forceinline__ AffineNode affine_node(const NodeView& nd, float3 o, 
     return a;
 }
 // Entry and exit (at most cull) of the ray in children 2 c and 2 c + 1:
-// entered where entry <= exit and 0 <= exit (never by a ray that is no number).
+// entered where entry <= exit and 0 <= exit.  A coordinate that is no number
+// bounds nothing: such a ray enters what its other axes meet, and hits nothing.
 __device__ __forceinline__ void affine_pair(const AffineNode& a, int c, float cull, float tn[2], float tf[2]) {
     const int h = c >> 1, b = 2 * (c & 1);
     float x0, x1, y0, y1, z0, z1;
@@ -603,11 +604,11 @@ __device__ __noinline__ int walk_ties(const WNode* __restrict__ wnodes, const WT
 // A point that is not finite, or farther than MAX_DIST from the root's box,
 // finds nothing and takes no part in the walk.
 //
-// Bound by instruction issue and the latency of node and triangle loads.
-// Measured against the walk with a lane per point and the records of
-// layout.h's first half (whole calls, today's other passes included): 1M
-// points on 5,120 faces 1.98 -> 0.92 ms, 384^3 grid on 177k faces 107.5 ->
-// 46.2 ms, 8.4M watertight points on 82k faces 9.70 -> 4.88 ms.
+// Bound by instruction issue and the latency of node and triangle loads; at 72
+// registers each variant spills 240 bytes of stores and 210 of loads.  Measured against the walk with a
+// lane per point and the records of layout.h's first half, whole calls: 1M
+// points on 5,120 faces 1.98 -> 0.99 ms, 384^3 grid on 177k faces 107.5 -> 48.0
+// ms, 8.4M watertight points on 82k faces 9.70 -> 5.52 ms.
 //
 // Heavy queries, served afterwards with a warp each (k_udf_heavy, from the
 // bound found so far): a point whose candidate list overflows (many
@@ -1094,7 +1095,7 @@ __global__ void __launch_bounds__(kQBlock) k_udf_heavy(const uint4* __restrict__
 // whole warp, four nodes a step (heavy_walk), as is one whose candidate list
 // overflows; so few queries get a warp each, more of them two or four.
 // Against unsorted packets (100 to 1,000 points on 82k faces 2.7 ms) 22 to 36
-// us; 16,000 points 544 -> 111 us, sorted packets of today 316.  The lines:
+// us; 16,000 points 544 -> 111 us, sorted packets 316.  The lines:
 // 32 and 96 visits are up to 1.5 and 2.5 times slower, fewer than the tree is
 // deep up to 3 times; at 64k queries packets draw level (82k-face mesh 376
 // against 302 us, 5,120 faces 389 against 396, 177k open tori 726 against 641).
@@ -1506,11 +1507,11 @@ __global__ void __launch_bounds__(kQBlock) k_sign_watertight_ovf(const uint32_t*
 // rounding of the double test lets slip between two triangles at their common
 // edge, about 1e-14 of all rays, is not seen this way.)  Inside points took
 // 64 rays, bound by divergence (12.5 of 32 lanes): 2.1M points in the box of a
-// closed 82k-face mesh, 18.9 -> 4.2 ms with the faster distance search (3.1 with
-// today's first pass).
+// closed 82k-face mesh, 18.9 -> 4.2 ms with the faster distance search.
 
 // Hash of an undirected edge by its end points' coordinates (0 for an edge
-// of no length): mesh edges cancel in pairs under XOR.
+// of no length): mesh edges cancel in pairs under XOR.  mix64 is David
+// Stafford's Mix01, a variant of MurmurHash3's 64-bit finaliser.
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
     x ^= x >> 31;
     x *= 0x7fb5d329728ea185ull;
@@ -1587,7 +1588,7 @@ __global__ void __launch_bounds__(256) k_edge_parity(int64_t nt, const CTri* __r
 // whenever kStabRefill are idle; its lanes stay on the same kind of step, inner
 // nodes until few are at one, then leaves.  Lanes refilled one by one, each on
 // its own step, took 2.2 of the 4.1 ms of 2.1M points on a closed 82k-face
-// mesh; now the call takes 3.0 (refill at 12 and 20 idle lanes 3.2 and 3.5).
+// mesh; in batches the call takes 3.0 (refill at 12 and 20 idle lanes 3.2 and 3.5).
 constexpr int kChunkMax = 2;      // packets per raystab chunk
 constexpr int kStabRefill = 6;   // idle lanes that take new queries
 constexpr int kStabInner = 12;    // fewer lanes at inner nodes than this wait for those at leaves
@@ -2037,12 +2038,13 @@ constexpr int kRayBlocks = 8;   // blocks of k_ray per SM
 // neighbouring pixels sweep nearly what they hit, so this keeps few children
 // that no ray needs, for about 100 instructions a node where a test per ray
 // and child with eight warp minima took 350 (33.5M camera rays on 82k faces:
-// 5.46 -> 3.11 ms a call; 32 warps per SM, 16 would be 20 % slower).  Children go onto the warp's
-// stack farthest entry first.  Each lane keeps U, an upper bound of its
+// 5.46 -> 3.14 ms a call; 32 warps per SM, 16 would be 20 % slower; at 64
+// registers 204 bytes of spill stores and 260 of loads).  Children go onto the
+// warp's stack farthest entry first.  Each lane keeps U, an upper bound of its
 // closest hit (certain FP32 hits: t + error bound), and a short list of
 // triangles that may still be closer (certain or undecided hits whose lower
-// bound is within U); the list is settled in double at the end: exact t of
-// the closest hit, ties -> lowest face index.
+// bound is within U); the list is settled in double at the end, or when one of
+// the warp's is full: exact t of the closest hit, ties -> lowest face index.
 __global__ void __launch_bounds__(kQBlock, kRayBlocks) k_ray(int64_t n, const uint32_t* __restrict__ order,
                                                  const float* __restrict__ ro,
                                                  const float* __restrict__ rd, float* __restrict__ pos,
@@ -2235,12 +2237,13 @@ constexpr int kFewLaneBlocks = 4, kFewLaneInner = 4;
 // wait until kLaneRefill lanes are idle, which settle their hits in double
 // together and take the next rays of the warp's packet.  A warp that walked
 // its 32 rays to the longest one's end had 6.8 lanes active and took 497
-// instructions a ray; now 11.3 and 287, with two children an instruction in
-// affine_pair: 5M random rays on 82k faces 3.36 -> 2.32 ms a call (refill at
-// 8 or 4 idle lanes 3 and 9 % slower, leaves at once 13 %; what is left is
-// load latency and divergence).  Filters,
-// candidate list and the FP64 settlement are k_ray's, so every result is the
-// one k_ray would give.
+// instructions a ray; refilled, with two children an instruction in
+// affine_pair, 11.3 and 287: 5M random rays on 82k faces 3.36 -> 2.32 ms a call
+// (refill at 8 or 4 idle lanes 3 and 9 % slower, leaves at once 13 %), 2.08 with
+// full lists settled out of line; what is left is load latency and divergence
+// (80 registers, 94 bytes of spill stores and 104 of loads).  Filters, candidate
+// list and the FP64 settlement are k_ray's, so every result is the one k_ray
+// would give.
 template <bool FEW>
 __global__ void __launch_bounds__(kQBlock, FEW ? kFewLaneBlocks : kLaneBlocks) k_ray_lanes(int64_t n, const uint32_t* __restrict__ order,
                                                        const float* __restrict__ ro, const float* __restrict__ rd,
