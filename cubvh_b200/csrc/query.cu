@@ -617,14 +617,22 @@ __device__ __noinline__ int walk_ties(const WNode* __restrict__ wnodes, const WT
 // is still walking after kHandOff visits when the queue is empty: deep
 // inside a closed mesh or near its medial axis points are about equally far
 // from very many triangles, and such a packet would hold the launch's end
-// alone.  When the heavy list is full both finish here instead, as do the
+// alone.  Only while few packets do so (kLateMost, counted from kLate visits
+// on): a warp a query is for idle SMs, and when most of a launch is such
+// packets it is many times the work (100,003 points at one place in 1.3M
+// faces 1,550 -> 567 us, within 0.1 of it 888 -> 678; a limit of 640 gives 569
+// and 526, but uniform points 820, 681 before and 672 at 1,500).  After
+// kHandOffAny visits packets are handed off in any case: the 384^3 grid has
+// unions of thousands of visits, 57 ms without that line, 51 at 1,024, 50.0 at 512.
+// When the heavy list is full both finish here instead, as do the
 // points of a packet most of which tie (faces that are there several times):
 // walked together once more they cost a fraction of a warp each (300k points
 // on 12 copies of 5,120 faces 36 against 5.1 ms, 1M at the middle of 3 copies
 // of 82k faces 7.7 against 5.5).  The grid of 384^3 points has packets of both
 // kinds and pays 2 % (48.9 against 50.0 ms); lines of 4 to 28 points measure
 // the same, so the line is a quarter of the packet.
-constexpr int kHandOff = 192;
+constexpr int kLate = 128, kHandOff = 192, kHandOffAny = 512;
+constexpr int kLateMost = 1500;
 constexpr int kTiesHere = 8;
 template <bool UVW, bool SLOT>
 __global__ void __launch_bounds__(kQBlock, kUdfBlocks) k_udf(Work w, const uint32_t* __restrict__ order,
@@ -633,7 +641,8 @@ __global__ void __launch_bounds__(kQBlock, kUdfBlocks) k_udf(Work w, const uint3
                                                  int32_t* __restrict__ slot_out, const DeviceTree tree,
                                                  unsigned long long* __restrict__ ctr, RunShape shape,
                                                  uint4* __restrict__ heavy, unsigned long long* __restrict__ n_heavy,
-                                                 int64_t heavy_cap, int block_grabs) {
+                                                 int64_t heavy_cap, unsigned long long* __restrict__ late,
+                                                 int block_grabs) {
     const CTri* __restrict__ tris = tree.tris;
     const int lane = threadIdx.x & 31;
     __shared__ uint2 s_cand[kQBlock / 32][kCand][32];
@@ -700,13 +709,18 @@ __global__ void __launch_bounds__(kQBlock, kUdfBlocks) k_udf(Work w, const uint3
         int cur = root;
         bool live = __any_sync(kFull, near_root);
         int work = 0;
-        bool handed_off = false;
+        bool handed_off = false, counted = false;
         while (live) {
-            if ((++work & 63) == 0 && work >= kHandOff) {   // warp-uniform
-                unsigned long long taken = 0;
-                if (lane == 0) taken = *reinterpret_cast<volatile unsigned long long*>(ctr);
+            if ((++work & 63) == 0 && work >= kLate) {   // warp-uniform
+                unsigned long long taken = 0, others = 0;
+                if (lane == 0) {
+                    taken = *reinterpret_cast<volatile unsigned long long*>(ctr);
+                    if (taken >= tickets) others = counted ? *reinterpret_cast<volatile unsigned long long*>(late) : atomicAdd(late, 1ull);
+                }
                 taken = __shfl_sync(kFull, taken, 0);
-                if (taken >= tickets) {
+                const bool first = !counted;
+                counted = taken >= tickets;
+                if (counted && !first && (work >= kHandOffAny || __shfl_sync(kFull, (int)others, 0) <= kLateMost)) {
                     unsigned long long b = 0;
                     if (lane == 0) b = atomicAdd(n_heavy, (unsigned long long)cnt);
                     b = __shfl_sync(kFull, b, 0);
@@ -787,6 +801,7 @@ __global__ void __launch_bounds__(kQBlock, kUdfBlocks) k_udf(Work w, const uint3
             }
         }
         if (handed_off) continue;
+        if (counted && lane == 0) atomicAdd(late, ~0ull);
         bool mine = act;
         const bool many = __popc(__ballot_sync(kFull, nc > kCand)) >= kTiesHere;
         bool again = false;
@@ -2640,6 +2655,7 @@ enum : int {
     kCtParity = 11,     // edge parity of a single BVH (k_edge_parity)
     kCtRayLanesN = 14,  // incoherent ray packets
     kCtRayLanesNext = 15,  // k_ray_lanes queue
+    kCtLate = 8,        // k_udf packets in a long walk after the queue is empty
     kCtRayPacketsN = 16,   // coherent ray packets
 };
 // packets per atomic grab: about 64 grabs per warp
@@ -2741,7 +2757,7 @@ void launch_nearest_t(const Work& w, int64_t n, const uint32_t* order, const flo
     const RunShape q = run_shape(n, g);
     const LaunchShape y = yield_shape(g, q.tickets(w.packets()), yield);
     k_udf<UVW, SLOT><<<y.grid, kQBlock, 0, stream>>>(w, order, pts, dist, fid, uvw, slots, tree, ctr + kCtUdf, q, heavy,
-                                                     ctr + kCtHeavyN, hcap, y.block_grabs); count_launch();
+                                                     ctr + kCtHeavyN, hcap, ctr + kCtLate, y.block_grabs); count_launch();
     const unsigned gh = persistent_grid(k_udf_heavy<UVW, SLOT>, 32 * hcap);
     k_udf_heavy<UVW, SLOT><<<gh, kQBlock, 0, stream>>>(heavy, ctr + kCtHeavyN, hcap, w.meshes, w.slot0, pts, dist, fid, uvw,
                                                        slots, tree, ctr + kCtHeavyNext); count_launch();
